@@ -25,6 +25,7 @@
 
 #include "../../include/blqh_gpu_debug.h"
 #include "krylov.cuh"
+#include "gs_ordered.cuh"
 #include "sector.cuh"
 
 double rayleigh_regen_impl(blqh_ctx* ctx, const blqh_basis* B, const blqh_params& p, const double* d_psi,
@@ -35,20 +36,6 @@ int hamil_build_impl(blqh_ctx* ctx, const blqh_basis* B, const blqh_params& p, i
 void free_csr(blqh_csr* m);
 
 namespace {
-
-constexpr int UPD_THREADS = 256;
-
-// device scalar block layout (doubles), per Lanczos object
-struct Scal {
-  double* alpha;  // [mmax]
-  double* beta;   // [mmax+1]; beta[0] = 0 internally
-  double* h;      // [2*(mmax+1)] Gram-Schmidt coefficients (re, im)
-  double* h2;     // [2*(mmax+1)] second pass
-  double* nrm;    // [4]: |w|^2 before, after pass 1, final
-  double* ritz;   // [mmax] lowest Ritz value at checks
-  int* flags;     // [8]: stop, pass2, steps, breakdown, a full-pass coefficient not small (FP64 update),
-                  //      the tridiagonal size of the last convergence check's Ritz value
-};
 
 // ---------------------------------------------------------------------------
 // SpMV: LPR lanes per row, FP64 accumulation. y = H x - b * xprev.
@@ -259,397 +246,6 @@ __global__ void k_split(const double* __restrict__ x, float2* __restrict__ xs, i
 }
 
 // ---------------------------------------------------------------------------
-// Gram-Schmidt dots: part[blk][k] = sum_{r in tile blk} conj(V_k[r]) w[r] for k
-// in [k0, k1), on tiles of GS_ROWS rows (one warp per vector at a time), and the
-// tile's |w|^2. cond: run only when the second pass was requested (flags[1]).
-constexpr int GS_ROWS = 1024;
-
-__device__ __forceinline__ double block_sum_256(double v, double* red) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double s = 0;
-  if (threadIdx.x == 0)
-    for (int i = 0; i < (int)(blockDim.x >> 5); i++) s += red[i];
-  __syncthreads();
-  return s;  // valid in thread 0
-}
-
-template <bool CPLX>
-__global__ void __launch_bounds__(256) k_dots(const double* __restrict__ V, int64_t dim, int k0, int k1,
-                                              const double* __restrict__ w, double* __restrict__ part, int stride,
-                                              double* __restrict__ part_norm, const int* flags, int cond) {
-  if (flags[0] || (cond && !flags[1])) return;
-  constexpr int VW = CPLX ? 2 : 1;
-  __shared__ double ws[GS_ROWS * VW];
-  __shared__ double red[8];
-  const int64_t r0 = (int64_t)blockIdx.x * GS_ROWS;
-  const int64_t rem = dim - r0;
-  const int nr = (int)(rem < GS_ROWS ? rem : GS_ROWS);
-  double nn = 0;
-  for (int t = threadIdx.x; t < GS_ROWS * VW; t += blockDim.x) {
-    const double v = (t < nr * VW) ? w[r0 * VW + t] : 0.0;
-    ws[t] = v;
-    nn += v * v;
-  }
-  const double tot = block_sum_256(nn, red);
-  if (threadIdx.x == 0 && part_norm) part_norm[blockIdx.x] = tot;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int k = k0 + wid; k < k1; k += (int)(blockDim.x >> 5)) {
-    const double* vk = V + ((int64_t)k * dim + r0) * VW;
-    double sr = 0, si = 0;
-    if (CPLX) {
-      for (int t = lane; t < nr; t += 32) {
-        const double2 a = reinterpret_cast<const double2*>(vk)[t];
-        const double br = ws[2 * t], bi = ws[2 * t + 1];
-        sr += a.x * br + a.y * bi;
-        si += a.x * bi - a.y * br;
-      }
-    } else {
-      for (int t = lane; t < nr; t += 32) sr += vk[t] * ws[t];
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      sr += __shfl_xor_sync(0xffffffffu, sr, o);
-      if (CPLX) si += __shfl_xor_sync(0xffffffffu, si, o);
-    }
-    if (lane == 0) {
-      part[((int64_t)blockIdx.x * stride + k) * 2] = sr;
-      part[((int64_t)blockIdx.x * stride + k) * 2 + 1] = si;
-    }
-  }
-}
-
-// One block per coefficient k (plus one for |w|^2 in stage 1): sums the tile
-// partials in a fixed order (deterministic).
-// stage 1: h = dots, alpha_j = Re h[j], nrm[0] = |w|^2
-// stage 2: h2 = dots (second pass), alpha_j += Re h2[j]
-__global__ void k_reduce_dots(const double* part, int nblk, int stride, int k0, int k1, const double* part_norm,
-                              Scal S, int j, int stage) {
-  if (S.flags[0] || (stage == 2 && !S.flags[1])) return;
-  __shared__ double red[8];
-  const int kb = blockIdx.x;
-  const bool is_norm = kb >= k1 - k0;
-  if (is_norm && (stage != 1 || !part_norm)) return;
-  double a = 0, b = 0;
-  if (!is_norm) {
-    const int k = k0 + kb;
-    for (int blk = threadIdx.x; blk < nblk; blk += blockDim.x) {
-      a += part[((int64_t)blk * stride + k) * 2];
-      b += part[((int64_t)blk * stride + k) * 2 + 1];
-    }
-  } else {
-    for (int blk = threadIdx.x; blk < nblk; blk += blockDim.x) a += part_norm[blk];
-  }
-  a = block_sum_256(a, red);
-  b = block_sum_256(b, red);
-  if (threadIdx.x != 0) return;
-  if (is_norm) {
-    S.nrm[0] = a;
-    return;
-  }
-  const int k = k0 + kb;
-  double* h = (stage == 1) ? S.h : S.h2;
-  h[2 * k] = a;
-  h[2 * k + 1] = b;
-  // the full pass's correction is summed on the FP32 pipes only while every
-  // coefficient is below 2^-30 |w| (see k_update)
-  if (stage == 2 && a * a + b * b > 0x1p-60 * S.nrm[1]) atomicOr(S.flags + 4, 1);
-  if (k == j) {
-    if (stage == 1) S.alpha[j] = a;
-    else S.alpha[j] += a;
-  }
-}
-
-// FP32 value with the 24 leading significant bits of x (truncated), from its
-// bit pattern with integer operations only (GB300's FP64 pipe issues ~2 lane
-// operations per clock per SM; this keeps the correction below off it).
-// |x| < 2^-126 gives 0; |x| < 2^128 is assumed (Krylov vectors have |x| <= 1).
-__device__ __forceinline__ float f64_lead_f32(double x) {
-  const unsigned long long bits = (unsigned long long)__double_as_longlong(x);
-  const unsigned hw = (unsigned)(bits >> 32), lw = (unsigned)bits;
-  const int e = (int)((hw >> 20) & 0x7FFu) - 896;  // FP32 biased exponent
-  const unsigned f = (hw & 0x80000000u) | ((unsigned)e << 23) | (__funnelshift_l(lw, hw, 3) & 0x7FFFFFu);
-  return e > 0 ? __uint_as_float(f) : 0.0f;
-}
-
-// w -= sum_k h[k] V_k over k in [k0, k1); partial |w|^2 per block.
-// The full pass (cond = 1) after the three-term step removes components that
-// are round-off sized (|h_k| <= 2^-30 |w|, checked by k_reduce_dots; flags[4]
-// is set otherwise): the correction sum_k h_k V_k is then accumulated in FP32
-// from FP32-truncated coefficients and vector entries (relative error ~2^-22
-// of a correction <= 2^-30 |w|, below FP64's rounding of w) and subtracted
-// from w in FP64. The local step (cond = 0) and a flagged pass use FP64 FMAs.
-template <bool CPLX>
-__global__ void __launch_bounds__(UPD_THREADS) k_update(const double* __restrict__ V, int64_t dim, int k0, int k1,
-                                                        const double* __restrict__ hcoef, double* __restrict__ w,
-                                                        double* __restrict__ part_norm, const int* flags, int cond) {
-  if (flags[0] || (cond && !flags[1])) return;
-  extern __shared__ double hs[];
-  const int nk = k1 - k0;
-  const bool lowp = cond && !flags[4];
-  float* hf = reinterpret_cast<float*>(hs + 2 * nk);
-  for (int t = threadIdx.x; t < 2 * nk; t += blockDim.x) {
-    const double c = hcoef[2 * k0 + t];
-    hs[t] = c;
-    hf[t] = f64_lead_f32(c);
-  }
-  __syncthreads();
-  double nn = 0;
-  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r < dim) {
-    if (CPLX) {
-      double2 acc = reinterpret_cast<const double2*>(w)[r];
-      if (lowp) {
-        float dr = 0.f, di = 0.f;
-        for (int k = 0; k < nk; k++) {
-          const double2 v = reinterpret_cast<const double2*>(V)[(int64_t)(k0 + k) * dim + r];
-          const float vr = f64_lead_f32(v.x), vi = f64_lead_f32(v.y);
-          const float hr = hf[2 * k], hi = hf[2 * k + 1];
-          dr = fmaf(hr, vr, fmaf(-hi, vi, dr));
-          di = fmaf(hr, vi, fmaf(hi, vr, di));
-        }
-        acc.x -= (double)dr;
-        acc.y -= (double)di;
-      } else {
-        for (int k = 0; k < nk; k++) {
-          const double2 v = reinterpret_cast<const double2*>(V)[(int64_t)(k0 + k) * dim + r];
-          const double hr = hs[2 * k], hi = hs[2 * k + 1];
-          acc.x -= hr * v.x - hi * v.y;
-          acc.y -= hr * v.y + hi * v.x;
-        }
-      }
-      reinterpret_cast<double2*>(w)[r] = acc;
-      nn = acc.x * acc.x + acc.y * acc.y;
-    } else {
-      double acc = w[r];
-      if (lowp) {
-        float d0 = 0.f, d1 = 0.f;
-        int k = 0;
-        for (; k + 2 <= nk; k += 2) {
-          d0 = fmaf(hf[2 * k], f64_lead_f32(V[(int64_t)(k0 + k) * dim + r]), d0);
-          d1 = fmaf(hf[2 * k + 2], f64_lead_f32(V[(int64_t)(k0 + k + 1) * dim + r]), d1);
-        }
-        if (k < nk) d0 = fmaf(hf[2 * k], f64_lead_f32(V[(int64_t)(k0 + k) * dim + r]), d0);
-        acc -= (double)(d0 + d1);
-      } else {
-        int k = 0;
-        for (; k + 4 <= nk; k += 4) {
-          const double v0 = V[(int64_t)(k0 + k) * dim + r], v1 = V[(int64_t)(k0 + k + 1) * dim + r];
-          const double v2 = V[(int64_t)(k0 + k + 2) * dim + r], v3 = V[(int64_t)(k0 + k + 3) * dim + r];
-          acc -= hs[2 * k] * v0;
-          acc -= hs[2 * k + 2] * v1;
-          acc -= hs[2 * k + 4] * v2;
-          acc -= hs[2 * k + 6] * v3;
-        }
-        for (; k < nk; k++) acc -= hs[2 * k] * V[(int64_t)(k0 + k) * dim + r];
-      }
-      w[r] = acc;
-      nn = acc * acc;
-    }
-  }
-  __shared__ double red[UPD_THREADS / 32];
-  const double tot = block_sum_256(nn, red);
-  if (threadIdx.x == 0) part_norm[blockIdx.x] = tot;
-}
-
-// ---------------------------------------------------------------------------
-// Gram-Schmidt on FP32 planes (FP32 values with double-float accumulation).
-// Next to each FP64 Krylov vector V_k the library keeps two FP32 planes, Vh_k =
-// the leading 24 bits of V_k (truncated, f64_lead_f32) and Vl_k = the rest
-// rounded to FP32, so that Vh + Vl = V_k to 2^-48. The full Gram-Schmidt pass
-// then runs on GB300's FP32 pipes (its FP64 pipe issues ~2 lane operations per
-// clock per SM, which capped the FP64 dots at ~35 % of HBM bandwidth):
-//   * dots conj(V_k) w in double-float from (Vh, Vl) and the split of w
-//     (error <= ~2^-46 sum |V_k| |w|, FP64-class): 8 bytes per entry;
-//   * the correction of k_update's FP32 path reads Vh only: 4 bytes per entry
-//     instead of 8, with the same values it used before.
-// Rows of a plane are padded to a multiple of 4 floats (zero-filled).
-
-// (hi, lo) planes of one vector: hi = leading 24 bits of x, lo = the rest rounded.
-__global__ void k_planes(const double* __restrict__ x, float* __restrict__ vh, float* __restrict__ vl, int64_t n) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const double v = x[i];
-    const float h = f64_lead_f32(v);
-    vh[i] = h;
-    vl[i] = (float)(v - (double)h);
-  }
-}
-
-// (ah, al) += (vh + vl) (wh + wl) in double-float (the vl wl term, ~2^-48 of the
-// product, is dropped).
-__device__ __forceinline__ void df_prod_split(float& ah, float& al, float vh, float vl, float wh, float wl) {
-  const float p = vh * wh;
-  const float pe = fmaf(vh, wh, -p);
-  const float t = fmaf(vh, wl, fmaf(vl, wh, pe));
-  float s, e;
-  two_sum(ah, p, s, e);
-  ah = s;
-  al += e + t;
-}
-
-// part[blk][k] = conj(V_k) w over the tile blk of GS_ROWS rows, for k in
-// [k0, k1), from the planes (row stride ld floats). One warp per vector at a
-// time, 16-byte loads. cond: run only when the second pass was requested.
-template <bool CPLX>
-__global__ void __launch_bounds__(256) k_dots_df(const float* __restrict__ Vh, const float* __restrict__ Vl,
-                                                 int64_t ld, int64_t dim, int k0, int k1,
-                                                 const double* __restrict__ w, double* __restrict__ part, int stride,
-                                                 const int* flags, int cond) {
-  if (flags[0] || (cond && !flags[1])) return;
-  constexpr int VW = CPLX ? 2 : 1;
-  constexpr int TF = GS_ROWS * VW;  // floats of a plane tile
-  __shared__ __align__(16) float wh[TF];
-  __shared__ __align__(16) float wl[TF];
-  const int64_t e0 = (int64_t)blockIdx.x * TF;
-  const int64_t n = dim * VW;
-  const int ne = (int)(n - e0 < TF ? n - e0 : TF);
-  for (int t = threadIdx.x; t < TF; t += blockDim.x) {
-    const double v = t < ne ? w[e0 + t] : 0.0;
-    const float h = (float)v;
-    wh[t] = h;
-    wl[t] = (float)(v - (double)h);
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int k = k0 + wid; k < k1; k += (int)(blockDim.x >> 5)) {
-    const float* ph = Vh + (int64_t)k * ld + e0;
-    const float* pl = Vl + (int64_t)k * ld + e0;
-    float sh = 0.f, sl = 0.f, ih = 0.f, il = 0.f;
-#pragma unroll 2
-    for (int t = lane * 4; t < ne; t += 128) {  // the row padding keeps t + 3 inside the plane
-      const float4 h4 = __ldcs(reinterpret_cast<const float4*>(ph + t));
-      const float4 l4 = __ldcs(reinterpret_cast<const float4*>(pl + t));
-      const float4 a4 = *reinterpret_cast<const float4*>(wh + t);
-      const float4 b4 = *reinterpret_cast<const float4*>(wl + t);
-      if (CPLX) {  // two entries (re, im): conj(v) w = (vr wr + vi wi, vr wi - vi wr)
-        df_prod_split(sh, sl, h4.x, l4.x, a4.x, b4.x);
-        df_prod_split(sh, sl, h4.y, l4.y, a4.y, b4.y);
-        df_prod_split(ih, il, h4.x, l4.x, a4.y, b4.y);
-        df_prod_split(ih, il, -h4.y, -l4.y, a4.x, b4.x);
-        df_prod_split(sh, sl, h4.z, l4.z, a4.z, b4.z);
-        df_prod_split(sh, sl, h4.w, l4.w, a4.w, b4.w);
-        df_prod_split(ih, il, h4.z, l4.z, a4.w, b4.w);
-        df_prod_split(ih, il, -h4.w, -l4.w, a4.z, b4.z);
-      } else {
-        df_prod_split(sh, sl, h4.x, l4.x, a4.x, b4.x);
-        df_prod_split(sh, sl, h4.y, l4.y, a4.y, b4.y);
-        df_prod_split(sh, sl, h4.z, l4.z, a4.z, b4.z);
-        df_prod_split(sh, sl, h4.w, l4.w, a4.w, b4.w);
-      }
-    }
-    df_seg_reduce<32>(sh, sl);
-    if (CPLX) df_seg_reduce<32>(ih, il);
-    if (lane == 0) {
-      part[((int64_t)blockIdx.x * stride + k) * 2] = (double)sh + (double)sl;
-      part[((int64_t)blockIdx.x * stride + k) * 2 + 1] = CPLX ? (double)ih + (double)il : 0.0;
-    }
-  }
-}
-
-// k_update with planes: four consecutive entries of w per thread (two complex
-// rows). The FP32 path reads Vh (16-byte loads); the FP64 path (the local step,
-// or a flagged pass) reads V. Same arithmetic, in the same order, as k_update.
-template <bool CPLX>
-__global__ void __launch_bounds__(UPD_THREADS) k_update_pl(const double* __restrict__ V,
-                                                           const float* __restrict__ Vh, int64_t ld, int64_t dim,
-                                                           int k0, int k1, const double* __restrict__ hcoef,
-                                                           double* __restrict__ w, double* __restrict__ part_norm,
-                                                           const int* flags, int cond) {
-  if (flags[0] || (cond && !flags[1])) return;
-  extern __shared__ double hs[];
-  const int nk = k1 - k0;
-  const bool lowp = cond && !flags[4];
-  float* hf = reinterpret_cast<float*>(hs + 2 * nk);
-  for (int t = threadIdx.x; t < 2 * nk; t += blockDim.x) {
-    const double c = hcoef[2 * k0 + t];
-    hs[t] = c;
-    hf[t] = f64_lead_f32(c);
-  }
-  __syncthreads();
-  constexpr int VW = CPLX ? 2 : 1;
-  const int64_t n = dim * VW;
-  const int64_t e0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
-  double nn = 0;
-  if (e0 < n) {
-    const int ne = (int)(n - e0 < 4 ? n - e0 : 4);  // 4, or the tail (complex: even)
-    double a[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) a[q] = q < ne ? w[e0 + q] : 0.0;
-    if (lowp) {
-      if (CPLX) {
-        float dr0 = 0.f, di0 = 0.f, dr1 = 0.f, di1 = 0.f;
-#pragma unroll 4
-        for (int k = 0; k < nk; k++) {
-          const float4 v = __ldcs(reinterpret_cast<const float4*>(Vh + (int64_t)(k0 + k) * ld + e0));
-          const float hr = hf[2 * k], hi = hf[2 * k + 1];
-          dr0 = fmaf(hr, v.x, fmaf(-hi, v.y, dr0));
-          di0 = fmaf(hr, v.y, fmaf(hi, v.x, di0));
-          dr1 = fmaf(hr, v.z, fmaf(-hi, v.w, dr1));
-          di1 = fmaf(hr, v.w, fmaf(hi, v.z, di1));
-        }
-        a[0] -= (double)dr0;
-        a[1] -= (double)di0;
-        a[2] -= (double)dr1;
-        a[3] -= (double)di1;
-      } else {
-        float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};  // even and odd k
-        int k = 0;
-#pragma unroll 2
-        for (; k + 2 <= nk; k += 2) {
-          const float4 v0 = __ldcs(reinterpret_cast<const float4*>(Vh + (int64_t)(k0 + k) * ld + e0));
-          const float4 v1 = __ldcs(reinterpret_cast<const float4*>(Vh + (int64_t)(k0 + k + 1) * ld + e0));
-          const float h0 = hf[2 * k], h1 = hf[2 * k + 2];
-          d0[0] = fmaf(h0, v0.x, d0[0]);
-          d0[1] = fmaf(h0, v0.y, d0[1]);
-          d0[2] = fmaf(h0, v0.z, d0[2]);
-          d0[3] = fmaf(h0, v0.w, d0[3]);
-          d1[0] = fmaf(h1, v1.x, d1[0]);
-          d1[1] = fmaf(h1, v1.y, d1[1]);
-          d1[2] = fmaf(h1, v1.z, d1[2]);
-          d1[3] = fmaf(h1, v1.w, d1[3]);
-        }
-        if (k < nk) {
-          const float4 v0 = __ldcs(reinterpret_cast<const float4*>(Vh + (int64_t)(k0 + k) * ld + e0));
-          const float h0 = hf[2 * k];
-          d0[0] = fmaf(h0, v0.x, d0[0]);
-          d0[1] = fmaf(h0, v0.y, d0[1]);
-          d0[2] = fmaf(h0, v0.z, d0[2]);
-          d0[3] = fmaf(h0, v0.w, d0[3]);
-        }
-#pragma unroll
-        for (int q = 0; q < 4; q++) a[q] -= (double)(d0[q] + d1[q]);
-      }
-    } else {
-      for (int k = 0; k < nk; k++) {
-        const double* vk = V + (int64_t)(k0 + k) * n + e0;
-        const double hr = hs[2 * k], hi = hs[2 * k + 1];
-        if (CPLX) {
-#pragma unroll
-          for (int q = 0; q < 4; q += 2)
-            if (q < ne) {
-              const double vr = vk[q], vi = vk[q + 1];
-              a[q] -= hr * vr - hi * vi;
-              a[q + 1] -= hr * vi + hi * vr;
-            }
-        } else {
-#pragma unroll
-          for (int q = 0; q < 4; q++)
-            if (q < ne) a[q] -= hr * vk[q];
-        }
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-      if (q < ne) {
-        w[e0 + q] = a[q];
-        nn += a[q] * a[q];
-      }
-  }
-  __shared__ double red[UPD_THREADS / 32];
-  const double tot = block_sum_256(nn, red);
-  if (threadIdx.x == 0) part_norm[blockIdx.x] = tot;
-}
-
 // <psi|H|psi> with each FP64 element carried as v32 + res (FP32 value and the
 // FP32 rest of the builder's FP64 value, 2^-48 relative): y = H32 psi comes
 // from the double-float SpMV; here one warp per row sums res * psi_hi in FP32
@@ -692,68 +288,6 @@ __global__ void __launch_bounds__(256) k_rq_res(const int64_t* __restrict__ rp, 
   }
   const double t = block_sum_256(acc, red);
   if (threadIdx.x == 0) part[blockIdx.x] = t;
-}
-
-// After pass 1: |w|^2 and whether a second Gram-Schmidt pass is needed (the
-// norm dropped below 1/sqrt(2) of its value before the pass); after pass 2:
-// the final |w|^2. which: 1 = after pass 1, 2 = after pass 2.
-// beta_{j+1} = |w| from the final |w|^2, the step count, and the breakdown test
-// (one thread).
-__device__ __forceinline__ void beta_from(Scal S, int j, double nrm2, double breakdown_tol) {
-  const double b = sqrt(nrm2);
-  S.beta[j + 1] = b;
-  S.flags[2] = j + 1;
-  const double scale = fabs(S.alpha[j]) + S.beta[j];
-  if (!(b > breakdown_tol * (scale > 0 ? scale : 1.0))) {
-    S.flags[3] = 1;
-    S.flags[0] = 1;
-  }
-}
-
-// After pass 1: |w|^2 and whether a second Gram-Schmidt pass is needed (the
-// norm dropped below 1/sqrt(2) of its value before the pass); after pass 2:
-// the final |w|^2. which: 1 = after pass 1, 2 = after pass 2. With
-// breakdown_tol > 0 this is the step's last norm: it also sets beta_{j+1}.
-__global__ void k_norm_step(const double* part_norm, int nblk, Scal S, int j, int which, int always_pass2,
-                            double breakdown_tol) {
-  if (S.flags[0]) return;
-  if (which == 2 && !S.flags[1]) {  // no second pass: the final norm is pass 1's
-    if (breakdown_tol > 0 && threadIdx.x == 0) beta_from(S, j, S.nrm[1], breakdown_tol);
-    return;
-  }
-  __shared__ double red[8];
-  double a = 0;
-  for (int b = threadIdx.x; b < nblk; b += blockDim.x) a += part_norm[b];
-  a = block_sum_256(a, red);
-  if (threadIdx.x != 0) return;
-  S.nrm[1] = a;
-  if (which == 1) {
-    S.flags[1] = always_pass2 ? 1 : (a < 0.5 * S.nrm[0]) ? 1 : 0;
-    S.flags[4] = 0;
-  }
-  if (breakdown_tol > 0) beta_from(S, j, a, breakdown_tol);
-}
-
-// V_{j+1} = w / beta_{j+1}
-// (and its FP32 planes when vh is set, and its (hi, lo) split for the next
-// double-float SpMV when xs is set, as k_split would write it)
-__global__ void k_scale(const double* __restrict__ w, double* __restrict__ vout, int64_t n, Scal S, int j,
-                        float* __restrict__ vh, float* __restrict__ vl, float2* __restrict__ xs) {
-  if (S.flags[0]) return;
-  const double inv = 1.0 / S.beta[j + 1];
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const double v = w[i] * inv;
-    vout[i] = v;
-    if (xs) {
-      const float hi = (float)v;
-      xs[i] = make_float2(hi, (float)(v - (double)hi));
-    }
-    if (vh) {
-      const float h = f64_lead_f32(v);
-      vh[i] = h;
-      vl[i] = (float)(v - (double)h);
-    }
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1077,13 +611,22 @@ struct blqh_lanczos {
   Scal S{};
   double* part = nullptr;  // dot partials [nblk_dot * (mmax+1) * 2]
   double* pnorm = nullptr; // [max(nblk_dot, nblk_upd)]
+  double2* apart = nullptr;  // partials of h_j (at most 2 blocks per SM)
+  double* npart = nullptr;   // [ntile] partials of |w|^2 after the three-term step
   double* work = nullptr;  // tridiagonal work [5*mmax + ...]
   double* y = nullptr;     // [mmax] Ritz coefficients
   float2* xs = nullptr;    // [dim * vw] (hi, lo) split of the SpMV input (double-float accumulation)
-  float* Vh = nullptr;     // [(mmax+1) * pld] FP32 planes of V for the Gram-Schmidt pass (or null)
+  // complex sectors: fixed-point planes of V and, in the last row, of w (or null)
+  int* Q1 = nullptr;       // [(mmax+2) * pld]
+  int* Q0 = nullptr;
+  int* QE = nullptr;       // [(mmax+2) * ntile] tile exponents
+  int tile = 0, ntile = 0; // doubles per tile, tiles of a vector
+  int64_t pld = 0;         // plane row stride: ntile * tile
+  // real sectors: FP32 planes of V for the Gram-Schmidt pass, hi and (double-float dots) lo (or null)
+  float* Vh = nullptr;     // [(mmax+1) * vld]
   float* Vl = nullptr;
-  int64_t pld = 0;         // plane row stride (floats): dim * vw rounded up to a multiple of 4
-  int nblk_dot = 0, nblk_upd = 0;
+  int64_t vld = 0;         // plane row stride (floats): dim rounded up to a multiple of 4
+  int nblk_dot = 0, nblk_upd = 0;  // 1024-row tiles; blocks of the ordered update
   int steps = 0;
   int last_check = -1;  // ritz[] slot of the last convergence check of the last run (-1: none)
   bool started = false, iterated = false, have_psi = false;
@@ -1094,6 +637,9 @@ namespace {
 void free_lanczos(blqh_lanczos* L) {
   if (!L) return;
   dev_free(L->xs);
+  dev_free(L->Q1);
+  dev_free(L->Q0);
+  dev_free(L->QE);
   dev_free(L->Vh);
   dev_free(L->Vl);
   dev_free(L->V);
@@ -1102,6 +648,8 @@ void free_lanczos(blqh_lanczos* L) {
   dev_free(L->scal);
   dev_free(L->part);
   dev_free(L->pnorm);
+  dev_free(L->apart);
+  dev_free(L->npart);
   dev_free(L->work);
   dev_free(L->y);
   delete L;
@@ -1206,59 +754,134 @@ int tri_smem(const blqh_lanczos* L, int per) {
   return b <= 48 * 1024 ? (int)b : 0;
 }
 
-template <bool CPLX>
-void gs_pass(blqh_lanczos* L, int k0, int k1, int j, int stage) {
+// A kernel of the step chain: its blocks may be placed while the previous kernel
+// on the stream drains; it waits for that kernel's results itself (pdl_begin).
+template <class... P, class... A>
+void launch_chained(blqh_ctx* ctx, void (*kern)(P...), int grid, int block, size_t smem, A... args) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = ctx->stream;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  BLQH_TRY_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
+}
+
+// Rows of the planes: vector k, and w after the stored vectors.
+int* q1_row(const blqh_lanczos* L, int k) { return L->Q1 ? L->Q1 + (int64_t)k * L->pld : nullptr; }
+int* q0_row(const blqh_lanczos* L, int k) { return L->Q0 ? L->Q0 + (int64_t)k * L->pld : nullptr; }
+int* qe_row(const blqh_lanczos* L, int k) { return L->QE ? L->QE + (int64_t)k * L->ntile : nullptr; }
+
+NextVec next_vec(const blqh_lanczos* L, int k) {
+  return {L->V + (int64_t)k * L->dim * L->vw, L->M->precision == BLQH_VAL_FP32 ? L->xs : nullptr, q1_row(L, k),
+          q0_row(L, k), qe_row(L, k)};
+}
+
+// The step after the SpMV on the fixed-point planes (complex sectors).
+template <int TILE>
+void gs_step_q(blqh_lanczos* L, int j) {
   blqh_ctx* ctx = L->ctx;
-  cudaStream_t st = ctx->stream;
-  const int stride = L->mmax + 1;
-  const int cond = (stage == 2);
-  if (L->Vh && stage == 2)  // the full pass on the FP32 planes (the local step stays in FP64)
-    k_dots_df<CPLX><<<L->nblk_dot, 256, 0, st>>>(L->Vh, L->Vl, L->pld, L->dim, k0, k1, L->w, L->part, stride,
-                                                 L->S.flags, cond);
+  constexpr bool LOCAL = TILE == 256;
+  const int64_t n = L->dim * 2;
+  const double* vj = L->V + (int64_t)j * n;
+  const int nk = j + 1, wr = L->mmax + 1, ng = (nk + DOT_GROUP - 1) / DOT_GROUP;
+  const int na = grid_for(ctx, L->dim, 1024, 2);
+  const WTile W{vj, L->w, L->apart, na, q1_row(L, wr), q0_row(L, wr), qe_row(L, wr), L->npart};
+  launch_chained(ctx, k_alpha<true>, na, 256, 0, vj, L->w, L->dim, L->apart, L->S);
+  if (!LOCAL)
+    launch_chained(ctx, k_local<true, TILE>, L->ntile, TILE / 4, 0, vj, L->w, n, L->apart, na, q1_row(L, wr),
+                   q0_row(L, wr), qe_row(L, wr), L->npart, L->S, j);
+  launch_chained(ctx, k_dots_q<true, TILE, LOCAL>, ng * L->ntile, 256, 0, L->Q1, L->Q0, L->QE, L->pld, L->ntile, n,
+                 nk, ng, W, L->part, L->S, j);
+  const size_t hsm = (size_t)nk * 2 * sizeof(float);
+  auto update = [&](auto kern, int threads) {
+    launch_chained(ctx, kern, L->ntile, threads, hsm, L->V, L->Q1, L->QE, L->pld, L->ntile, n, nk, W, L->w, L->pnorm,
+                   L->S, j, 1e-13, next_vec(L, j + 1));
+  };
+  // one slice of vectors per block while the blocks alone give every SM four
+  if constexpr (LOCAL) update(k_update_q<true, 256, 16, true>, 1024);
+  else if (L->ntile >= 4 * ctx->num_sms) update(k_update_q<true, 1024, 1, false>, 256);
+  else update(k_update_q<true, 1024, 4, false>, 1024);
+  count_launch(ctx, TM_REORTH, LOCAL ? 3 : 4);
+}
+
+NextPlanes next_planes(const blqh_lanczos* L, int k) {
+  return {L->V + (int64_t)k * L->dim * L->vw, L->M->precision == BLQH_VAL_FP32 ? L->xs : nullptr,
+          L->Vh ? L->Vh + (int64_t)k * L->vld : nullptr, L->Vl ? L->Vl + (int64_t)k * L->vld : nullptr, L->vld};
+}
+
+// The step after the SpMV in the fixed order of operations (real sectors, and
+// complex ones without fixed-point planes).
+template <bool CPLX>
+void gs_step_o(blqh_lanczos* L, int j) {
+  blqh_ctx* ctx = L->ctx;
+  const int64_t n = L->dim * L->vw;
+  const double* vj = L->V + (int64_t)j * n;
+  const int nt = L->nblk_dot, nu = L->nblk_upd;
+  const bool df = L->Vl != nullptr;  // double-float dots, four entries per thread in the updates
+  double* apart = reinterpret_cast<double*>(L->apart);
+  launch_chained(ctx, k_alpha_o<CPLX>, nt, 32, 0, vj, L->w, L->dim, apart, L->S);
+  const int lg = std::min(nu, 4 * ctx->num_sms);
+  if (df)
+    launch_chained(ctx, k_local_o<false, 4>, lg, 256, 0, vj, L->w, L->dim, apart, nt, L->pnorm, nu, L->S, j);
   else
-    k_dots<CPLX><<<L->nblk_dot, 256, 0, st>>>(L->V, L->dim, k0, k1, L->w, L->part, stride, L->pnorm, L->S.flags,
-                                              cond);
-  k_reduce_dots<<<k1 - k0 + 1, 256, 0, st>>>(L->part, L->nblk_dot, stride, k0, k1, L->pnorm, L->S, j, stage);
-  const double* hc = (stage == 1) ? L->S.h : L->S.h2;
-  const size_t hsm = 2 * (k1 - k0) * (sizeof(double) + sizeof(float));
-  if (L->Vh)
-    k_update_pl<CPLX><<<L->nblk_upd, UPD_THREADS, hsm, st>>>(L->V, L->Vh, L->pld, L->dim, k0, k1, hc, L->w,
-                                                             L->pnorm, L->S.flags, cond);
-  else
-    k_update<CPLX><<<L->nblk_upd, UPD_THREADS, hsm, st>>>(L->V, L->dim, k0, k1, hc, L->w, L->pnorm, L->S.flags,
-                                                          cond);
+    launch_chained(ctx, k_local_o<CPLX, 1>, lg, 256, 0, vj, L->w, L->dim, apart, nt, L->pnorm, nu, L->S, j);
+  if (L->o.reorth) {
+    const int nk = j + 1;
+    // up to 64 tiles: 8 vectors per block (one per warp), summed by each group's last block; beyond, a
+    // kernel for the sums, and more vectors per block once the blocks would fill the GPU over and over:
+    // 4 times for double-float dots (staging w's tile splits it), 16 for FP64 ones (32 at least: 4 per warp)
+    const int finish = nt <= 64;
+    const int step = finish || df || CPLX ? 8 : 32;
+    const int waves = (int)((int64_t)nt * ((nk + step - 1) / step) / ((df ? 4 : 16) * ctx->num_sms));
+    const int gk = step * (finish ? 1 : std::max(1, waves)), ng = (nk + gk - 1) / gk;
+    auto dots = [&](auto kern) {
+      launch_chained(ctx, kern, ng * nt, 256, 0, L->V, L->Vh, L->Vl, L->vld, L->dim, nt, nk, gk, ng, L->w, L->part,
+                     L->pnorm, nu, finish, L->S, j);
+      if (!finish) launch_chained(ctx, k_reduce_o<CPLX>, nk, 256, 0, L->part, nt, L->pnorm, nu, L->S, j);
+    };
+    const size_t hsm = 2 * nk * (sizeof(double) + sizeof(float));
+    auto update = [&](auto kern) {
+      launch_chained(ctx, kern, nu, 256, hsm, L->V, L->Vh, L->vld, L->dim, nk, L->w, L->pnorm, L->S);
+    };
+    if constexpr (CPLX) {
+      dots(k_dots_o<true, false, 1>);
+      update(k_update_o<true, 1, false>);
+    } else if (df) {
+      dots(k_dots_o<false, true, 1>);
+      update(k_update_o<false, 4, true>);
+    } else {
+      if (finish) dots(k_dots_o<false, false, 1>);
+      else dots(k_dots_o<false, false, 4>);
+      if (L->Vh) update(k_update_o<false, 1, true>);
+      else update(k_update_o<false, 1, false>);
+    }
+    count_launch(ctx, TM_REORTH, finish ? 2 : 3);
+  }
+  launch_chained(ctx, k_scale_o, grid_for(ctx, n, 256, 2), 256, 0, L->w, n, 0, L->pnorm, nu, L->S, j, 1e-13,
+                 next_planes(L, j + 1));
   count_launch(ctx, TM_REORTH, 3);
 }
 
-template <bool CPLX>
 void lanczos_step(blqh_lanczos* L, int j) {
   blqh_ctx* ctx = L->ctx;
-  cudaStream_t st = ctx->stream;
   const int64_t n = L->dim * L->vw;
   double* vj = L->V + (int64_t)j * n;
   const double* vprev = j > 0 ? L->V + (int64_t)(j - 1) * n : nullptr;
-  // from the second step on, the previous step's k_scale left v_j's split in xs
+  // from the second step on, the previous step left v_j's split in xs
   spmv_dev(ctx, L->M, vj, L->w, j > 0 ? L->S.beta + j : nullptr, vprev, L->S.flags, L->xs, j > 0);
-  {
-    TimerScope ts(ctx, TM_REORTH);
-    // three-term step: the SpMV removed beta_j v_{j-1}; remove the v_j component
-    // (alpha_j). With reorth, one classical Gram-Schmidt pass against every stored
-    // vector follows; taking the local step first keeps that pass from having to
-    // be repeated (the norm drop of the alpha_j removal no longer enters it).
-    gs_pass<CPLX>(L, j, j + 1, j, 1);
-    // the step's last norm step also sets beta_{j+1} (breakdown below 1e-13 of |alpha_j| + beta_j)
-    k_norm_step<<<1, 256, 0, st>>>(L->pnorm, L->nblk_upd, L->S, j, 1, L->o.reorth ? 1 : 0,
-                                    L->o.reorth ? 0.0 : 1e-13);
-    if (L->o.reorth) {
-      gs_pass<CPLX>(L, 0, j + 1, j, 2);
-      k_norm_step<<<1, 256, 0, st>>>(L->pnorm, L->nblk_upd, L->S, j, 2, 0, 1e-13);
-    }
-    k_scale<<<grid_for(ctx, n, 256, 8), 256, 0, st>>>(L->w, L->V + (int64_t)(j + 1) * n, n, L->S, j,
-                                                      L->Vh ? L->Vh + (int64_t)(j + 1) * L->pld : nullptr,
-                                                      L->Vl ? L->Vl + (int64_t)(j + 1) * L->pld : nullptr,
-                                                      L->M->precision == BLQH_VAL_FP32 ? L->xs : nullptr);
-    count_launch(ctx, TM_REORTH, L->o.reorth ? 3 : 2);
-  }
+  // three-term step: the SpMV removed beta_j v_{j-1}; remove the v_j component
+  // (alpha_j). With reorth, one classical Gram-Schmidt pass against every stored
+  // vector follows; taking the local step first keeps that pass from having to
+  // be repeated (the norm drop of the alpha_j removal no longer enters it). The
+  // step's last norm also sets beta_{j+1} (breakdown below 1e-13 of |alpha_j| + beta_j).
+  TimerScope ts(ctx, TM_REORTH);
+  if (L->Q1) L->tile == 1024 ? gs_step_q<1024>(L, j) : gs_step_q<256>(L, j);
+  else L->cplx ? gs_step_o<true>(L, j) : gs_step_o<false>(L, j);
 }
 
 void iterate_impl(blqh_lanczos* L) {
@@ -1283,15 +906,19 @@ void iterate_impl(blqh_lanczos* L) {
     }
     L->started = true;
   }
-  if (L->Vh) {  // planes of the start vector (the steps write the others)
-    TimerScope tm(ctx, TM_MISC);
-    const int64_t n = L->dim * L->vw;
-    k_planes<<<grid_for(ctx, n, 256, 8), 256, 0, st>>>(L->V, L->Vh, L->Vl, n);
-    BLQH_TRY_CUDA(ctx, cudaGetLastError());
-    count_launch(ctx, TM_MISC);
-  }
   BLQH_TRY_CUDA(ctx, cudaMemsetAsync(L->S.flags, 0, 4 * sizeof(int), st));
   BLQH_TRY_CUDA(ctx, cudaMemsetAsync(L->S.flags + 5, 0xFF, sizeof(int), st));  // no check's size yet
+  if (L->Q1 || L->Vh) {  // planes of the start vector (the steps write the others)
+    TimerScope tm(ctx, TM_MISC);
+    const int64_t n = L->dim * L->vw;
+    if (L->Q1)
+      launch_chained(ctx, L->tile == 1024 ? k_planes_q<1024> : k_planes_q<256>, L->ntile, L->tile / 4, 0, L->V, n,
+                     next_vec(L, 0));
+    else
+      launch_chained(ctx, k_scale_o, grid_for(ctx, n, 256, 2), 256, 0, L->V, n, 1, nullptr, 0, L->S, 0, 0.0,
+                     next_planes(L, 0));
+    count_launch(ctx, TM_MISC);
+  }
   BLQH_TRY_CUDA(ctx, cudaMemsetAsync(L->S.beta, 0, sizeof(double), st));
   const int chunk = std::max(1, L->o.check_every);
   const bool conv = L->o.tol > 0;
@@ -1304,10 +931,7 @@ void iterate_impl(blqh_lanczos* L) {
   bool stop = false;
   while (j < L->mmax && !stop) {
     const int jend = std::min(L->mmax, j + chunk);
-    for (; j < jend; j++) {
-      if (L->cplx) lanczos_step<true>(L, j);
-      else lanczos_step<false>(L, j);
-    }
+    for (; j < jend; j++) lanczos_step(L, j);
     if (conv) {  // with tol = 0 the recurrence runs to max_steps: no check needed
       TimerScope tm(ctx, TM_MISC);
       k_tri_lowest<<<1, 32, tri_smem(L, 2), st>>>(L->S, 1, L->o.tol, launched_chunks, tri_smem(L, 2) > 0);
@@ -1439,8 +1063,8 @@ void tune_spmv(blqh_lanczos* L) {
   else if (M->blk_state > 0) blocked_release(M);
 }
 
-// The full Gram-Schmidt pass of FP32-valued runs (accumulate = 0) works on FP32
-// planes of the Krylov basis; BLQH_GS_FP64=1 keeps it in FP64.
+// The full Gram-Schmidt pass works on planes next to the Krylov basis (fixed point
+// in complex sectors, FP32 in real ones); BLQH_GS_FP64=1 keeps it on the FP64 vectors.
 bool gs_planes_enabled() {
   const char* e = getenv("BLQH_GS_FP64");
   return !(e && e[0] == '1');
@@ -1487,17 +1111,22 @@ blqh_lanczos* create_impl(blqh_ctx* ctx, const blqh_csr* M, const blqh_lanczos_o
   L->mmax = (int)std::min<int64_t>(o.max_steps, M->dim);
   const_cast<blqh_csr*>(M)->lanes_per_row = spmv_lpr(M->mean_row);
   const int upd_smem = 2 * (L->mmax + 1) * (int)(sizeof(double) + sizeof(float));
-  smem_attr_at_least(k_update<false>, upd_smem);
-  smem_attr_at_least(k_update<true>, upd_smem);
-  smem_attr_at_least(k_update_pl<false>, upd_smem);
-  smem_attr_at_least(k_update_pl<true>, upd_smem);
+  smem_attr_at_least(k_update_o<false, 1, false>, upd_smem);
+  smem_attr_at_least(k_update_o<false, 1, true>, upd_smem);
+  smem_attr_at_least(k_update_o<false, 4, true>, upd_smem);
+  smem_attr_at_least(k_update_o<true, 1, false>, upd_smem);
+  const int q_smem = 2 * (L->mmax + 1) * (int)sizeof(float);
+  smem_attr_at_least(k_update_q<true, 256, 16, true>, q_smem);
+  smem_attr_at_least(k_update_q<true, 1024, 4, false>, q_smem);
+  smem_attr_at_least(k_update_q<true, 1024, 1, false>, q_smem);
   try {
     const int64_t n = L->dim * L->vw;
     L->V = dalloc<double>(ctx, (size_t)(L->mmax + 1) * n);
     L->w = dalloc<double>(ctx, n);
     L->psi = dalloc<double>(ctx, n);
     const int m = L->mmax;
-    const size_t ns = (size_t)m + (m + 1) + 2 * (m + 1) + 2 * (m + 1) + 4 + m + 4;
+    const int max_groups = m / DOT_GROUP + 2;  // vector groups of the dots, one arrival counter each
+    const size_t ns = (size_t)m + (m + 1) + 2 * (m + 1) + 2 * (m + 1) + 4 + m + 4 + (CNT_DOTS + max_groups + 1) / 2;
     L->scal = dalloc<double>(ctx, ns);
     BLQH_TRY_CUDA(ctx, cudaMemsetAsync(L->scal, 0, ns * 8, ctx->stream));
     double* p = L->scal;
@@ -1514,36 +1143,47 @@ blqh_lanczos* create_impl(blqh_ctx* ctx, const blqh_csr* M, const blqh_lanczos_o
     L->S.ritz = p;
     p += m;
     L->S.flags = reinterpret_cast<int*>(p);
+    p += 4;
+    L->S.cnt = reinterpret_cast<unsigned*>(p);
+    // short tiles spread small sectors over more blocks
+    L->tile = n <= 65536 ? 256 : 1024;
+    L->ntile = (int)((n + L->tile - 1) / L->tile);
+    L->pld = (int64_t)L->ntile * L->tile;
     L->nblk_dot = (int)((L->dim + GS_ROWS - 1) / GS_ROWS);
-    L->nblk_upd = (int)((L->dim + UPD_THREADS - 1) / UPD_THREADS);
-    L->part = dalloc<double>(ctx, (size_t)L->nblk_dot * (m + 1) * 2);
-    // block partials of the dot, update and norm kernels, and of k_rq_res (at most 8 blocks per SM)
-    L->pnorm = dalloc<double>(ctx, std::max<int64_t>(std::max<int64_t>(std::max(L->nblk_dot, L->nblk_upd),
-                                                                       (L->dim + 255) / 256),
-                                                     (int64_t)ctx->num_sms * 8) +
-                                       1024);
+    L->nblk_upd = (int)((L->dim + 255) / 256);
+    L->part = dalloc<double>(ctx, (size_t)std::max(L->nblk_dot, L->ntile) * (m + 1) * 2);
+    // block partials: at most one per 256 rows, or 8 per SM
+    L->pnorm = dalloc<double>(ctx, std::max<int64_t>((n + 255) / 256, (int64_t)ctx->num_sms * 8) + 1024);
+    L->apart = dalloc<double2>(ctx, std::max((size_t)L->nblk_dot, (size_t)ctx->num_sms * 2));
+    L->npart = dalloc<double>(ctx, L->ntile);
     L->work = dalloc<double>(ctx, 8 * (size_t)m + 16);
     L->y = dalloc<double>(ctx, m + 1);
     if (M->precision == BLQH_VAL_FP32 && o.accumulate == 0) L->xs = dalloc<float2>(ctx, n + 2);
-    if (M->precision == BLQH_VAL_FP32 && o.accumulate == 0 && o.reorth && gs_planes_enabled()) {
-      // the planes double the Krylov basis' memory; without room for them the
-      // run keeps the FP64 Gram-Schmidt kernels
-      const int64_t pld = (n + 3) & ~(int64_t)3;
+    if (o.reorth && gs_planes_enabled()) {
+      // the planes take up to the Krylov basis' memory again; without room for
+      // them the run works on the FP64 vectors
       try {
-        L->Vh = dalloc<float>(ctx, (size_t)(L->mmax + 1) * pld);
-        L->Vl = dalloc<float>(ctx, (size_t)(L->mmax + 1) * pld);
+        if (L->cplx) {
+          const size_t rows = (size_t)m + 2;
+          L->Q1 = dalloc<int>(ctx, rows * L->pld);
+          L->Q0 = dalloc<int>(ctx, rows * L->pld);
+          L->QE = dalloc<int>(ctx, rows * L->ntile);
+        } else {
+          L->vld = (n + 3) & ~(int64_t)3;
+          L->Vh = dalloc<float>(ctx, (size_t)(m + 1) * L->vld);
+          if (M->precision == BLQH_VAL_FP32 && o.accumulate == 0) {
+            L->Vl = dalloc<float>(ctx, (size_t)(m + 1) * L->vld);
+            L->nblk_upd = (int)((n + 1023) / 1024);
+          }
+        }
       } catch (const BlqhError& e) {
         if (e.code != BLQH_ERR_NOMEM) throw;
+        dev_free(L->Q1);
+        dev_free(L->Q0);
         dev_free(L->Vh);
-        dev_free(L->Vl);
+        L->Q1 = L->Q0 = L->QE = nullptr;
         L->Vh = L->Vl = nullptr;
         ctx->last_error.clear();
-      }
-      if (L->Vh) {
-        L->pld = pld;
-        BLQH_TRY_CUDA(ctx, cudaMemsetAsync(L->Vh, 0, (size_t)(L->mmax + 1) * pld * sizeof(float), ctx->stream));
-        BLQH_TRY_CUDA(ctx, cudaMemsetAsync(L->Vl, 0, (size_t)(L->mmax + 1) * pld * sizeof(float), ctx->stream));
-        L->nblk_upd = (int)((n + 4 * UPD_THREADS - 1) / (4 * UPD_THREADS));
       }
     }
     tune_spmv(L);

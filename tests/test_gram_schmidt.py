@@ -1,0 +1,72 @@
+"""The Lanczos step's Gram-Schmidt passes: fixed-point planes (complex sectors) and the ordered FP64 / FP32-plane
+passes (real sectors), against the FP64 pass on the stored vectors and a dense diagonalization of the same matrix.
+
+Sizes sit at the edges of the tiles: vectors shorter than one 256-double tile, one entry short of and past tile
+borders, and beyond the 65,536 doubles where 1024-double tiles take over."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SECTORS = [  # (nphi, nel, nel_up, J, K): dimension 11 .. 60,096, complex and real
+    (6, 6, 3, 1, 2), (8, 8, 4, 0, 1), (8, 7, -1, 3, 1), (10, 10, 5, 0, 3), (10, 9, 4, 3, 2), (12, 12, 6, 3, 5),
+    (14, 14, 7, 0, 3), (8, 8, 4, 2, 0), (10, 10, 5, 5, 0), (12, 12, 6, 3, 0), (14, 14, 7, 3, 7),
+]
+
+
+@pytest.fixture(scope="module")
+def B():
+    import blqh_gb300
+
+    return blqh_gb300
+
+
+def _run(B, sec, prec, steps, d=0.9):
+    b = B.Basis(*sec)
+    H = B.Hamiltonian(b, d, precision=prec)
+    L = B.Lanczos(H, max_steps=steps, tol=0.0, seed=3)
+    m = L.iterate()
+    e, _ = L.eig()
+    psi = L.ritz_vector()
+    E = L.rayleigh()
+    a, be = L.coeffs()
+    res = np.linalg.norm(H.spmv(psi) - E * psi)
+    out = dict(m=m, e=e, psi=psi, E=E, a=a, b=be, res=res, dim=H.dim)
+    if H.dim <= 700:
+        rp, col, val = H.csr()
+        D = np.zeros((H.dim, H.dim), val.dtype)
+        D[np.repeat(np.arange(H.dim), np.diff(rp)), col] = val
+        out["dense"] = np.linalg.eigvalsh((D + D.conj().T) / 2)
+    for x in (L, H, b):
+        x.close()
+    return out
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+@pytest.mark.parametrize("sec", SECTORS, ids=str)
+def test_against_fp64_pass(B, monkeypatch, sec, prec):
+    """Same recurrence as the FP64 pass: the first coefficients to 1e-11 (rounding times the growth of 15 steps),
+    the lowest Ritz value of 120 steps to 1e-12 of its size (FP32 values: the pass's own 2^-46), residual of the
+    ground state as small as the FP64 pass's."""
+    p = B.VAL_FP64 if prec == "f64" else B.VAL_FP32
+    r = _run(B, sec, p, 120)
+    monkeypatch.setenv("BLQH_GS_FP64", "1")
+    f = _run(B, sec, p, 120)
+    k = min(15, r["m"], f["m"], r["dim"] // 2)
+    assert np.max(np.abs(r["a"][:k] - f["a"][:k])) < 1e-11
+    assert np.max(np.abs(r["b"][:k] - f["b"][:k])) < 1e-11
+    assert abs(r["e"][0] - f["e"][0]) < 1e-12 * max(1.0, abs(f["e"][0]))
+    assert r["res"] <= 2 * f["res"] + 1e-11
+    if "dense" in r:
+        assert abs(r["e"][0] - r["dense"][0]) < 1e-11
+
+
+@pytest.mark.parametrize("sec", [s for s in SECTORS if s[:2] in ((6, 6), (8, 8))], ids=str)
+def test_exhausted_krylov_space(B, sec):
+    """As many steps as the sector has states: the run ends at an invariant subspace (the coefficients of the full
+    pass are then not small and it subtracts in FP64), without copies of the ground level."""
+    r = _run(B, sec, B.VAL_FP64, 400)
+    assert r["m"] <= r["dim"]
+    assert abs(r["e"][0] - r["dense"][0]) < 1e-11
+    assert np.sum(np.abs(r["e"] - r["dense"][0]) < 1e-9) == np.sum(np.abs(r["dense"] - r["dense"][0]) < 1e-9) or \
+        np.sum(np.abs(r["e"] - r["dense"][0]) < 1e-9) == 1
