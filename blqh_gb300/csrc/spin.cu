@@ -32,12 +32,25 @@
 // sorted by column. No sector-size limit. Values are FP64 (the accumulation
 // order differs from the reference's by the threads' atomics: values agree to
 // rounding); FP32 values are the FP64 sums rounded once.
+//
+// Work per row. Only the row's occupied pairs are walked (28 at Ne = 8, not every
+// pair of 32 orbitals), each target is looked up once in the orbit-member table
+// (members.cuh), and for even nphi the hop operator commutes with the signed
+// translations (the empty-orbital parities then equal the occupied ones up to one
+// common sign per family), so the untranslated row state stands for all Dl
+// translates: the sum over them is Dl times one phase when the target orbit
+// carries momentum K, an explicit signed sum otherwise (short orbits). Odd nphi, a
+// twist theta_x (the tables are read at |mt - n|, which a wrapped translate turns
+// into nphi - |mt - n|) and a parallel-field phase with tunnelling are not
+// translation covariant and enumerate every translate. Rows are generated once, into a staging buffer, and
+// compacted after the scan. Bound by issue and shared-memory latency: Nphi = 8,
+// 16,024 states, K = 3: 257 -> 1.0 ms.
 #include <algorithm>
 #include <cmath>
 #include <string>
 #include <vector>
 
-#include "blqh_internal.h"
+#include "members.cuh"
 
 namespace {
 
@@ -156,13 +169,25 @@ __global__ void k_spin_period(const uint64_t* __restrict__ ids, int64_t dim, int
 }
 
 // ---- Hamiltonian --------------------------------------------------------------
+struct SpinRot {
+  int nphi;
+  __device__ uint64_t operator()(uint64_t c, int k) const {
+    int p;
+    return rot4(c, k, nphi, 0, &p);
+  }
+};
+
 struct SpinGen {
   const uint64_t* id;
   const uint8_t* period;
   int64_t dim;
   int nphi, nel, K;
+  int literal;       // 1: enumerate every translation of the row state
   double Ec, d, dsas, dv, dz, theta_b, theta_y;
-  const double* V;  // [2][nphi][nphi]
+  const double* V;   // [2][nphi][nphi]
+  const double2* FT; // [2 nphi - 1]: (cos, sin)(2 pi m K / nphi), m = -(nphi - 1) .. nphi - 1; (1, 0) for K <= 0
+  const double* isq; // [16][16]: 1 / sqrt(Dl Dr)
+  MemberTable mem;
 };
 
 // Parity of the empty orbitals of c strictly between a and b (a < b): get_sign(c, n, nt), basis.cpp:187-197.
@@ -184,11 +209,6 @@ __device__ __forceinline__ int pair_parity(uint64_t c, int n, int m, int nt, int
   if ((nt > mt && m > n) || (mt > nt && m < n)) ns++;
   return ns & 1;
 }
-
-// The ten two-body families in the reference's order: block of n, block of m,
-// n < m within one block, interlayer table, twist phase.
-__constant__ int c_fam[10][5] = {{0, 0, 1, 0, 0}, {1, 1, 1, 0, 0}, {0, 1, 0, 0, 0}, {2, 2, 1, 0, 0}, {3, 3, 1, 0, 0},
-                                 {2, 3, 0, 0, 0}, {0, 2, 0, 1, 0}, {1, 3, 0, 1, 0}, {0, 3, 0, 1, 1}, {1, 2, 0, 1, 1}};
 
 // A row under construction: open-addressing table in shared memory.
 struct RowTable {
@@ -214,60 +234,97 @@ __device__ __forceinline__ int table_slot(const RowTable& T, int j) {
   return -1;
 }
 
-__device__ __forceinline__ void cadd(const RowTable& T, int64_t j, double re, double im) {
-  const int h = table_slot(T, (int)j);
-  if (h < 0) return;
-  atomicAdd(T.acc + 2 * h, re);
-  atomicAdd(T.acc + 2 * h + 1, im);
+// Sum over the translates of a row state (period Dl) of sign * FT for a target
+// reached from the untranslated state, whose orbit (period Dr) has its
+// representative qr translations away: (re, im) without 1 / sqrt(Dl Dr).
+__device__ __forceinline__ double2 translate_sum(const SpinGen& G, uint64_t rb0, int qr, int Dl, int Dr) {
+  int par;
+  if (G.K < 0) return make_double2(1.0, 0.0);
+  bool coherent = Dr == G.nphi;
+  if (!coherent) {  // T^Dr on the orbit's states: sign times e^{2 pi i K Dr / nphi} = 1?
+    rot4(rb0, Dr, G.nphi, 0, &par);
+    coherent = (2 * G.K * Dr + par * G.nphi) % (2 * G.nphi) == 0;
+  }
+  if (coherent) {
+    rot4(rb0, qr, G.nphi, 1, &par);
+    const double2 f = G.FT[G.nphi - 1 - qr];
+    const double s = (qr && par) ? -(double)Dl : (double)Dl;
+    return make_double2(s * f.x, s * f.y);
+  }
+  double2 g = make_double2(0.0, 0.0);
+  for (int q = 0; q < Dl; q++) {
+    int p1 = 0, p2 = 0;
+    const uint64_t y = q ? rot4(rb0, q, G.nphi, 0, &p1) : rb0;
+    const int q2 = (qr + q) % Dr;
+    if (q2) rot4(y, q2, G.nphi, 1, &p2);
+    const double2 f = G.FT[G.nphi - 1 + q - q2];
+    const double s = ((p1 + p2) & 1) ? -1.0 : 1.0;
+    g.x += s * f.x;
+    g.y += s * f.y;
+  }
+  return g;
 }
 
 // Adds the contribution of target rbasis_0 (before the right-hand translations) to the row.
-__device__ void add_target(const SpinGen& G, const RowTable& acc, uint64_t rb0, int ql, int Dl, int parl, int parh,
-                           double amp_re, double amp_im) {
-  int Dr = G.nphi;
-  for (int D = 1; D < G.nphi; D++) {
-    int p;
-    if (rot4(rb0, D, G.nphi, 0, &p) == rb0) {
-      Dr = D;
-      break;
-    }
-  }
-  if (G.K < 0) Dr = 1;
-  for (int qr = 0; qr < Dr; qr++) {
+template <bool CPLX>
+__device__ __forceinline__ void add_target(const SpinGen& G, const RowTable& T, uint64_t rb0, int ql, int Dl, int parl,
+                                           int parh, double amp_re, double amp_im) {
+  uint32_t mv;
+  if (!member_find(G.mem, rb0, &mv)) return;
+  const int j = (int)(mv >> 5), qr = (int)(mv & 31);
+  const int Dr = G.K < 0 ? 1 : G.period[j];
+  double2 f;
+  if (G.literal) {
     int parr = 0;
-    const uint64_t rb = qr == 0 ? rb0 : rot4(rb0, qr, G.nphi, 1, &parr);
-    const int64_t j = find_key(G.id, G.dim, rb);
-    if (j < 0) continue;
-    const double sign = ((parh + parl + parr) & 1) ? -1.0 : 1.0;
-    // FT[ql][qr] = exp(2 pi i (ql - qr) K / nphi)
-    double fr = 1.0, fi = 0.0;
-    if (G.K > 0) {
-      const double ang = 2.0 * M_PI * (ql - qr) * G.K / G.nphi;
-      fr = cos(ang);
-      fi = sin(ang);
-    }
-    const double f = sign / sqrt((double)(Dl * Dr));
-    cadd(acc, j, (amp_re * fr - amp_im * fi) * f, (amp_re * fi + amp_im * fr) * f);
+    if (qr) rot4(rb0, qr, G.nphi, 1, &parr);
+    f = G.FT[G.nphi - 1 + ql - qr];
+    if ((parl + parr) & 1) f = make_double2(-f.x, -f.y);
+  } else {
+    f = translate_sum(G, rb0, qr, Dl, Dr);
   }
+  const double c = __ldg(G.isq + (Dl - 1) * 16 + (Dr - 1)) * (parh ? -1.0 : 1.0);
+  const int h = table_slot(T, j);
+  if (h < 0) return;
+  atomicAdd(T.acc + 2 * h, (CPLX ? amp_re * f.x - amp_im * f.y : amp_re * f.x) * c);
+  if (CPLX) atomicAdd(T.acc + 2 * h + 1, (amp_re * f.y + amp_im * f.x) * c);
+}
+
+// |value| > 1e-10 (the squared norm settles all but values within 1e-7 of the threshold).
+__device__ __forceinline__ bool kept(double re, double im) {
+  const double q = re * re + im * im;
+  return q > 1.0000001e-20 || (q >= 0.9999999e-20 && sqrt(q) > 1e-10);
+}
+
+// Orbital of the k-th (0-based) electron of c.
+__device__ __forceinline__ int nth_bit(uint64_t c, int k) {
+  for (int i = 0; i < k; i++) c &= c - 1;
+  return __ffsll((long long)c) - 1;
 }
 
 // Per row: all candidates accumulate into the row's table; its occupied slots
 // are sorted by column (bitonic, in shared memory); pass 0 counts kept entries,
-// pass 1 writes them at row_ptr (ascending columns); pass 2 (regenerated
-// Rayleigh quotient) writes rq_part[i] = Re(conj(psi_i) sum_k H_ik psi_k) over
-// the row's kept entries in column order, FP64, nothing stored.
-__global__ void __launch_bounds__(256) k_spin_rows(SpinGen G, int pass, int slots, int64_t* __restrict__ row_nnz,
-                                                   const int64_t* __restrict__ row_ptr, int32_t* __restrict__ col,
-                                                   double* __restrict__ val, int cplx, int* overflow,
-                                                   const double* __restrict__ psi, double* __restrict__ rq_part) {
+// pass 1 writes them at row_ptr (ascending columns), pass 3 does both at once into
+// a staging buffer (row i at i * stride); pass 2 (regenerated Rayleigh quotient)
+// writes rq_part[i] = Re(conj(psi_i) sum_k H_ik psi_k) over the row's kept entries
+// in column order, FP64, nothing stored.
+constexpr int SPIN_THREADS = 128;
+
+template <bool CPLX>
+__global__ void __launch_bounds__(SPIN_THREADS)
+    k_spin_rows(SpinGen G, int pass, int slots, int64_t stride, int64_t* __restrict__ row_nnz,
+                const int64_t* __restrict__ row_ptr, int32_t* __restrict__ col, double* __restrict__ val, int* overflow,
+                const double* __restrict__ psi, double* __restrict__ rq_part) {
   extern __shared__ __align__(16) unsigned char sm_raw[];
   RowTable acc{reinterpret_cast<int*>(sm_raw + (size_t)slots * 16), reinterpret_cast<double*>(sm_raw), slots,
                overflow};
   int2* order = reinterpret_cast<int2*>(sm_raw + (size_t)slots * 20);  // [slots] (column, slot)
   __shared__ int n_occ;
-  const int nphi = G.nphi;
+  const int nphi = G.nphi, nel = G.nel;
+  const int nt_range = 2 * nphi - 1, hop_items = nel * (nel - 1) / 2 * nt_range;
+  const int tun_items = G.dsas > 0 ? 6 * nphi : 0;
+  const int per_ql = hop_items + tun_items;
   for (int64_t i = blockIdx.x; i < G.dim; i += gridDim.x) {
-    for (int k = threadIdx.x; k < slots; k += blockDim.x) {
+    for (int k = threadIdx.x; k < slots; k += SPIN_THREADS) {
       acc.keys[k] = -1;
       acc.acc[2 * k] = acc.acc[2 * k + 1] = 0.0;
     }
@@ -275,60 +332,43 @@ __global__ void __launch_bounds__(256) k_spin_rows(SpinGen G, int pass, int slot
     __syncthreads();
     const uint64_t idi = G.id[i];
     const int Dl = G.K < 0 ? 1 : G.period[i];
-    const int npair_same = nphi * (nphi - 1) / 2, npair_cross = nphi * nphi, nt_range = 2 * nphi - 1;
-    const int hop_items = (4 * npair_same + 6 * npair_cross) * nt_range;
-    const int tun_items = G.dsas > 0 ? 6 * nphi : 0;
-    const int per_ql = hop_items + tun_items;
-    for (int it = threadIdx.x; it < Dl * per_ql; it += blockDim.x) {
+    const int nql = G.literal ? Dl : 1;
+    for (int it = threadIdx.x; it < nql * per_ql; it += SPIN_THREADS) {
       const int ql = it / per_ql;
       int w = it - ql * per_ql;
       int parl = 0;
       const uint64_t lb = ql == 0 ? idi : rot4(idi, ql, nphi, 0, &parl);
       if (w < hop_items) {
-        // family, pair, t
-        int f = 0;
-        for (; f < 10; f++) {
-          const int np = (c_fam[f][2] ? npair_same : npair_cross) * nt_range;
-          if (w < np) break;
-          w -= np;
-        }
+        // occupied pair n < m (the reference's ten families: two electrons of one
+        // block, or of two blocks; within a layer the intralayer table, between
+        // layers the interlayer one, with the twist phase for opposite spins), t
         const int ti = w % nt_range, pi = w / nt_range;
         const int t = ti - (nphi - 1);
-        const int ba = c_fam[f][0], bb = c_fam[f][1];
-        int n, m;
-        if (c_fam[f][2]) {
-          // pi-th pair (a < b) of one block, in the reference's loop order
-          int a = 0, r = pi;
-          while (r >= nphi - 1 - a) {
-            r -= nphi - 1 - a;
-            a++;
-          }
-          n = ba * nphi + a;
-          m = ba * nphi + a + 1 + r;
-        } else {
-          n = ba * nphi + pi / nphi;
-          m = bb * nphi + pi % nphi;
+        int a = 0, r = pi;
+        while (r >= nel - 1 - a) {
+          r -= nel - 1 - a;
+          a++;
         }
-        const uint64_t mask = (1ULL << n) | (1ULL << m);
-        if ((lb & mask) != mask) continue;
-        const uint64_t b = lb ^ mask;
+        const int n = nth_bit(lb, a), m = nth_bit(lb, a + 1 + r);
+        const int ba = n / nphi, bb = m / nphi;
+        const int inter = (ba >> 1) != (bb >> 1);
+        const uint64_t b = lb ^ ((1ULL << n) | (1ULL << m));
         const int offa = ba * nphi, offb = bb * nphi;
         int nt = n + t, mt = m - t;
         if (nt >= offa + nphi) nt -= nphi;
         else if (nt < offa) nt += nphi;
         if (mt < offb) mt += nphi;
         else if (mt >= offb + nphi) mt -= nphi;
-        const int s = abs((mt - offb) - (n - offa));
         const uint64_t mt_mask = (1ULL << nt) | (1ULL << mt);
-        if ((mt_mask & b) != 0) continue;
-        if (!c_fam[f][3] && nt == mt) continue;
-        const double v = G.V[c_fam[f][3] * nphi * nphi + s * nphi + abs(t)];
+        if (nt == mt || (mt_mask & b) != 0) continue;
+        const int s = abs((mt - offb) - (n - offa));
+        const double v = __ldg(G.V + inter * nphi * nphi + s * nphi + abs(t));
         double are = v, aim = 0.0;
-        if (c_fam[f][4] && G.theta_y != 0.0) {
+        if (CPLX && inter && (ba & 1) != (bb & 1) && G.theta_y != 0.0) {
           are = v * cos(G.theta_y * t / nphi);
           aim = v * sin(G.theta_y * t / nphi);
         }
-        add_target(G, acc, mt_mask + b, ql, Dl, parl, pair_parity(lb, n, m, nt, mt), are, aim);
+        add_target<CPLX>(G, acc, mt_mask | b, ql, Dl, parl, pair_parity(lb, n, m, nt, mt), are, aim);
       } else {
         w -= hop_items;
         const int kind = w / nphi, r = w % nphi;
@@ -347,7 +387,9 @@ __global__ void __launch_bounds__(256) k_spin_rows(SpinGen G, int pass, int slot
         const uint64_t kn = mask & lb;
         if (kn == mask || kn == 0) continue;
         const uint64_t rb0 = lb - kn + (kn ^ mask);
-        add_target(G, acc, rb0, ql, Dl, parl, empties_between(lb, lo, hi), amp * cos(ph), amp * sin(ph));
+        double cr = 1.0, ci = 0.0;
+        if (CPLX && ph != 0.0) sincos(ph, &ci, &cr);
+        add_target<CPLX>(G, acc, rb0, ql, Dl, parl, empties_between(lb, lo, hi), amp * cr, amp * ci);
       }
     }
     __syncthreads();
@@ -367,17 +409,17 @@ __global__ void __launch_bounds__(256) k_spin_rows(SpinGen G, int pass, int slot
     }
     __syncthreads();
     // occupied slots, sorted by column
-    for (int k = threadIdx.x; k < slots; k += blockDim.x)
+    for (int k = threadIdx.x; k < slots; k += SPIN_THREADS)
       if (acc.keys[k] >= 0) order[atomicAdd(&n_occ, 1)] = make_int2(acc.keys[k], k);
     __syncthreads();
     const int n = n_occ;
     int P = 1;
     while (P < n) P <<= 1;
-    for (int k = n + threadIdx.x; k < P; k += blockDim.x) order[k] = make_int2(0x7FFFFFFF, -1);
+    for (int k = n + threadIdx.x; k < P; k += SPIN_THREADS) order[k] = make_int2(0x7FFFFFFF, -1);
     __syncthreads();
     for (int k = 2; k <= P; k <<= 1)
       for (int jj = k >> 1; jj > 0; jj >>= 1) {
-        for (int t = threadIdx.x; t < P; t += blockDim.x) {
+        for (int t = threadIdx.x; t < P; t += SPIN_THREADS) {
           const int u = t ^ jj;
           if (u > t) {
             const int2 a = order[t], b = order[u];
@@ -397,8 +439,8 @@ __global__ void __launch_bounds__(256) k_spin_rows(SpinGen G, int pass, int slot
         if (k < n) {
           const int c = order[k].x;
           const double re = acc.acc[2 * order[k].y], im = acc.acc[2 * order[k].y + 1];
-          if (sqrt(re * re + im * im) > 1e-10) {
-            const double xr = cplx ? psi[2 * (int64_t)c] : psi[c], xi = cplx ? psi[2 * (int64_t)c + 1] : 0.0;
+          if (kept(re, im)) {
+            const double xr = CPLX ? psi[2 * (int64_t)c] : psi[c], xi = CPLX ? psi[2 * (int64_t)c + 1] : 0.0;
             sr += re * xr - im * xi;
             si += re * xi + im * xr;
           }
@@ -409,12 +451,13 @@ __global__ void __launch_bounds__(256) k_spin_rows(SpinGen G, int pass, int slot
         si += __shfl_xor_sync(0xffffffffu, si, o);
       }
       if (lane == 0) {
-        const double pr = cplx ? psi[2 * i] : psi[i], pim = cplx ? psi[2 * i + 1] : 0.0;
+        const double pr = CPLX ? psi[2 * i] : psi[i], pim = CPLX ? psi[2 * i + 1] : 0.0;
         rq_part[i] = pr * sr + pim * si;  // Re(conj(psi_i) s)
       }
     } else if (threadIdx.x < 32) {
       // kept entries in ascending column order: count (warp ballots) or write
-      int64_t out = pass ? row_ptr[i] : 0;
+      const int64_t base = pass == 3 ? i * stride : pass ? row_ptr[i] : 0;
+      int64_t out = base;
       for (int k0 = 0; k0 < n; k0 += 32) {
         const int k = k0 + lane;
         bool keep = false;
@@ -424,13 +467,13 @@ __global__ void __launch_bounds__(256) k_spin_rows(SpinGen G, int pass, int slot
           c = order[k].x;
           re = acc.acc[2 * order[k].y];
           im = acc.acc[2 * order[k].y + 1];
-          keep = sqrt(re * re + im * im) > 1e-10;
+          keep = kept(re, im);
         }
         const unsigned bal = __ballot_sync(0xffffffffu, keep);
         if (pass && keep) {
           const int64_t o = out + __popc(bal & ((1u << lane) - 1));
           col[o] = (int32_t)c;
-          if (cplx) {
+          if (CPLX) {
             val[2 * o] = re;
             val[2 * o + 1] = im;
           } else {
@@ -439,7 +482,7 @@ __global__ void __launch_bounds__(256) k_spin_rows(SpinGen G, int pass, int slot
         }
         out += __popc(bal);
       }
-      if (!pass && lane == 0) row_nnz[i] = out;
+      if (pass != 1 && lane == 0) row_nnz[i] = out - base;
     }
     __syncthreads();
   }
@@ -463,75 +506,75 @@ __global__ void __launch_bounds__(256) k_spin_rows(SpinGen G, int pass, int slot
 // [4 + 2 p .. 5 + 2 p] M of move pair p (re, im), [20 ..] occupations (block 0, then 1).
 __constant__ int c_move_pairs[8][2] = {{0, 2}, {2, 0}, {1, 3}, {3, 1}, {0, 3}, {3, 0}, {1, 2}, {2, 1}};
 
+// One warp per state: for each move pair the lanes take (translate, orbital), the
+// target's representative comes from the orbit-member table.
 __global__ void __launch_bounds__(256) k_spin_observables(const uint64_t* __restrict__ id,
-                                                          const uint8_t* __restrict__ period, int64_t dim, int nphi,
-                                                          int K, const double* __restrict__ psi, int cplx,
+                                                          const uint8_t* __restrict__ period, MemberTable mem,
+                                                          const double2* __restrict__ FT,
+                                                          const double* __restrict__ isq, int64_t dim, int nphi, int K,
+                                                          const double* __restrict__ psi, int cplx,
                                                           double* __restrict__ part) {
   __shared__ double acc[20 + 2 * 15];
   const int nv = 20 + 2 * nphi;
   for (int k = threadIdx.x; k < nv; k += blockDim.x) acc[k] = 0.0;
   __syncthreads();
   const uint64_t mk = (1ULL << nphi) - 1;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < dim; i += (int64_t)gridDim.x * blockDim.x) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < dim; i += warps) {
     const double pr = cplx ? psi[2 * i] : psi[i], pim = cplx ? psi[2 * i + 1] : 0.0;
     const double w = pr * pr + pim * pim;
     const uint64_t idi = id[i];
-    const int n0 = pc64(idi & mk), n1 = pc64((idi >> nphi) & mk), n2 = pc64((idi >> (2 * nphi)) & mk),
-              n3 = pc64((idi >> (3 * nphi)) & mk);
-    atomicAdd(acc + 0, (n0 + n1) * w);
-    atomicAdd(acc + 1, (n0 + n2) * w);
-    atomicAdd(acc + 2, (2.0 * n0 - (n0 + n1)) / (2.0 * (n0 + n1) + 1e-8) * w);
-    atomicAdd(acc + 3, (2.0 * n2 - (n2 + n3)) / (2.0 * (n2 + n3) + 1e-8) * w);
     const int Dl = K < 0 ? 1 : period[i];
-    double mr[8], mi[8];
-    for (int p = 0; p < 8; p++) mr[p] = mi[p] = 0.0;
-    for (int ql = 0; ql < Dl; ql++) {
-      int parl = 0;
-      const uint64_t lb = ql == 0 ? idi : rot4(idi, ql, nphi, 0, &parl);
-      for (int j = 0; j < nphi; j++) {
-        if ((lb >> j) & 1) atomicAdd(acc + 20 + j, w / Dl);
-        if ((lb >> (j + nphi)) & 1) atomicAdd(acc + 20 + nphi + j, w / Dl);
-      }
-      for (int p = 0; p < 8; p++) {
-        for (int o = 0; o < nphi; o++) {
-          const int n = c_move_pairs[p][0] * nphi + o, nt = c_move_pairs[p][1] * nphi + o;
-          const uint64_t mask = (1ULL << n) | (1ULL << nt);
-          const uint64_t kn = lb & mask;
-          if (kn == mask || kn == 0) continue;
-          const uint64_t rb0 = lb ^ mask;
-          int Dr = nphi;
-          for (int D = 1; D < nphi; D++) {
-            int q;
-            if (rot4(rb0, D, nphi, 0, &q) == rb0) {
-              Dr = D;
-              break;
-            }
-          }
-          if (K < 0) Dr = 1;
-          const int hpar = empties_between(lb, n < nt ? n : nt, n < nt ? nt : n);
-          for (int qr = 0; qr < Dr; qr++) {
-            int parr = 0;
-            const uint64_t rb = qr == 0 ? rb0 : rot4(rb0, qr, nphi, 1, &parr);
-            const int64_t jj = find_key(id, dim, rb);
-            if (jj < 0) continue;
-            const double qr_ = cplx ? psi[2 * jj] : psi[jj], qi_ = cplx ? -psi[2 * jj + 1] : 0.0;  // conj(psi_j)
-            const double cr = pr * qr_ - pim * qi_, ci = pr * qi_ + pim * qr_;                      // psi_i conj(psi_j)
-            double fr = 1.0, fi = 0.0;
-            if (K > 0) {
-              const double ang = 2.0 * M_PI * (ql - qr) * K / nphi;
-              fr = cos(ang);
-              fi = sin(ang);
-            }
-            const double f = (((hpar + parl + parr) & 1) ? -1.0 : 1.0) / sqrt((double)(Dl * Dr));
-            mr[p] += (cr * fr - ci * fi) * f;
-            mi[p] += (cr * fi + ci * fr) * f;
-          }
-        }
-      }
+    if (lane == 0) {
+      const int n0 = pc64(idi & mk), n1 = pc64((idi >> nphi) & mk), n2 = pc64((idi >> (2 * nphi)) & mk),
+                n3 = pc64((idi >> (3 * nphi)) & mk);
+      atomicAdd(acc + 0, (n0 + n1) * w);
+      atomicAdd(acc + 1, (n0 + n2) * w);
+      atomicAdd(acc + 2, (2.0 * n0 - (n0 + n1)) / (2.0 * (n0 + n1) + 1e-8) * w);
+      atomicAdd(acc + 3, (2.0 * n2 - (n2 + n3)) / (2.0 * (n2 + n3) + 1e-8) * w);
+    }
+    if (lane < 2 * nphi) {  // orbital `lane` of blocks 0 and 1 over the translates
+      const int b = lane / nphi, o = lane - b * nphi;
+      const uint64_t x = (idi >> (b * nphi)) & mk;
+      int c = 0;
+      for (int ql = 0; ql < Dl; ql++) c += (int)((x >> ((o - ql + nphi) % nphi)) & 1);
+      if (c) atomicAdd(acc + 20 + lane, c * (w / Dl));
     }
     for (int p = 0; p < 8; p++) {
-      if (mr[p] != 0.0) atomicAdd(acc + 4 + 2 * p, mr[p]);
-      if (mi[p] != 0.0) atomicAdd(acc + 5 + 2 * p, mi[p]);
+      double mr = 0.0, mi = 0.0;
+      for (int it = lane; it < Dl * nphi; it += 32) {
+        const int ql = it / nphi, o = it - ql * nphi;
+        int parl = 0;
+        const uint64_t lb = ql == 0 ? idi : rot4(idi, ql, nphi, 0, &parl);
+        const int n = c_move_pairs[p][0] * nphi + o, nt = c_move_pairs[p][1] * nphi + o;
+        const uint64_t mask = (1ULL << n) | (1ULL << nt);
+        const uint64_t kn = lb & mask;
+        if (kn == mask || kn == 0) continue;
+        const uint64_t rb0 = lb ^ mask;
+        uint32_t mv;
+        if (!member_find(mem, rb0, &mv)) continue;
+        const int64_t jj = mv >> 5;
+        const int qr = (int)(mv & 31), Dr = K < 0 ? 1 : period[jj];
+        int parr = 0;
+        if (qr) rot4(rb0, qr, nphi, 1, &parr);
+        const int hpar = empties_between(lb, n < nt ? n : nt, n < nt ? nt : n);
+        const double qr_ = cplx ? psi[2 * jj] : psi[jj], qi_ = cplx ? -psi[2 * jj + 1] : 0.0;  // conj(psi_j)
+        const double cr = pr * qr_ - pim * qi_, ci = pr * qi_ + pim * qr_;                      // psi_i conj(psi_j)
+        const double2 ft = FT[nphi - 1 + ql - qr];
+        const double f = (((hpar + parl + parr) & 1) ? -1.0 : 1.0) * isq[(Dl - 1) * 16 + (Dr - 1)];
+        mr += (cr * ft.x - ci * ft.y) * f;
+        mi += (cr * ft.y + ci * ft.x) * f;
+      }
+      if (!__any_sync(0xffffffffu, mr != 0.0 || mi != 0.0)) continue;
+      for (int o = 16; o > 0; o >>= 1) {
+        mr += __shfl_xor_sync(0xffffffffu, mr, o);
+        mi += __shfl_xor_sync(0xffffffffu, mi, o);
+      }
+      if (lane == 0) {
+        atomicAdd(acc + 4 + 2 * p, mr);
+        atomicAdd(acc + 5 + 2 * p, mi);
+      }
     }
   }
   __syncthreads();
@@ -648,16 +691,46 @@ void build_spin_basis(blqh_ctx* ctx, blqh_basis* B) {
   BLQH_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
 }
 
+// Phases, 1 / sqrt(Dl Dr) and the orbit-member table of a basis.
+struct SpinTables {
+  const double2* FT = nullptr;
+  const double* isq = nullptr;
+  MemberTable mem{};
+};
+
+SpinTables spin_tables(blqh_ctx* ctx, const blqh_basis* B, DevBufs& G, int* derr) {
+  const blqh_sector_spin& s = B->ssector;
+  const int nphi = s.nphi;
+  std::vector<double> t(2 * (2 * nphi - 1) + 256);
+  for (int m = -(nphi - 1); m <= nphi - 1; m++) {
+    const double ang = 2.0 * M_PI * m * s.K / nphi;  // the reference's FT[ql][qr], m = ql - qr
+    t[2 * (m + nphi - 1)] = s.K > 0 ? cos(ang) : 1.0;
+    t[2 * (m + nphi - 1) + 1] = s.K > 0 ? sin(ang) : 0.0;
+  }
+  double* q = t.data() + 2 * (2 * nphi - 1);
+  for (int dl = 1; dl <= 16; dl++)
+    for (int dr = 1; dr <= 16; dr++) q[(dl - 1) * 16 + (dr - 1)] = 1.0 / sqrt((double)(dl * dr));
+  double* d = G.add(upload_vec(ctx, t));
+  SpinTables T;
+  T.FT = reinterpret_cast<const double2*>(d);
+  T.isq = d + 2 * (2 * nphi - 1);
+  T.mem = build_members(ctx, G, B, SpinRot{nphi}, s.K >= 0, nphi, derr);
+  return T;
+}
+
 // Row generator set-up shared by the build and the regenerated Rayleigh quotient.
 struct SpinSetup {
   SpinGen g{};
   bool cplx = false;
   int slots = 0;
+  int64_t stride = 0;  // a row's largest number of entries
   size_t smem = 0;
+  decltype(&k_spin_rows<true>) rows = nullptr;
   int grid = 0;
 };
 
-SpinSetup spin_setup(blqh_ctx* ctx, const blqh_basis* B, const blqh_params_spin& p, DevBufs& G) {
+// err: set when a table insert finds no free slot (never, by the sizing).
+SpinSetup spin_setup(blqh_ctx* ctx, const blqh_basis* B, const blqh_params_spin& p, DevBufs& G, int* derr) {
   const blqh_sector_spin& s = B->ssector;
   const int nphi = s.nphi;
   // interaction tables: the spinful table has cos((2 pi s - theta_x) q_x / nphi)
@@ -690,6 +763,12 @@ SpinSetup spin_setup(blqh_ctx* ctx, const blqh_basis* B, const blqh_params_spin&
   g.theta_b = p.theta_b;
   g.theta_y = p.theta_y;
   g.V = dV;
+  // translation covariance: see the file comment
+  g.literal = s.K >= 0 && (nphi % 2 == 1 || p.theta_x != 0.0 || (p.theta_b != 0.0 && p.delta_sas > 0));
+  const SpinTables T = spin_tables(ctx, B, G, derr);
+  g.FT = T.FT;
+  g.isq = T.isq;
+  g.mem = T.mem;
   // table slots: a power of two >= twice the distinct columns a row can have
   const int64_t moves = (int64_t)s.nel * (s.nel - 1) / 2 * (2 * nphi - 1) + 6 * nphi + 1;
   S.slots = 64;
@@ -702,8 +781,10 @@ SpinSetup spin_setup(blqh_ctx* ctx, const blqh_basis* B, const blqh_params_spin&
                                              " slots) exceeds shared memory (too many electrons)");
     throw BlqhError{BLQH_ERR_UNSUPPORTED, "spin row table"};
   }
-  BLQH_TRY_CUDA(ctx, smem_attr_at_least(k_spin_rows, (int)S.smem));
-  S.grid = (int)std::min<int64_t>(B->dim, (int64_t)ctx->num_sms * 8);
+  S.stride = moves;
+  S.rows = S.cplx ? k_spin_rows<true> : k_spin_rows<false>;
+  BLQH_TRY_CUDA(ctx, smem_attr_at_least(S.rows, (int)S.smem));
+  S.grid = (int)std::min<int64_t>(B->dim, (int64_t)ctx->num_sms * 16);
   return S;
 }
 
@@ -712,7 +793,7 @@ void check_overflow(blqh_ctx* ctx, const int* over) {
   BLQH_TRY_CUDA(ctx, cudaMemcpyAsync(&ov, over, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   BLQH_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   if (ov) {
-    set_error(ctx, BLQH_ERR_CAPACITY, "spinful row generator: a row had more distinct columns than its table");
+    set_error(ctx, BLQH_ERR_CAPACITY, "spinful model: a row or the orbit-member table had no free slot");
     throw BlqhError{BLQH_ERR_CAPACITY, "spin row table"};
   }
 }
@@ -722,20 +803,39 @@ __global__ void k_f64_to_f32(const double* __restrict__ a, float* __restrict__ b
     b[i] = (float)a[i];
 }
 
+// Staged rows (k_spin_rows pass 3) into the CSR: one warp per row.
+__global__ void k_spin_unstage(const int32_t* __restrict__ scol, const double* __restrict__ sval, int64_t stride,
+                               int vw, const int64_t* __restrict__ row_ptr, int64_t dim, int32_t* __restrict__ col,
+                               double* __restrict__ val) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < dim; i += warps) {
+    const int64_t o = row_ptr[i], n = row_ptr[i + 1] - o, src = i * stride;
+    for (int64_t k = lane; k < n; k += 32) col[o + k] = scol[src + k];
+    for (int64_t k = lane; k < n * vw; k += 32) val[o * vw + k] = sval[src * vw + k];
+  }
+}
+
 void build_spin_hamil(blqh_ctx* ctx, const blqh_basis* B, const blqh_params_spin& p, int prec, blqh_csr* M) {
   DevBufs G;
-  const SpinSetup S = spin_setup(ctx, B, p, G);
+  int* over = G.add(dalloc<int>(ctx, 1));
+  BLQH_TRY_CUDA(ctx, cudaMemsetAsync(over, 0, sizeof(int), ctx->stream));
+  const SpinSetup S = spin_setup(ctx, B, p, G, over);
   const int64_t dim = B->dim;
   const bool cplx = S.cplx;
+  const int vw = cplx ? 2 : 1;
   M->dim = dim;
   M->is_complex = cplx;
   M->precision = BLQH_VAL_FP64;
   M->d_row_ptr = dalloc<int64_t>(ctx, dim + 1);
-  int* over = G.add(dalloc<int>(ctx, 1));
-  BLQH_TRY_CUDA(ctx, cudaMemsetAsync(over, 0, sizeof(int), ctx->stream));
+  // rows are generated once into a staging buffer that holds any row when it fits
+  // in 8 GB, else twice (counted, then written)
+  const bool staged = (double)dim * S.stride * (4 + 8 * vw) <= 8.0 * (1ULL << 30);
+  int32_t* scol = staged ? G.add(dalloc<int32_t>(ctx, (size_t)dim * S.stride)) : nullptr;
+  double* sval = staged ? G.add(dalloc<double>(ctx, (size_t)dim * S.stride * vw)) : nullptr;
   TimerScope ts(ctx, TM_BUILD);
-  k_spin_rows<<<S.grid, 256, S.smem, ctx->stream>>>(S.g, 0, S.slots, M->d_row_ptr, nullptr, nullptr, nullptr, cplx,
-                                                    over, nullptr, nullptr);
+  S.rows<<<S.grid, SPIN_THREADS, S.smem, ctx->stream>>>(S.g, staged ? 3 : 0, S.slots, S.stride, M->d_row_ptr, nullptr,
+                                                        scol, sval, over, nullptr, nullptr);
   BLQH_TRY_CUDA(ctx, cudaGetLastError());
   int64_t nnz = 0;
   scan_exclusive_i64(ctx, M->d_row_ptr, M->d_row_ptr, dim, &nnz);
@@ -744,8 +844,13 @@ void build_spin_hamil(blqh_ctx* ctx, const blqh_basis* B, const blqh_params_spin
   M->mean_row = dim ? (double)nnz / dim : 0;
   M->d_col = dalloc<int32_t>(ctx, std::max<int64_t>(1, nnz));
   M->d_val = dev_alloc(ctx, std::max<int64_t>(1, nnz) * (cplx ? 16 : 8) + 16);
-  k_spin_rows<<<S.grid, 256, S.smem, ctx->stream>>>(S.g, 1, S.slots, nullptr, M->d_row_ptr, M->d_col,
-                                                    reinterpret_cast<double*>(M->d_val), cplx, over, nullptr, nullptr);
+  double* val = reinterpret_cast<double*>(M->d_val);
+  if (staged)
+    k_spin_unstage<<<grid_for(ctx, dim * 32, 256), 256, 0, ctx->stream>>>(scol, sval, S.stride, vw, M->d_row_ptr, dim,
+                                                                          M->d_col, val);
+  else
+    S.rows<<<S.grid, SPIN_THREADS, S.smem, ctx->stream>>>(S.g, 1, S.slots, S.stride, nullptr, M->d_row_ptr, M->d_col,
+                                                          val, over, nullptr, nullptr);
   BLQH_TRY_CUDA(ctx, cudaGetLastError());
   count_launch(ctx, TM_BUILD, 2);
   check_overflow(ctx, over);
@@ -768,22 +873,22 @@ void build_spin_hamil(blqh_ctx* ctx, const blqh_basis* B, const blqh_params_spin
 // (the reference's order), out[6 .. 6 + 2 nphi) = occupations (alpha 0, then 1).
 void spin_observables_impl(blqh_ctx* ctx, const blqh_basis* B, const double* psi, int cplx, double* out) {
   const int nphi = B->ssector.nphi, nel = B->ssector.nel, nv = 20 + 2 * nphi;
-  const int grid = grid_for(ctx, B->dim, 256, 4);
-  double* part = dalloc<double>(ctx, (size_t)grid * nv);
+  const int grid = grid_for(ctx, B->dim * 32, 256, 4);
+  DevBufs G;
+  double* part = G.add(dalloc<double>(ctx, (size_t)grid * nv));
+  int* derr = G.add(dalloc<int>(ctx, 1));
+  BLQH_TRY_CUDA(ctx, cudaMemsetAsync(derr, 0, sizeof(int), ctx->stream));
   std::vector<double> h((size_t)grid * nv);
-  try {
+  const SpinTables T = spin_tables(ctx, B, G, derr);
+  {
     TimerScope tm(ctx, TM_MISC);
-    k_spin_observables<<<grid, 256, 0, ctx->stream>>>(B->d_id, B->d_period, B->dim, nphi, B->ssector.K, psi, cplx,
-                                                      part);
+    k_spin_observables<<<grid, 256, 0, ctx->stream>>>(B->d_id, B->d_period, T.mem, T.FT, T.isq, B->dim, nphi,
+                                                      B->ssector.K, psi, cplx, part);
     BLQH_TRY_CUDA(ctx, cudaGetLastError());
     count_launch(ctx, TM_MISC);
-    BLQH_TRY_CUDA(ctx, cudaMemcpyAsync(h.data(), part, h.size() * 8, cudaMemcpyDeviceToHost, ctx->stream));
-    BLQH_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  } catch (...) {
-    dev_free(part);
-    throw;
   }
-  dev_free(part);
+  BLQH_TRY_CUDA(ctx, cudaMemcpyAsync(h.data(), part, h.size() * 8, cudaMemcpyDeviceToHost, ctx->stream));
+  check_overflow(ctx, derr);
   std::vector<double> t(nv, 0.0);
   for (int g = 0; g < grid; g++)
     for (int k = 0; k < nv; k++) t[k] += h[(size_t)g * nv + k];
@@ -806,14 +911,14 @@ void spin_observables_impl(blqh_ctx* ctx, const blqh_basis* B, const double* psi
 // per-row partials written by k_spin_rows (pass 2), summed in row order on the host.
 double spin_rayleigh_regen_impl(blqh_ctx* ctx, const blqh_basis* B, const blqh_params_spin& p, const double* x) {
   DevBufs G;
-  const SpinSetup S = spin_setup(ctx, B, p, G);
   double* part = G.add(dalloc<double>(ctx, B->dim));
   int* over = G.add(dalloc<int>(ctx, 1));
   BLQH_TRY_CUDA(ctx, cudaMemsetAsync(over, 0, sizeof(int), ctx->stream));
+  const SpinSetup S = spin_setup(ctx, B, p, G, over);
   {
     TimerScope ts(ctx, TM_BUILD);
-    k_spin_rows<<<S.grid, 256, S.smem, ctx->stream>>>(S.g, 2, S.slots, nullptr, nullptr, nullptr, nullptr, S.cplx,
-                                                      over, x, part);
+    S.rows<<<S.grid, SPIN_THREADS, S.smem, ctx->stream>>>(S.g, 2, S.slots, S.stride, nullptr, nullptr, nullptr,
+                                                          nullptr, over, x, part);
     BLQH_TRY_CUDA(ctx, cudaGetLastError());
     count_launch(ctx, TM_BUILD);
   }
