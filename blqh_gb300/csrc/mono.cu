@@ -16,26 +16,30 @@
 // order among its orbit members (the erase-while-iterating rule).
 //
 // Hamiltonian (replaces lhamil::set_hamil, lanczos_hamiltonian.cpp:77-198):
-// one warp per row. Work item w = ((k1 * npairs + p) * T + ti) walks the
-// reference's loops in their order: left translation k1, occupied pair p =
-// (n, m) in ascending order, hop t = ti - nphi / 2 in [-nphi / 2, nphi / 2].
-// Each lane looks the target up in a table of every orbit member (member ->
-// representative index and the translations that lead there; one member of an
-// orbit is a representative), which gives the column, the right translation k2
-// and the period Cr the reference finds by trying each k2 in turn. The warp then
-// groups equal columns of a round
-// of 32 items, and the lowest lane of each group adds the group's terms one by
-// one, in item order, to the column's accumulator in a per-warp open-addressing
-// table in shared memory. Every column therefore receives the reference's
-// terms in the reference's order, and the values equal the reference's sums.
-// The charging energy E_cl * nel joins the diagonal last, as in the reference
-// (:187). Pass 0 counts the entries with |value| > 1e-10; pass 1 sorts them by
-// column (bitonic, per warp) and writes them.
+// one warp per row. The reference walks the left translations k1 of the row state,
+// the occupied pairs (n, m) and the hops t in [-nphi / 2, nphi / 2]; the hop
+// operator commutes with the signed translations, so here the untranslated state
+// stands for all Cl translates and each hop carries the sum over k1: Cl times one
+// phase when the target orbit carries momentum K, an explicit signed sum otherwise
+// (short orbits). Work item w = (pair p, hop) in ascending order; per pair a mask
+// of the hops with both targets empty, so that lanes take only those. Each lane
+// looks the target up in the orbit-member table (members.cuh), which gives the
+// column, the right translation k2 and the period Cr the reference finds by trying
+// each k2 in turn. The warp then groups equal columns of a round of 32 items, and
+// the lowest lane of each group adds the group's terms one by one, in item order,
+// to the column's accumulator in a per-warp open-addressing table in shared memory:
+// rows are reproducible, and equal the reference's sums to rounding (its Cl equal
+// terms per hop are one product here). The charging energy E_cl * nel joins the
+// diagonal last, as in the reference (:187). Pass 0 counts the entries with |value|
+// > 1e-10; pass 1 sorts them by column (bitonic, per warp) and writes them.
+//
+// Bound by instruction issue and shared-memory latency. Nphi = 30, Ne = 10 (100,141
+// rows, 10 translations), whole build: 93 -> 10 ms against every translate.
 #include <algorithm>
 #include <cmath>
 #include <vector>
 
-#include "blqh_internal.h"
+#include "members.cuh"
 
 namespace {
 
@@ -161,65 +165,47 @@ struct MonoGen {
   const double* V2;     // [nphi][nphi]: 2 V[s][|t|]
   const double2* F;     // [C][C][2 C - 1]: (cos, sin)(2 pi K d / C) / sqrt(Cl Cr) at [Cl-1][Cr-1][d + C - 1]
   int* err;             // set when a table insert finds no free slot (never, by the sizing)
-  int compact;          // 1: per-(k1, pair) hop masks, only hops with empty targets become items
-  const uint64_t* mkey; // orbit-member table: keys (~0 = empty)
-  const uint32_t* mval; //   (representative index << 5) | translations from the representative
-  uint64_t mmask;       //   slots - 1
+  MemberTable mem;
 };
 
-constexpr uint64_t MEMBER_EMPTY = ~0ULL;
-
-// 64-bit mixing (the finalizer of MurmurHash3) for the member table's slots.
-__device__ __forceinline__ uint64_t mix64(uint64_t x) {
-  x ^= x >> 33;
-  x *= 0xff51afd7ed558ccdULL;
-  x ^= x >> 33;
-  x *= 0xc4ceb9fe1a85ec53ULL;
-  x ^= x >> 33;
-  return x;
-}
-
-// Every member translate(id_i, k), k in [0, period_i) (k = 0 only without
-// translation symmetry), keyed to (i << 5) | k. Open addressing with linear
-// probing in at least twice as many slots as members.
-__global__ void k_member_insert(const uint64_t* __restrict__ id, const uint8_t* __restrict__ period, int64_t dim,
-                                int nphi, int nel, int q, int orbits, uint64_t* __restrict__ key,
-                                uint32_t* __restrict__ val, uint64_t mask, int* err) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < dim; i += (int64_t)gridDim.x * blockDim.x) {
-    const int P = orbits ? period[i] : 1;
-    for (int k = 0; k < P; k++) {
-      int par;
-      const uint64_t m = k == 0 ? id[i] : mrot(id[i], k * q, nphi, nel, 0, &par);
-      uint64_t h = mix64(m) & mask;
-      bool done = false;
-      for (uint64_t probe = 0; probe <= mask; probe++) {
-        const unsigned long long prev = atomicCAS(reinterpret_cast<unsigned long long*>(key + h),
-                                                  (unsigned long long)MEMBER_EMPTY, (unsigned long long)m);
-        if (prev == MEMBER_EMPTY || prev == m) {
-          val[h] = (uint32_t)(i << 5) | (uint32_t)k;
-          done = true;
-          break;
-        }
-        h = (h + 1) & mask;
-      }
-      if (!done) atomicExch(err, 1);
-    }
+struct MonoRot {
+  int q, nphi, nel;
+  __device__ uint64_t operator()(uint64_t c, int k) const {
+    int p;
+    return mrot(c, k * q, nphi, nel, 0, &p);
   }
-}
+};
 
-__device__ __forceinline__ bool member_find(const uint64_t* __restrict__ key, const uint32_t* __restrict__ val,
-                                            uint64_t mask, uint64_t m, uint32_t* out) {
-  uint64_t h = mix64(m) & mask;
-  for (uint64_t probe = 0; probe <= mask; probe++) {
-    const uint64_t k = key[h];
-    if (k == m) {
-      *out = val[h];
-      return true;
-    }
-    if (k == MEMBER_EMPTY) return false;
-    h = (h + 1) & mask;
+// Sum over the translates k1 < Cl of a row state of sign * F for a target x reached
+// from the untranslated state, whose representative is k2 inverse translations away.
+__device__ __forceinline__ double2 translate_sum(const MonoGen& G, uint64_t x, int k2, int Cl, int Cr) {
+  const double2* F = G.F + (size_t)((Cl - 1) * G.C + (Cr - 1)) * (2 * G.C - 1) + G.C - 1;
+  int par = 0;
+  if (G.K < 0) return F[0];
+  bool coherent = Cr == G.C;
+  if (!coherent) {  // T^Cr on the orbit's states: sign times e^{2 pi i K Cr / C} = 1?
+    mrot(x, Cr * G.q, G.nphi, G.nel, 0, &par);
+    coherent = (2 * G.K * Cr + par * G.C) % (2 * G.C) == 0;
   }
-  return false;
+  if (coherent) {
+    par = 0;
+    if (k2) mrot(x, k2 * G.q, G.nphi, G.nel, 1, &par);
+    const double2 f = F[-k2];
+    const double s = par ? -(double)Cl : (double)Cl;
+    return make_double2(s * f.x, s * f.y);
+  }
+  double2 g = make_double2(0.0, 0.0);
+  for (int k1 = 0; k1 < Cl; k1++) {
+    int p1 = 0, p2 = 0;
+    const uint64_t y = k1 ? mrot(x, k1 * G.q, G.nphi, G.nel, 0, &p1) : x;
+    const int kk = (k2 + k1) % Cr;
+    if (kk) mrot(y, kk * G.q, G.nphi, G.nel, 1, &p2);
+    const double2 f = F[k1 - kk];
+    const double s = ((p1 + p2) & 1) ? -1.0 : 1.0;
+    g.x += s * f.x;
+    g.y += s * f.y;
+  }
+  return g;
 }
 
 constexpr int EMPTY = -1;
@@ -254,10 +240,9 @@ __device__ __forceinline__ int table_slot(int* __restrict__ key, int cap, int co
 }
 
 // Per-warp shared memory: the table (cap slots: 16-byte value, 4-byte column, 8-byte sort key),
-// 32 round terms and a counter, and with compaction (cq > 0) a hop mask and a prefix count per
-// (k1, occupied pair).
-__host__ __device__ inline size_t mono_warp_bytes(int cap, int cq) {
-  return (size_t)cap * (16 + 4 + 8) + 640 + (size_t)((cq + 1) & ~1) * 8;  // a multiple of 16 bytes
+// 32 round terms and a counter, and a hop mask and a prefix count per occupied pair.
+__host__ __device__ inline size_t mono_warp_bytes(int cap, int npairs) {
+  return (size_t)cap * (16 + 4 + 8) + 640 + (size_t)((npairs + 1) & ~1) * 8;  // a multiple of 16 bytes
 }
 
 // Pair p (0-based, ascending (a, b) with a < b) of the occupied orbitals: the a-th and b-th set bits.
@@ -306,18 +291,17 @@ __global__ void __launch_bounds__(256) k_mono_rows(MonoGen G, RowPass R, int pas
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   const int cap = R.cap;
-  const int cq = G.compact ? G.C * G.npairs : 0;
-  unsigned char* base = smem + (size_t)wib * mono_warp_bytes(cap, cq);
+  unsigned char* base = smem + (size_t)wib * mono_warp_bytes(cap, G.npairs);
   double2* tv = reinterpret_cast<double2*>(base);                       // [cap] accumulators
   uint64_t* sb = reinterpret_cast<uint64_t*>(base + (size_t)cap * 16);  // [cap] (col << 32 | slot), sorted
   int* tk = reinterpret_cast<int*>(base + (size_t)cap * 24);            // [cap] column or EMPTY
   double2* sval = reinterpret_cast<double2*>(base + (size_t)cap * 28);  // [32] round terms
   int* used = reinterpret_cast<int*>(base + (size_t)cap * 28 + 512);    // columns in the table
-  uint32_t* pm = reinterpret_cast<uint32_t*>(base + (size_t)cap * 28 + 640);  // [cq] hop masks
-  int* pp = reinterpret_cast<int*>(pm + cq);                                    // [cq] prefix counts
+  uint32_t* pm = reinterpret_cast<uint32_t*>(base + (size_t)cap * 28 + 640);  // [npairs] hop masks
+  int* pp = reinterpret_cast<int*>(pm + G.npairs);                             // [npairs] prefix counts
   const int nphi = G.nphi, half = nphi / 2;
   const uint64_t nmask = (1ULL << nphi) - 1;
-  const int per_k1 = G.npairs * G.T;
+  const int nq = G.npairs;
   for (int64_t r_ = (int64_t)blockIdx.x * wpb + wib; r_ < R.nrows; r_ += (int64_t)gridDim.x * wpb) {
     const int64_t i = R.rows ? R.rows[r_] : r_;
     if (pass == 1 && !R.rows && R.ovf[i]) continue;
@@ -328,61 +312,43 @@ __global__ void __launch_bounds__(256) k_mono_rows(MonoGen G, RowPass R, int pas
     if (lane == 0) *used = 0;
     __syncwarp();
     bool full = false;
-    const uint64_t idi = G.id[i];
+    const uint64_t lb = G.id[i];
     const int Cl = G.K < 0 ? 1 : G.period[i];
-    const int nq = Cl * G.npairs;
-    int nitems = Cl * per_k1;
-    if (G.compact) {
-      // only the hops with both targets empty, in the same (k1, pair, t) order
-      for (int qq = lane; qq < nq; qq += 32) {
-        const int k1 = qq / G.npairs, p = qq - k1 * G.npairs;
-        int par, n, m;
-        const uint64_t lb = k1 == 0 ? idi : mrot(idi, k1 * G.q, nphi, G.nel, 0, &par);
-        pair_orbitals(lb, p, G.nel, &n, &m);
-        pm[qq] = hop_mask(lb, n, m, nphi, G.T);
+    // only the hops with both targets empty, in (pair, t) order
+    int nitems = 0;
+    for (int q0 = 0; q0 < nq; q0 += 32) {
+      const int qq = q0 + lane;
+      int c = 0;
+      if (qq < nq) {
+        int n, m;
+        pair_orbitals(lb, qq, G.nel, &n, &m);
+        const uint32_t mask = hop_mask(lb, n, m, nphi, G.T);
+        pm[qq] = mask;
+        c = __popc(mask);
       }
-      __syncwarp();
-      int run = 0;
-      for (int q0 = 0; q0 < nq; q0 += 32) {
-        const int qq = q0 + lane;
-        const int c = qq < nq ? __popc(pm[qq]) : 0;
-        int incl = c;
-        for (int o = 1; o < 32; o <<= 1) {
-          const int y = __shfl_up_sync(0xffffffffu, incl, o);
-          if (lane >= o) incl += y;
-        }
-        if (qq < nq) pp[qq] = run + incl - c;
-        run += __shfl_sync(0xffffffffu, incl, 31);
+      int incl = c;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
       }
-      __syncwarp();
-      nitems = run;
+      if (qq < nq) pp[qq] = nitems + incl - c;
+      nitems += __shfl_sync(0xffffffffu, incl, 31);
     }
+    __syncwarp();
     for (int base_w = 0; base_w < nitems; base_w += 32) {
       const int w = base_w + lane;
       int hit_col = -1;
       double2 term = make_double2(0.0, 0.0);
       if (w < nitems) {
-        int k1, p, t;
-        if (G.compact) {
-          int lo = 0, hi = nq - 1;  // the last (k1, pair) whose prefix count is <= w
-          while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (pp[mid] <= w) lo = mid;
-            else hi = mid - 1;
-          }
-          uint32_t x = pm[lo];
-          for (int k = w - pp[lo]; k > 0; k--) x &= x - 1;
-          k1 = lo / G.npairs;
-          p = lo - k1 * G.npairs;
-          t = __ffs(x) - 1 - half;
-        } else {
-          k1 = w / per_k1;
-          const int r = w - k1 * per_k1;
-          p = r / G.T;
-          t = r - p * G.T - half;
+        int lo = 0, hi = nq - 1;  // the last pair whose prefix count is <= w
+        while (lo < hi) {
+          const int mid = (lo + hi + 1) >> 1;
+          if (pp[mid] <= w) lo = mid;
+          else hi = mid - 1;
         }
-        int parl = 0;
-        const uint64_t lb = k1 == 0 ? idi : mrot(idi, k1 * G.q, nphi, G.nel, 0, &parl);
+        uint32_t x = pm[lo];
+        for (int k = w - pp[lo]; k > 0; k--) x &= x - 1;
+        const int p = lo, t = __ffs(x) - 1 - half;
         int n, m;
         pair_orbitals(lb, p, G.nel, &n, &m);
         const uint64_t b = lb ^ ((1ULL << n) | (1ULL << m));
@@ -393,31 +359,24 @@ __global__ void __launch_bounds__(256) k_mono_rows(MonoGen G, RowPass R, int pas
         else if (mt >= nphi) mt -= nphi;
         // nt == mt: the reference's two masks carry into one bit and the target,
         // with nel - 1 electrons, is never in the basis
-        const uint64_t mt_mask = (1ULL << nt) | (1ULL << mt);
-        if (nt != mt && (mt_mask & b) == 0) {
-          const uint64_t rb0 = (b | mt_mask) & nmask;
+        if (nt != mt) {
+          const uint64_t rb0 = (b | (1ULL << nt) | (1ULL << mt)) & nmask;
           // The reference tries inv_translate(rb0, k2) for k2 in [0, Cr), Cr the period of
           // rb0, and adds the one that is a representative (lanczos_hamiltonian.cpp:160-184);
           // the member table gives that representative and k2 in one lookup, and Cr is
           // the representative's period.
           uint32_t mv;
-          if (member_find(G.mkey, G.mval, G.mmask, rb0, &mv)) {
+          if (member_find(G.mem, rb0, &mv)) {
             const int j = (int)(mv >> 5), k2 = (int)(mv & 31);
             const int Cr = G.K < 0 ? 1 : G.period[j];
-            int parr = 0;
-            if (k2) {
-              const int nc = pc64(rb0 & ((1ULL << (k2 * G.q)) - 1));
-              parr = (nc * (G.nel - nc)) & 1;
-            }
             // get_sign (basis.cpp:152-174): electrons of b between n and nt and between m and mt,
             // plus one when nt > mt (the pair crosses; n < m here)
-            const int par = occupied_between(b, n, nt) + occupied_between(b, m, mt) + (nt > mt ? 1 : 0) + parl + parr;
-            // 2 V sign FT / sqrt(Cl Cr) (lanczos_hamiltonian.cpp:180-181): the factor is
-            // tabulated on the host from the reference's expression, sign flips are exact
+            const int par = occupied_between(b, n, nt) + occupied_between(b, m, mt) + (nt > mt ? 1 : 0);
+            // 2 V sign FT / sqrt(Cl Cr) (lanczos_hamiltonian.cpp:180-181) summed over k1
             const double v2 = G.V2[(mt > n ? mt - n : n - mt) * nphi + (t < 0 ? -t : t)];
-            const double x = (par & 1) ? -v2 : v2;
-            const double2 f = G.F[((Cl - 1) * G.C + (Cr - 1)) * (2 * G.C - 1) + (k1 - k2 + G.C - 1)];
-            term = make_double2(x * f.x, G.imag ? x * f.y : 0.0);
+            const double v = (par & 1) ? -v2 : v2;
+            const double2 f = translate_sum(G, rb0, k2, Cl, Cr);
+            term = make_double2(v * f.x, G.imag ? v * f.y : 0.0);
             hit_col = j;
           }
         }
@@ -687,24 +646,7 @@ void build_mono_hamil(blqh_ctx* ctx, const blqh_basis* B, const blqh_params_mono
   g.V2 = dV;
   g.F = reinterpret_cast<const double2*>(dF);
   g.err = derr;
-  {
-    // orbit-member table: at most dim * C members (dim without translation symmetry)
-    const int64_t members = s.K >= 0 ? B->dim * C : B->dim;
-    uint64_t slots = 1024;
-    while (slots < (uint64_t)(2 * members)) slots <<= 1;
-    uint64_t* mkey = G.add(dalloc<uint64_t>(ctx, slots));
-    uint32_t* mval = G.add(dalloc<uint32_t>(ctx, slots));
-    BLQH_TRY_CUDA(ctx, cudaMemsetAsync(mkey, 0xFF, slots * 8, ctx->stream));
-    TimerScope tb(ctx, TM_BUILD);
-    k_member_insert<<<grid_for(ctx, B->dim, 256), 256, 0, ctx->stream>>>(B->d_id, B->d_period, B->dim, nphi, nel,
-                                                                         nphi / C, s.K >= 0, mkey, mval, slots - 1,
-                                                                         derr);
-    BLQH_TRY_CUDA(ctx, cudaGetLastError());
-    count_launch(ctx, TM_BUILD, 1);
-    g.mkey = mkey;
-    g.mval = mval;
-    g.mmask = slots - 1;
-  }
+  g.mem = build_members(ctx, G, B, MonoRot{nphi / C, nphi, nel}, s.K >= 0, C, derr);
   const int64_t dim = B->dim;
   M->dim = dim;
   M->is_complex = cplx;
@@ -726,10 +668,8 @@ void build_mono_hamil(blqh_ctx* ctx, const blqh_basis* B, const blqh_params_mono
   int* ovf_count = G.add(dalloc<int>(ctx, 1));
   BLQH_TRY_CUDA(ctx, cudaMemsetAsync(ovf, 0, dim, ctx->stream));
   BLQH_TRY_CUDA(ctx, cudaMemsetAsync(ovf_count, 0, 4, ctx->stream));
-  g.compact = C * g.npairs <= 1024 && g.T <= 32;
-  const int cq = g.compact ? C * g.npairs : 0;
   auto launch = [&](const RowPass& R, int pass, int32_t* dcol, double* dval) {
-    const size_t per_warp = mono_warp_bytes(R.cap, cq);
+    const size_t per_warp = mono_warp_bytes(R.cap, g.npairs);
     const int wpb = (int)std::max<size_t>(1, std::min<size_t>(8, (110 * 1024) / per_warp));
     const size_t sm = per_warp * wpb;
     BLQH_TRY_CUDA(ctx, smem_attr_at_least(kern, (int)sm));
@@ -859,7 +799,7 @@ int blqh_hamil_build_mono(blqh_ctx* ctx, const blqh_basis* b, const blqh_params_
     set_error(ctx, BLQH_ERR_ARG, "blqh_hamil_build_mono: lx, ly > 0 and nLL >= 0 required");
     return BLQH_ERR_ARG;
   }
-  if (mono_warp_bytes(mono_table_cap(b->msector.nphi, b->msector.nel), 1024) > 200 * 1024) {
+  if (mono_warp_bytes(mono_table_cap(b->msector.nphi, b->msector.nel), 1024) > 200 * 1024) {  // (at most 465 pairs)
     set_error(ctx, BLQH_ERR_UNSUPPORTED, "blqh_hamil_build_mono: row table larger than shared memory");
     return BLQH_ERR_UNSUPPORTED;
   }
