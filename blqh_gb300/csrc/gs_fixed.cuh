@@ -130,6 +130,22 @@ __device__ __forceinline__ void quantize(double x, int E, int& q1, int& q0) {
   q0 = (int)(q - ((long long)q1 << 29));
 }
 
+// x = (q.x 2^29 + q.y) 2^-59, |x| <= 1, rounded to nearest (the vector operand of
+// the fixed-point SpMV). Larger and non-finite values give zero (the SpMV's FP64
+// diagonal term carries them on).
+__device__ __forceinline__ int2 fix_unit(double x) {
+  const long long b = __double_as_longlong(x);
+  const int ex = (int)((b >> 52) & 0x7FF) - 1023;
+  long long m = (b & 0xFFFFFFFFFFFFFLL) | 0x10000000000000LL;
+  const int sh = ex + 7;  // m 2^(ex - 52) in units of 2^-59
+  if (ex > 0 || sh < -60) m = 0;
+  else if (sh >= 0) m <<= sh;
+  else m = (m + (1LL << (-sh - 1))) >> -sh;
+  const long long q = b < 0 ? -m : m;
+  const int hi = (int)((q + (1LL << 28)) >> 29);
+  return make_int2(hi, (int)(q - ((long long)hi << 29)));
+}
+
 // Exponent E of the largest |x| over the block, from each thread's largest high
 // word (sign cleared). All zero (or denormal): -1023.
 __device__ __forceinline__ int block_exponent(unsigned hw, unsigned* red) {
@@ -524,16 +540,18 @@ __device__ __forceinline__ float2 split_f64(double x) {
   return make_float2((float)hi * sh, (float)lo * sl);
 }
 
-// One vector entry: V_{j+1} and its split for the next double-float SpMV.
-__device__ __forceinline__ void store_entry(double v, int64_t i, double* vout, float2* xs) {
+// One vector entry: V_{j+1} and its split for the next SpMV (double-float xs, or fixed point xq).
+__device__ __forceinline__ void store_entry(double v, int64_t i, double* vout, float2* xs, int2* xq) {
   vout[i] = v;
   if (xs) xs[i] = split_f64(v);
+  if (xq) xq[i] = fix_unit(v);
 }
 
 // Where v_{j+1} goes: its row of V, of the planes, and the SpMV's split input.
 struct NextVec {
   double* v;
   float2* xs;
+  int2* xq;
   int* q1;
   int* q0;
   int* E;
@@ -669,7 +687,7 @@ __global__ void __launch_bounds__(KS * TILE / 4) k_update_q(const double* V, con
 #pragma unroll
         for (int z = 0; z < KS; z++) c += sred[z * TILE + i];
         a[q] = (a[q] - (double)c) * inv;
-        store_entry(a[q], r0 + i, nx.v, nx.xs);
+        store_entry(a[q], r0 + i, nx.v, nx.xs, nx.xq);
         hw = max(hw, abs_high_word(a[q]));
       }
     }
@@ -713,7 +731,7 @@ __global__ void __launch_bounds__(KS * TILE / 4) k_update_q(const double* V, con
       a[q] = 0.0;
       if (q * NT + (int)threadIdx.x < TILE && i < n) {
         a[q] = __ldcg(nx.v + i) * inv;
-        store_entry(a[q], i, nx.v, nx.xs);
+        store_entry(a[q], i, nx.v, nx.xs, nx.xq);
         hw = max(hw, abs_high_word(a[q]));
       }
     }

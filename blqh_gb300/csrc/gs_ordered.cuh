@@ -459,6 +459,7 @@ __global__ void __launch_bounds__(256) k_update_o(const double* V, const float* 
 struct NextPlanes {
   double* v;
   float2* xs;
+  int2* xq;
   float* vh;
   float* vl;
   int64_t ld;
@@ -489,7 +490,7 @@ __global__ void __launch_bounds__(256) k_scale_o(const double* src, int64_t n, i
       v = src[i];
       if (!start) {
         v *= inv;
-        store_entry(v, i, nx.v, nx.xs);
+        store_entry(v, i, nx.v, nx.xs, nx.xq);
       }
     }
     if (nx.vh) {

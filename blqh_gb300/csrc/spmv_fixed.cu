@@ -1,0 +1,233 @@
+// SpMV of complex FP64 matrices in fixed point (y = H x - b xprev, the Lanczos
+// product of Mat::operator*, BLQH_without_spin/matrix.cpp:244-267).
+//
+// The FP64 row kernel issues four FP64 FMAs per nonzero and ten FP64 additions per
+// row on a pipe of ~1.6 lane operations per clock per SM: that pipe, not memory,
+// sets its time. Here both operands are integers, split once: the matrix per row (57
+// bits below the row's largest off-diagonal entry; the diagonal stays FP64 and
+// apart), the vector on one scale (|x| <= 1, unit 2^-59),
+//   v = (v1 2^29 + v0) 2^(E - 56), |v1|, |v0| <= 2^28,
+//   x = (x1 2^29 + x0) 2^-59,      |x1| <= 2^30, |x0| <= 2^28,
+// and a row's sum is exact integer arithmetic: four IMAD.WIDE (27 lanes per clock
+// per SM) per real product into three 64-bit sums, folded into 128 bits every
+// eight nonzeros (the largest sum, of 2 x 8 cross products below 1.25 x 2^58, stays
+// below 2^63), one conversion to FP64 per row. What is lost is the operands'
+// rounding to 2^-57 of the row's largest entry and 2^-60 of the vector's norm,
+// below the 2^-53 an FP64 product rounds to.
+//
+// The split matrix takes 16 bytes per nonzero next to the CSR values. What is left
+// is the latency of the column, then the gather behind it (long-scoreboard stalls,
+// 12 of 20 cycles per issue; DRAM 46 %), so a lane has eight columns, then four
+// values and four gathers in flight. Measured (one GB300): 60,096 rows,
+// 1.54e7 nonzeros 212 -> 84 us; 100,141 rows, 2.4e7 nonzeros 318 -> 119 us;
+// 16,024 rows, 2.1e6 nonzeros 54 -> 22 us.
+#include <algorithm>
+#include <cstdlib>
+#include <type_traits>
+
+#include "blqh_internal.h"
+#include "krylov.cuh"
+#include "gs_fixed.cuh"
+
+namespace {
+
+// Row exponents, split off-diagonal values and the diagonal: one warp per row.
+__global__ void __launch_bounds__(256) k_fix_matrix(const int64_t* __restrict__ rp, const int32_t* __restrict__ col,
+                                                    const double2* __restrict__ val, int64_t dim,
+                                                    int4* __restrict__ qv, int* __restrict__ qe,
+                                                    double2* __restrict__ diag) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < dim; r += warps) {
+    const int64_t s = rp[r], e = rp[r + 1];
+    unsigned hw = 0;
+    bool has = false;
+    for (int64_t k = s + lane; k < e; k += 32) {
+      const double2 v = val[k];
+      if (col[k] == r) {
+        diag[r] = v;
+        has = true;
+      } else {
+        hw = max(hw, max(abs_high_word(v.x), abs_high_word(v.y)));
+      }
+    }
+    hw = __reduce_max_sync(0xffffffffu, hw);
+    has = __any_sync(0xffffffffu, has);
+    const int E = (int)(hw >> 20) - 1023;
+    if (lane == 0) {
+      qe[r] = E;
+      if (!has) diag[r] = make_double2(0.0, 0.0);
+    }
+    for (int64_t k = s + lane; k < e; k += 32) {
+      int4 q = make_int4(0, 0, 0, 0);
+      if (col[k] != r) {
+        const double2 v = val[k];
+        quantize(v.x, E, q.x, q.y);
+        quantize(v.y, E, q.z, q.w);
+      }
+      qv[k] = q;
+    }
+  }
+}
+
+// x in the vector's fixed point, for products whose previous kernel did not leave it.
+__global__ void k_fix_vector(const double* __restrict__ x, int2* __restrict__ xq, int64_t n, const int* stop) {
+  if (stop && *stop) return;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    xq[i] = fix_unit(x[i]);
+}
+
+struct Acc128 {
+  unsigned long long lo;
+  long long hi;
+  __device__ __forceinline__ void add(unsigned long long l, long long h) {
+    lo += l;
+    hi += h + (lo < l ? 1 : 0);
+  }
+  // + s[0] 2^58 + s[1] 2^29 + s[2]
+  __device__ __forceinline__ void fold(const long long* s) {
+    const __int128 t = ((__int128)s[0] << 58) + ((__int128)s[1] << 29) + s[2];
+    add((unsigned long long)t, (long long)(t >> 64));
+  }
+};
+
+__device__ __forceinline__ void fx_mul(long long* s, int a1, int a0, int b1, int b0) {
+  s[0] += (long long)a1 * b1;
+  s[1] += (long long)a1 * b0;
+  s[1] += (long long)a0 * b1;
+  s[2] += (long long)a0 * b0;
+}
+
+// LPR lanes per row. The real and imaginary sums are reduced together: after the
+// first exchange the lower half of a row's lanes carries the real part, the upper
+// half the imaginary part.
+template <int LPR>
+__global__ void __launch_bounds__(256, 3) k_spmv_fixed(const int64_t* __restrict__ rp, const int32_t* __restrict__ col,
+                                                    const int4* __restrict__ qv, const int* __restrict__ qe,
+                                                    const double2* __restrict__ diag, const int4* xq,
+                                                    const double2* x, double2* __restrict__ y, int64_t dim,
+                                                    const double* bptr, const double2* xprev, const int* stop) {
+  if (stop && *stop) return;
+  const int lane = threadIdx.x & 31;
+  constexpr int GPW = 32 / LPR;
+  const int gi = lane / LPR, sub = lane % LPR;
+  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  const double b = bptr ? *bptr : 0.0;
+  for (int64_t rb = warp * GPW; rb < dim; rb += nwarps * GPW) {  // the same rounds for every lane
+    const int64_t r = rb + gi;
+    const bool ok = r < dim;
+    const int64_t s = ok ? __ldg(rp + r) : 0;
+    const int len = ok ? (int)(__ldg(rp + r + 1) - s) : 0;
+    const int4* vp = qv + s;
+    const int32_t* cp = col + s;
+    Acc128 re{0, 0}, im{0, 0};
+    // eight nonzeros per lane at a time: the eight columns, then values and
+    // gathers of four; `full`: none of them past the row's end
+    auto group = [&](int k, auto full) {
+      constexpr bool F = decltype(full)::value;
+      int c[8];
+#pragma unroll
+      for (int u = 0; u < 8; u++) c[u] = F || k + u * LPR < len ? __ldcs(cp + k + u * LPR) : 0;
+      long long sr[3] = {0, 0, 0}, si[3] = {0, 0, 0};
+#pragma unroll
+      for (int h = 0; h < 8; h += 4) {
+        int4 v[4], g[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          v[u] = F || k + (h + u) * LPR < len ? __ldcs(vp + k + (h + u) * LPR) : make_int4(0, 0, 0, 0);
+          g[u] = __ldg(xq + c[h + u]);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          fx_mul(sr, v[u].x, v[u].y, g[u].x, g[u].y);
+          fx_mul(sr, -v[u].z, -v[u].w, g[u].z, g[u].w);
+          fx_mul(si, v[u].x, v[u].y, g[u].z, g[u].w);
+          fx_mul(si, v[u].z, v[u].w, g[u].x, g[u].y);
+        }
+      }
+      re.fold(sr);
+      im.fold(si);
+    };
+    int k = sub;
+    for (; k + 7 * LPR < len; k += 8 * LPR) group(k, std::true_type());
+    if (k < len) group(k, std::false_type());
+    const bool upper = sub >= LPR / 2;
+    Acc128 a = upper ? im : re;
+    const Acc128 o = upper ? re : im;
+    a.add(__shfl_xor_sync(0xffffffffu, o.lo, LPR / 2), __shfl_xor_sync(0xffffffffu, o.hi, LPR / 2));
+#pragma unroll
+    for (int d = LPR / 4; d > 0; d >>= 1)
+      a.add(__shfl_xor_sync(0xffffffffu, a.lo, d), __shfl_xor_sync(0xffffffffu, a.hi, d));
+    const double part = ok ? fx_to_double(a.hi, a.lo, __ldg(qe + r) - 115) : 0.0;
+    const double other = __shfl_xor_sync(0xffffffffu, part, LPR / 2);
+    if (ok && sub == 0) {
+      const double2 d = __ldg(diag + r), xr = x[r];
+      double2 w = make_double2(part + (d.x * xr.x - d.y * xr.y), other + (d.x * xr.y + d.y * xr.x));
+      if (xprev) {
+        const double2 p = xprev[r];
+        w.x -= b * p.x;
+        w.y -= b * p.y;
+      }
+      y[r] = w;
+    }
+  }
+}
+
+}  // namespace
+
+// The split copy of a complex FP64 matrix; false (and the FP64 kernel stays) without
+// room for it or with BLQH_SPMV_FIXED=0.
+bool fixed_prepare(blqh_ctx* ctx, blqh_csr* M) {
+  if (!M->is_complex || M->precision != BLQH_VAL_FP64) return false;
+  const char* env = getenv("BLQH_SPMV_FIXED");
+  if (env && env[0] == '0') return false;
+  if (M->d_qval) return true;
+  try {
+    M->d_qval = dev_alloc(ctx, std::max<int64_t>(1, M->nnz) * sizeof(int4));
+    M->d_qexp = dalloc<int>(ctx, M->dim);
+    M->d_qdiag = dalloc<double>(ctx, 2 * M->dim);
+  } catch (const BlqhError& e) {
+    if (e.code != BLQH_ERR_NOMEM) throw;
+    fixed_release(M);
+    ctx->last_error.clear();
+    return false;
+  }
+  TimerScope ts(ctx, TM_MISC);
+  k_fix_matrix<<<grid_for(ctx, M->dim * 32, 256, 16), 256, 0, ctx->stream>>>(
+      M->d_row_ptr, M->d_col, reinterpret_cast<const double2*>(M->d_val), M->dim, reinterpret_cast<int4*>(M->d_qval),
+      M->d_qexp, reinterpret_cast<double2*>(M->d_qdiag));
+  BLQH_TRY_CUDA(ctx, cudaGetLastError());
+  count_launch(ctx, TM_MISC);
+  return true;
+}
+
+void fixed_release(blqh_csr* M) {
+  dev_free(M->d_qval);
+  dev_free(M->d_qexp);
+  dev_free(M->d_qdiag);
+  M->d_qval = nullptr;
+  M->d_qexp = nullptr;
+  M->d_qdiag = nullptr;
+}
+
+void fixed_vector(blqh_ctx* ctx, const double* x, int2* xq, int64_t n, const int* stop) {
+  TimerScope tm(ctx, TM_MISC);
+  k_fix_vector<<<grid_for(ctx, n, 256, 8), 256, 0, ctx->stream>>>(x, xq, n, stop);
+  BLQH_TRY_CUDA(ctx, cudaGetLastError());
+  count_launch(ctx, TM_MISC);
+}
+
+// y = H x - b xprev; xq: x in fixed point (|x| <= 1, as Krylov vectors are).
+void fixed_spmv(blqh_ctx* ctx, const blqh_csr* M, const double* x, const int2* xq, double* y, const double* bptr,
+                const double* xprev, const int* stop) {
+  // 8 lanes per row (four rows per warp): 84 us at 60,096 rows of 256 nonzeros, against
+  // 92 with 4 lanes, 95 with 16 and 121 with 32 (longer reductions per row)
+  constexpr int LPR = 8;
+  const int64_t blocks = std::min<int64_t>((M->dim * LPR + 255) / 256, (int64_t)ctx->num_sms * 16);
+  k_spmv_fixed<LPR><<<(int)std::max<int64_t>(1, blocks), 256, 0, ctx->stream>>>(
+      M->d_row_ptr, M->d_col, reinterpret_cast<const int4*>(M->d_qval), M->d_qexp,
+      reinterpret_cast<const double2*>(M->d_qdiag), reinterpret_cast<const int4*>(xq),
+      reinterpret_cast<const double2*>(x), reinterpret_cast<double2*>(y), M->dim, bptr,
+      reinterpret_cast<const double2*>(xprev), stop);
+}

@@ -70,3 +70,45 @@ def test_exhausted_krylov_space(B, sec):
     assert abs(r["e"][0] - r["dense"][0]) < 1e-11
     assert np.sum(np.abs(r["e"] - r["dense"][0]) < 1e-9) == np.sum(np.abs(r["dense"] - r["dense"][0]) < 1e-9) or \
         np.sum(np.abs(r["e"] - r["dense"][0]) < 1e-9) == 1
+
+
+COMPLEX = [(6, 6, 3, 1, 2), (8, 8, 4, 0, 1), (8, 7, -1, 3, 1), (10, 10, 5, 0, 3), (12, 12, 6, 3, 5)]
+
+
+@pytest.mark.parametrize("sharp", [False, True], ids=["spread", "concentrated"])
+@pytest.mark.parametrize("sec", COMPLEX, ids=str)
+def test_fixed_point_product(B, monkeypatch, sec, sharp):
+    """The fixed-point SpMV of complex FP64 matrices against an extended-precision product of the same matrix: alpha_0
+    and beta_1 of a start vector (spread, or nearly one basis state) are no further off than the FP64 kernel's, or
+    below 4 ulp of the matrix's size where both are at rounding."""
+    b = B.Basis(*sec)
+    H = B.Hamiltonian(b, 0.9)
+    assert H.is_complex
+    r = np.random.RandomState(5)
+    x = r.standard_normal(H.dim) + 1j * r.standard_normal(H.dim)
+    if sharp:
+        x *= 1e-7
+        x[H.dim // 3] = 1.0
+    rp, col, val = H.csr()
+    x = x / np.linalg.norm(x)
+    xl = x.astype(np.clongdouble) / np.sqrt(np.sum(np.abs(x.astype(np.clongdouble)) ** 2))
+    y = np.add.reduceat(val.astype(np.clongdouble) * xl[col], rp[:-1])
+    a0 = np.sum(xl.conj() * y).real
+    b1 = np.sqrt(np.sum(np.abs(y - a0 * xl) ** 2))
+
+    def off():
+        L = B.Lanczos(H, max_steps=2, tol=0.0, start=x)
+        L.iterate()
+        a, be = L.coeffs()
+        L.close()
+        return max(abs(float(a[0] - a0)), abs(float(be[1] - b1)))
+
+    fixed = off()
+    monkeypatch.setenv("BLQH_SPMV_FIXED", "0")
+    H2 = B.Hamiltonian(b, 0.9)
+    H.close()
+    H = H2
+    native = off()
+    assert fixed <= max(native, 4 * np.finfo(float).eps * float(abs(a0) + b1)), (fixed, native)
+    H.close()
+    b.close()
