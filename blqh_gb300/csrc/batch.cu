@@ -16,7 +16,13 @@
 // components along v_j and v_{j-1}), then one full classical Gram-Schmidt
 // pass against every stored vector, and a further pass when the norm fell
 // below 1/sqrt(2) of its value after the three-term step (the
-// Daniel-Gragg-Kaufman-Stewart criterion). The lowest Ritz pair comes from
+// Daniel-Gragg-Kaufman-Stewart criterion). Real instances run the pass in FP64, in
+// a fixed order of operations (their ground states can be degenerate, see
+// gs_ordered.cuh, and then depend on it); complex instances take it on fixed-point
+// planes of the Krylov basis (gs_fixed.cuh), one exponent per vector: exact integer
+// dots, and the correction in FP32 while every coefficient is below 2^-30 |w|. The
+// FP64 pass of a complex instance took the SM's FP64 pipe 8 FMAs per entry and
+// vector; 96 instances of 5,940 states, 150 steps: 348 -> 134 ms. The lowest Ritz pair comes from
 // Sturm multisection and inverse iteration; the finisher is the FP64
 // regenerated Rayleigh quotient for FP32 values, the stored FP64 CSR otherwise.
 #include <algorithm>
@@ -27,6 +33,7 @@
 #include <vector>
 
 #include "krylov.cuh"
+#include "gs_fixed.cuh"
 #include "sector.cuh"
 
 namespace {
@@ -45,6 +52,9 @@ struct BInst {
   double* ab;     // alpha [lam], beta [lam + 1] (beta[0] = 0)
   double* res;    // [5]: energy, lowest Ritz value, residual estimate, steps, repeated Gram-Schmidt passes
   double* xg;     // [N] staging of the SpMV input in global memory when it does not fit shared memory
+  // complex: fixed-point planes of V [(lam + 1) * NP] and of w [NP], NP = N rounded up to 4 (null: FP64 pass)
+  int* q1;
+  int* q0;
 };
 
 constexpr int RED = 66;  // doubles of the block-reduction area
@@ -57,18 +67,20 @@ __host__ __device__ inline int batch_fixed_doubles(int lam) {
 
 // Per-instance device storage, in doubles from the instance's block (each array 256-byte aligned).
 struct Lay {
-  size_t V, w, psi, ab, res, xg, total;
+  size_t V, w, psi, ab, xg, q1, q0, total;
 };
-inline Lay instance_layout(int64_t N, int lam, bool xsmem) {
+inline Lay instance_layout(int64_t N, int lam, bool xsmem, bool planes) {
   auto up = [](size_t v) { return (v + 31) / 32 * 32; };
   Lay L;
   L.V = 0;
   L.w = up((size_t)N * (lam + 1));
   L.psi = up(L.w + N);
   L.ab = up(L.psi + N);
-  L.res = L.ab + 2 * lam + 1;
-  L.xg = up(L.res + 5);
-  L.total = up(L.xg + (xsmem ? 0 : (size_t)N));
+  L.xg = up(L.ab + 2 * lam + 1);
+  const size_t q = planes ? up((size_t)(lam + 2) * (size_t)((N + 3) / 4 * 4) / 2 + 1) : 0;  // ints
+  L.q1 = up(L.xg + (xsmem ? 0 : (size_t)N));
+  L.q0 = L.q1 + q;
+  L.total = L.q0 + q;
   return L;
 }
 
@@ -102,40 +114,136 @@ __device__ __forceinline__ void block_sum2(double& a, double& b, double* red) {
   b = red[65];
 }
 
+// Calls use(i, load(i)) for this thread's i < n in ascending order, U loads in flight
+// (stores in `use` would otherwise order every load behind the previous entry's).
+template <int NT, int U, class L, class F>
+__device__ __forceinline__ void sweep(int64_t n_, L load, F use) {
+  const int n = (int)n_;
+  int i = threadIdx.x;
+  for (; i + (U - 1) * NT < n; i += U * NT) {
+    decltype(load(i)) r[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) r[u] = load(i + u * NT);
+#pragma unroll
+    for (int u = 0; u < U; u++) use(i + u * NT, r[u]);
+  }
+#pragma unroll 1
+  for (; i < n; i += NT) use(i, load(i));
+}
+
+template <bool CPLX, bool F32>
+struct ValT;
+template <>
+struct ValT<false, false> {
+  using T = double;
+};
+template <>
+struct ValT<true, false> {
+  using T = double2;
+};
+template <>
+struct ValT<false, true> {
+  using T = float;
+};
+template <>
+struct ValT<true, true> {
+  using T = float2;
+};
+
 // w = H x (rq = false), or the partial Re <x, H x> of this thread (rq = true,
-// FP64 values only). x: FP32 pairs (hi, lo) per double when F32, FP64
-// otherwise; in shared or global memory. F32: w receives the unevaluated
+// FP64 values only). x: FP32 pairs (hi, lo) per double when F32 (complex entries as
+// (re hi, im hi, re lo, im lo), so that both parts go through packed FP32 operations
+// at once), FP64 otherwise; in shared or global memory. F32: w receives the unevaluated
 // (hi, lo) pair of every component (same 8 bytes); converting here would cost
 // every lane of a row group an FP64 instruction, so run_instance converts them
 // lane-parallel.
+// A block is all its SM runs, so the matrix stream's latency shows: each lane keeps
+// the next BS nonzeros (of its row, or the first ones of its next row) in flight
+// behind the ones it works on. Sums are in column order per lane as without it.
 template <int NT, int LPR, bool CPLX, bool F32>
 __device__ __forceinline__ double bspmv(const BInst& I, const void* __restrict__ x, double* __restrict__ w,
                                         bool rq) {
+  using VT = typename ValT<CPLX, F32>::T;
   constexpr int NG = NT / LPR;
+  constexpr int BS = 8;
   const int grp = threadIdx.x / LPR, sub = threadIdx.x % LPR;
+  const VT* __restrict__ val = reinterpret_cast<const VT*>(I.val);
   double dot = 0.0;
+  auto range = [&](int64_t r, int64_t& s, int64_t& e) {
+    const bool ok = r < I.dim;
+    s = ok ? __ldg(I.rp + r) : 0;
+    e = ok ? __ldg(I.rp + r + 1) : 0;
+  };
+  int32_t cc[BS];
+  VT vv[BS];
+  auto load = [&](int32_t (&c)[BS], VT (&v)[BS], int64_t k, int64_t e) {
+#pragma unroll
+    for (int u = 0; u < BS; u++) {
+      c[u] = 0;
+      v[u] = VT{};
+      if (k + u * LPR < e) {
+        c[u] = __ldg(I.col + k + u * LPR);
+        v[u] = __ldg(val + k + u * LPR);
+      }
+    }
+  };
+  int64_t s, e, s1, e1;  // this row's range and the next one's
+  range(grp, s, e);
+  range(grp + NG, s1, e1);
+  load(cc, vv, s + sub, e);
   for (int64_t rb = 0; rb < I.dim; rb += NG) {
     const int64_t r = rb + grp;
     const bool ok = r < I.dim;
-    const int64_t s = ok ? __ldg(I.rp + r) : 0, e = ok ? __ldg(I.rp + r + 1) : 0;
-    if (F32) {
-      float rh = 0.f, rl = 0.f, ih = 0.f, il = 0.f;
-#pragma unroll 4
-      for (int64_t k = s + sub; k < e; k += LPR) {
-        const int32_t c = __ldg(I.col + k);
-        if (CPLX) {
-          const float2 v = __ldg(reinterpret_cast<const float2*>(I.val) + k);
-          const float4 xv = reinterpret_cast<const float4*>(x)[c];
-          df_add_prod(rh, rl, v.x, xv.x, xv.y);
-          df_add_prod(rh, rl, -v.y, xv.z, xv.w);
-          df_add_prod(ih, il, v.x, xv.z, xv.w);
-          df_add_prod(ih, il, v.y, xv.x, xv.y);
-        } else {
-          const float v = __ldg(reinterpret_cast<const float*>(I.val) + k);
-          const float2 xv = reinterpret_cast<const float2*>(x)[c];
-          df_add_prod(rh, rl, v, xv.x, xv.y);
+    int64_t s2, e2;
+    range(r + 2 * NG, s2, e2);
+    float rh = 0.f, rl = 0.f, ih = 0.f, il = 0.f;
+    double ar = 0.0, ai = 0.0;
+    f32x2 ah = 0, al = 0, bh = 0, bl = 0;  // F32 complex: sums of Re v (re, im) x and of (Im v, -Im v) (re, im) x
+    int64_t k = s + sub;
+    for (;;) {
+      const bool more = k + BS * LPR < e;
+      int32_t cn[BS];
+      VT vn[BS];
+      load(cn, vn, more ? k + BS * LPR : s1 + sub, more ? e : e1);
+#pragma unroll
+      for (int u = 0; u < BS; u++) {
+        if (k + u * LPR < e) {
+          const int32_t c = cc[u];
+          if constexpr (F32 && CPLX) {
+            const ulonglong2 xv = reinterpret_cast<const ulonglong2*>(x)[c];
+            df_add_prod2(ah, al, pack2(vv[u].x, vv[u].x), xv.x, xv.y);
+            df_add_prod2(bh, bl, pack2(vv[u].y, -vv[u].y), xv.x, xv.y);
+          } else if constexpr (F32) {
+            const float2 xv = reinterpret_cast<const float2*>(x)[c];
+            df_add_prod(rh, rl, vv[u], xv.x, xv.y);
+          } else if constexpr (CPLX) {
+            const double2 xv = reinterpret_cast<const double2*>(x)[c];
+            ar += vv[u].x * xv.x - vv[u].y * xv.y;
+            ai += vv[u].x * xv.y + vv[u].y * xv.x;
+          } else {
+            ar += vv[u] * reinterpret_cast<const double*>(x)[c];
+          }
         }
       }
+#pragma unroll
+      for (int u = 0; u < BS; u++) {
+        cc[u] = cn[u];
+        vv[u] = vn[u];
+      }
+      if (!more) break;
+      k += BS * LPR;
+    }
+    __syncwarp();
+    if (F32 && CPLX) {  // re = a.re + b.im (-Im v Im x), im = a.im + b.re
+      const float2 a = unpack2(ah), b = unpack2(al), c = unpack2(bh), d = unpack2(bl);
+      rh = a.x;
+      rl = b.x;
+      ih = a.y;
+      il = b.y;
+      df_add(rh, rl, c.y, d.y);
+      df_add(ih, il, c.x, d.x);
+    }
+    if (F32) {
       df_seg_reduce<LPR>(rh, rl);
       if (CPLX) df_seg_reduce<LPR>(ih, il);
       if (ok && sub == 0) {
@@ -148,19 +256,6 @@ __device__ __forceinline__ double bspmv(const BInst& I, const void* __restrict__
         }
       }
     } else {
-      double ar = 0.0, ai = 0.0;
-#pragma unroll 4
-      for (int64_t k = s + sub; k < e; k += LPR) {
-        const int32_t c = __ldg(I.col + k);
-        if (CPLX) {
-          const double2 v = __ldg(reinterpret_cast<const double2*>(I.val) + k);
-          const double2 xv = reinterpret_cast<const double2*>(x)[c];
-          ar += v.x * xv.x - v.y * xv.y;
-          ai += v.x * xv.y + v.y * xv.x;
-        } else {
-          ar += __ldg(reinterpret_cast<const double*>(I.val) + k) * reinterpret_cast<const double*>(x)[c];
-        }
-      }
 #pragma unroll
       for (int o = LPR / 2; o > 0; o >>= 1) {
         ar += __shfl_xor_sync(0xffffffffu, ar, o, LPR);
@@ -181,6 +276,10 @@ __device__ __forceinline__ double bspmv(const BInst& I, const void* __restrict__
         }
       }
     }
+    s = s1;
+    e = e1;
+    s1 = s2;
+    e1 = e2;
   }
   return dot;
 }
@@ -199,6 +298,7 @@ __device__ __forceinline__ void cgs_dots(const double* __restrict__ V, int64_t N
       const double2* b2 = reinterpret_cast<const double2*>(w);
       const int64_t n2 = N / 2;
       int64_t i = lane;
+#pragma unroll 2
       for (; i + 32 < n2; i += 64) {
         const double2 a = a2[i], b = b2[i], c = a2[i + 32], d = b2[i + 32];
         sr += a.x * b.x + a.y * b.y;
@@ -213,6 +313,7 @@ __device__ __forceinline__ void cgs_dots(const double* __restrict__ V, int64_t N
       }
     } else {
       int64_t i = lane;
+#pragma unroll 4
       for (; i + 32 < N; i += 64) {
         sr += vk[i] * w[i];
         tr += vk[i + 32] * w[i + 32];
@@ -281,11 +382,151 @@ __device__ __forceinline__ double cgs_update(const double* __restrict__ V, int64
   return nn;
 }
 
-// Write v (FP64) into the SpMV input area: FP32 pairs or FP64.
+// ---- the full pass of complex instances on fixed-point planes --------------------
+// Extra bits of headroom of an N-entry vector's exponent: 2 (57 - s) + log2 N + 1 bits
+// of a whole vector's sum stay below 2^126.
+__device__ __forceinline__ int plane_headroom(int64_t N) {
+  const int lg = 64 - __clzll(N);
+  return lg > 11 ? (lg - 10) / 2 : 0;
+}
+
+// Exponent of the block's largest |x| plus the headroom (in every thread).
+template <int NT>
+__device__ __forceinline__ int plane_exponent(unsigned hw, int64_t N, double* red) {
+  unsigned* ur = reinterpret_cast<unsigned*>(red);
+  hw = __reduce_max_sync(0xffffffffu, hw);
+  if ((threadIdx.x & 31) == 0) ur[threadIdx.x >> 5] = hw;
+  __syncthreads();
+  unsigned m = 0;
+#pragma unroll
+  for (int i = 0; i < NT / 32; i++) m = max(m, ur[i]);
+  __syncthreads();
+  return (int)(m >> 20) - 1023 + plane_headroom(N);
+}
+
+// Planes of x (N entries, FP64, written by this block) with exponent E; zeros up to NP.
+template <int NT>
+__device__ __forceinline__ void write_planes(const double* x, int64_t N, int64_t NP, int E, int* q1, int* q0) {
+  sweep<NT, 4>(
+      NP, [&](int i) { return i < N ? x[i] : 0.0; },
+      [&](int i, double v) {
+        int a, b;
+        quantize(v, E, a, b);
+        q1[i] = a;
+        q0[i] = b;
+      });
+}
+
+// h[k] = conj(V_k) w from the planes, a warp two vectors at a time (w read once for both).
+template <int NT>
+__device__ __forceinline__ void cgs_dots_q(const int* __restrict__ q1, const int* __restrict__ q0, int64_t NP,
+                                           const int* qe, int nk, const int* w1, const int* w0, int we, double* h) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int n4 = (int)(NP / 4);
+  for (int k = 2 * wid; k < nk; k += 2 * (NT / 32)) {
+    const int kb = min(k + 1, nk - 1);  // a missing second vector repeats the first
+    const int4* a1 = reinterpret_cast<const int4*>(q1 + k * NP);
+    const int4* a0 = reinterpret_cast<const int4*>(q0 + k * NP);
+    const int4* b1 = reinterpret_cast<const int4*>(q1 + kb * NP);
+    const int4* b0 = reinterpret_cast<const int4*>(q0 + kb * NP);
+    Acc128 t[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};  // (re, im) of both
+    auto one = [&](long long (&s)[3], long long (&r)[3], const int4& x1, const int4& x0, const int4& y1,
+                   const int4& y0) {  // conj(x) y of two entries
+      fx_add(s, x1.x, x0.x, y1.x, y0.x);
+      fx_add(s, x1.y, x0.y, y1.y, y0.y);
+      fx_add(s, x1.z, x0.z, y1.z, y0.z);
+      fx_add(s, x1.w, x0.w, y1.w, y0.w);
+      fx_add(r, x1.x, x0.x, y1.y, y0.y);
+      fx_add(r, -x1.y, -x0.y, y1.x, y0.x);
+      fx_add(r, x1.z, x0.z, y1.w, y0.w);
+      fx_add(r, -x1.w, -x0.w, y1.z, y0.z);
+    };
+    for (int i0 = lane; i0 < n4; i0 += 8 * 32) {  // 32 products per 64-bit sum
+      long long s[4][3] = {};
+#pragma unroll 2
+      for (int u = 0; u < 8; u++) {
+        const int i = i0 + 32 * u;
+        if (i >= n4) break;
+        const int4 x1 = __ldcg(a1 + i), x0 = __ldcg(a0 + i), z1 = __ldcg(b1 + i), z0 = __ldcg(b0 + i);
+        const int4 y1 = reinterpret_cast<const int4*>(w1)[i], y0 = reinterpret_cast<const int4*>(w0)[i];
+        one(s[0], s[1], x1, x0, y1, y0);
+        one(s[2], s[3], z1, z0, y1, y0);
+      }
+#pragma unroll
+      for (int c = 0; c < 4; c++) t[c].fold(s[c]);
+    }
+    const int ea = qe[k] + we - 112, eb = qe[kb] + we - 112;
+    const double ar = t[0].warp_sum(ea), ai = t[1].warp_sum(ea), br = t[2].warp_sum(eb), bi = t[3].warp_sum(eb);
+    if (lane == 0) {
+      h[2 * k] = ar;
+      h[2 * k + 1] = ai;
+      if (k + 1 < nk) {
+        h[2 * k + 2] = br;
+        h[2 * k + 3] = bi;
+      }
+    }
+  }
+}
+
+// Whether every coefficient is below 2^-30 of |w| (|w|^2 = nn), by exponents, and the
+// coefficients times the planes' scale as FP32: value = q1 2^(E - 27). One flag in *ok.
+template <int NT>
+__device__ __forceinline__ void plane_coefs(const double* h, const int* qe, int nk, double nn, float2* hf, int* ok) {
+  if (threadIdx.x == 0) *ok = 1;
+  __syncthreads();
+  const int en = (int)(abs_high_word(nn) >> 20) - 1023;
+  bool small = true;
+  for (int k = threadIdx.x; k < nk; k += NT) {
+    const int eh = (int)(max(abs_high_word(h[2 * k]), abs_high_word(h[2 * k + 1])) >> 20) - 1023;
+    small = small && 2 * (eh + 2) <= en - 60;
+    const int e = qe[k] - 27;
+    const float sc = e < -126 ? 0.0f : __uint_as_float((unsigned)(e + 127) << 23);
+    hf[k] = make_float2(f64_lead_f32(h[2 * k]) * sc, f64_lead_f32(h[2 * k + 1]) * sc);
+  }
+  if (!small) atomicExch(ok, 0);
+  __syncthreads();
+}
+
+// w -= sum_k h_k V_k, the sum in FP32 from the leading planes; this thread's partial |w|^2.
+template <int NT>
+__device__ __forceinline__ double cgs_update_q(const int* __restrict__ q1, int64_t NP, int nk, const float2* hf,
+                                               double* w, int64_t N) {
+  double nn = 0.0;
+  for (int64_t i = 4 * threadIdx.x; i < N; i += 4 * NT) {
+    float d[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
+    for (int k = 0; k < nk; k++) {
+      const int4 v = __ldcg(reinterpret_cast<const int4*>(q1 + k * NP + i));
+      const float v0 = (float)v.x, v1 = (float)v.y, v2 = (float)v.z, v3 = (float)v.w;
+      const float2 c = hf[k];
+      d[0] = fmaf(c.x, v0, fmaf(-c.y, v1, d[0]));
+      d[1] = fmaf(c.x, v1, fmaf(c.y, v0, d[1]));
+      d[2] = fmaf(c.x, v2, fmaf(-c.y, v3, d[2]));
+      d[3] = fmaf(c.x, v3, fmaf(c.y, v2, d[3]));
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      if (i + q < N) {
+        const double a = w[i + q] - (double)d[q];
+        w[i + q] = a;
+        nn += a * a;
+      }
+  }
+  return nn;
+}
+
+// Write v (FP64, double i of the vector) into the SpMV input area: FP32 pairs or FP64 (see bspmv).
+template <bool CPLX>
 __device__ __forceinline__ void stage_x(void* x, int64_t i, double v, bool f32) {
   if (f32) {
-    const float hi = (float)v;
-    reinterpret_cast<float2*>(x)[i] = make_float2(hi, (float)(v - (double)hi));
+    const float2 p = split_f64(v);
+    if (CPLX) {
+      float* f = reinterpret_cast<float*>(x) + 4 * (i >> 1) + (i & 1);
+      f[0] = p.x;
+      f[2] = p.y;
+    } else {
+      reinterpret_cast<float2*>(x)[i] = p;
+    }
   } else {
     reinterpret_cast<double*>(x)[i] = v;
   }
@@ -301,7 +542,8 @@ __device__ __forceinline__ double splitmix_unit(uint64_t seed, uint64_t stream, 
 }
 
 template <int NT, int LPR, bool CPLX, bool F32>
-__device__ void run_instance(const BInst& I, int lam, uint64_t seed, double bd_tol, double* sm, void* xs_sm) {
+__device__ void run_instance(const BInst& I, int lam, uint64_t seed, double bd_tol, int use_planes, double* sm,
+                             void* xs_sm) {
   double* red = sm;
   double* hs = red + RED;
   double* h2 = hs + 2 * (lam + 1);
@@ -312,6 +554,14 @@ __device__ void run_instance(const BInst& I, int lam, uint64_t seed, double bd_t
   double* scal = trw + 6 * lam;
   void* x = I.xsmem ? xs_sm : static_cast<void*>(I.xg);
   const int64_t N = I.dim * (CPLX ? 2 : 1);
+  // planes: per vector an exponent (ys is free until the tridiagonal solve, as is trw)
+  const bool planes = CPLX && use_planes && I.q1;
+  const int64_t NP = (N + 3) / 4 * 4;
+  int* qe = reinterpret_cast<int*>(ys);
+  float2* hf = reinterpret_cast<float2*>(trw);
+  int* ok = reinterpret_cast<int*>(scal + 1);
+  int* w1 = planes ? I.q1 + (int64_t)(lam + 1) * NP : nullptr;
+  int* w0 = planes ? I.q0 + (int64_t)(lam + 1) * NP : nullptr;
 
   // start vector: splitmix64 of (seed, instance number, index) - 1/2, normalized
   double nn = 0.0, z0 = 0.0;
@@ -323,10 +573,19 @@ __device__ void run_instance(const BInst& I, int lam, uint64_t seed, double bd_t
   block_sum2<NT>(nn, z0, red);
   {
     const double inv = 1.0 / sqrt(nn);
-    for (int64_t i = threadIdx.x; i < N; i += NT) {
-      const double v = I.V[i] * inv;
-      I.V[i] = v;
-      stage_x(x, i, v, F32);
+    unsigned hw = 0;
+    sweep<NT, 4>(
+        N, [&](int i) { return I.V[i]; },
+        [&](int i, double u) {
+          const double v = u * inv;
+          I.V[i] = v;
+          stage_x<CPLX>(x, i, v, F32);
+          hw = max(hw, abs_high_word(v));
+        });
+    if (planes) {
+      const int E = plane_exponent<NT>(hw, N, red);
+      if (threadIdx.x == 0) qe[0] = E;
+      write_planes<NT>(I.V, N, NP, E, I.q1, I.q0);
     }
   }
   if (threadIdx.x == 0) I.ab[lam] = 0.0;  // beta[0]
@@ -338,12 +597,13 @@ __device__ void run_instance(const BInst& I, int lam, uint64_t seed, double bd_t
     __syncthreads();
     double n0 = 0.0, z = 0.0;
     if (F32) {
-      for (int64_t i = threadIdx.x; i < N; i += NT) {
-        const float2 pr = reinterpret_cast<const float2*>(I.w)[i];
-        const double v = (double)pr.x + (double)pr.y;
-        I.w[i] = v;
-        n0 += v * v;
-      }
+      sweep<NT, 4>(
+          N, [&](int i) { return reinterpret_cast<const float2*>(I.w)[i]; },
+          [&](int i, float2 pr) {
+            const double v = (double)pr.x + (double)pr.y;
+            I.w[i] = v;
+            n0 += v * v;
+          });
       __syncthreads();
     } else {
       for (int64_t i = threadIdx.x; i < N; i += NT) n0 += I.w[i] * I.w[i];
@@ -356,9 +616,23 @@ __device__ void run_instance(const BInst& I, int lam, uint64_t seed, double bd_t
     z = 0.0;
     block_sum2<NT>(nloc, z, red);
     // full classical Gram-Schmidt pass against V_0..V_j
-    cgs_dots<NT, CPLX>(I.V, N, j + 1, I.w, hs);
-    __syncthreads();
-    double n1 = cgs_update<NT, CPLX>(I.V, N, j + 1, hs, I.w);
+    double n1;
+    if (planes) {
+      unsigned hw = 0;
+      sweep<NT, 4>(
+          N, [&](int i) { return I.w[i]; }, [&](int, double v) { hw = max(hw, abs_high_word(v)); });
+      const int we = plane_exponent<NT>(hw, N, red);
+      write_planes<NT>(I.w, N, NP, we, w1, w0);
+      __syncthreads();
+      cgs_dots_q<NT>(I.q1, I.q0, NP, qe, j + 1, w1, w0, we, hs);
+      __syncthreads();
+      plane_coefs<NT>(hs, qe, j + 1, nloc, hf, ok);
+      n1 = *ok ? cgs_update_q<NT>(I.q1, NP, j + 1, hf, I.w, N) : cgs_update<NT, CPLX>(I.V, N, j + 1, hs, I.w);
+    } else {
+      cgs_dots<NT, CPLX>(I.V, N, j + 1, I.w, hs);
+      __syncthreads();
+      n1 = cgs_update<NT, CPLX>(I.V, N, j + 1, hs, I.w);
+    }
     z = 0.0;
     block_sum2<NT>(n1, z, red);
     for (int t = threadIdx.x; t < 2 * nl; t += NT) hs[2 * k0 + t] += h2[t];
@@ -390,10 +664,19 @@ __device__ void run_instance(const BInst& I, int lam, uint64_t seed, double bd_t
     if (j + 1 == lam) break;
     const double inv = 1.0 / beta;
     double* vn = I.V + (int64_t)(j + 1) * N;
-    for (int64_t i = threadIdx.x; i < N; i += NT) {
-      const double v = I.w[i] * inv;
-      vn[i] = v;
-      stage_x(x, i, v, F32);
+    unsigned hw = 0;
+    sweep<NT, 4>(
+        N, [&](int i) { return I.w[i]; },
+        [&](int i, double u) {
+          const double v = u * inv;
+          vn[i] = v;
+          stage_x<CPLX>(x, i, v, F32);
+          hw = max(hw, abs_high_word(v));
+        });
+    if (planes) {
+      const int E = plane_exponent<NT>(hw, N, red);
+      if (threadIdx.x == 0) qe[j + 1] = E;
+      write_planes<NT>(vn, N, NP, E, I.q1 + (int64_t)(j + 1) * NP, I.q0 + (int64_t)(j + 1) * NP);
     }
     __syncthreads();
   }
@@ -445,7 +728,7 @@ __device__ void run_instance(const BInst& I, int lam, uint64_t seed, double bd_t
     for (int64_t i = threadIdx.x; i < N; i += NT) {
       const double v = I.psi[i] * inv;
       I.psi[i] = v;
-      if (!F32) stage_x(x, i, v, false);
+      if (!F32) stage_x<CPLX>(x, i, v, false);
     }
   }
   __syncthreads();
@@ -469,24 +752,27 @@ __device__ void run_instance(const BInst& I, int lam, uint64_t seed, double bd_t
 
 template <int NT, int LPR>
 __global__ void __launch_bounds__(NT) k_batch_lanczos(const BInst* __restrict__ insts, const int* __restrict__ order,
-                                                      int n, int lam, uint64_t seed, double bd_tol, int* counter) {
+                                                      int n, int lam, uint64_t seed, double bd_tol, int use_planes,
+                                                      int* counter) {
   extern __shared__ __align__(16) double bsm[];
   void* xs_sm = bsm + batch_fixed_doubles(lam);
   __shared__ int s_idx;
+  __shared__ BInst I;  // (its pointers would take thirty registers of every thread)
   for (;;) {
-    if (threadIdx.x == 0) s_idx = atomicAdd(counter, 1);
-    __syncthreads();
-    const int idx = s_idx;
-    __syncthreads();
-    if (idx >= n) break;
-    const BInst I = insts[order[idx]];
-    if (I.cplx) {
-      if (I.fp32) run_instance<NT, LPR, true, true>(I, lam, seed, bd_tol, bsm, xs_sm);
-      else run_instance<NT, LPR, true, false>(I, lam, seed, bd_tol, bsm, xs_sm);
-    } else {
-      if (I.fp32) run_instance<NT, LPR, false, true>(I, lam, seed, bd_tol, bsm, xs_sm);
-      else run_instance<NT, LPR, false, false>(I, lam, seed, bd_tol, bsm, xs_sm);
+    if (threadIdx.x == 0) {
+      s_idx = atomicAdd(counter, 1);
+      if (s_idx < n) I = insts[order[s_idx]];
     }
+    __syncthreads();
+    if (s_idx >= n) break;
+    if (I.cplx) {
+      if (I.fp32) run_instance<NT, LPR, true, true>(I, lam, seed, bd_tol, use_planes, bsm, xs_sm);
+      else run_instance<NT, LPR, true, false>(I, lam, seed, bd_tol, use_planes, bsm, xs_sm);
+    } else {
+      if (I.fp32) run_instance<NT, LPR, false, true>(I, lam, seed, bd_tol, use_planes, bsm, xs_sm);
+      else run_instance<NT, LPR, false, false>(I, lam, seed, bd_tol, use_planes, bsm, xs_sm);
+    }
+    __syncthreads();  // I and s_idx are written again
   }
 }
 
@@ -508,7 +794,7 @@ __global__ void k_rq_reduce(const double* __restrict__ part, const int64_t* __re
   }
 }
 
-using KFn = void (*)(const BInst*, const int*, int, int, uint64_t, double, int*);
+using KFn = void (*)(const BInst*, const int*, int, int, uint64_t, double, int, int*);
 KFn batch_kernel(int threads, int lpr) {
 #define BLQH_K(T, L) \
   if (threads == T && lpr == L) return k_batch_lanczos<T, L>;
@@ -533,6 +819,7 @@ struct blqh_batch {
   std::vector<int64_t> N;            // doubles per vector
   std::vector<size_t> pool_off;      // doubles from the pool start
   double* pool = nullptr;
+  double* d_resall = nullptr;        // [n][5] results
   BInst* d_inst = nullptr;
   int* d_order = nullptr;
   int* d_counter = nullptr;
@@ -549,7 +836,12 @@ struct blqh_batch {
   cudaGraphExec_t gexec = nullptr;
   cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};  // before the Lanczos launch, after it, after the finisher
   bool solved = false;
-  Lay layout(int i) const { return instance_layout(N[i], o.lambda, N[i] * 8 <= x_cap); }
+  bool planes = true;                // fixed-point planes for complex instances
+  Lay layout(int i) const {
+    const bool cplx = csr[i]->is_complex;
+    // (the x area may grow after the tuning, so complex instances keep a global one)
+    return instance_layout(N[i], o.lambda, !cplx && N[i] * 8 <= x_cap, planes && cplx);
+  }
 };
 
 namespace {
@@ -564,6 +856,7 @@ void batch_free(blqh_batch* b) {
   for (auto* m : b->csr) free_csr(m);
   for (auto* s : b->bases) blqh_basis_destroy(s);
   dev_free(b->pool);
+  dev_free(b->d_resall);
   dev_free(b->d_inst);
   dev_free(b->d_order);
   dev_free(b->d_counter);
@@ -621,7 +914,7 @@ void tune_shape(blqh_batch* b) {
           BLQH_TRY_CUDA(ctx, cudaMemsetAsync(b->d_counter, 0, sizeof(int), ctx->stream));
           BLQH_TRY_CUDA(ctx, cudaEventRecord(b->ev[0], ctx->stream));
           b->kern<<<std::min(b->grid, nsub), b->threads, b->smem, ctx->stream>>>(b->d_inst, b->d_order, nsub, lam_t,
-                                                                                 b->o.seed, 1e-13, b->d_counter);
+                                                                                 b->o.seed, 1e-13, 0, b->d_counter);
           BLQH_TRY_CUDA(ctx, cudaGetLastError());
           BLQH_TRY_CUDA(ctx, cudaEventRecord(b->ev[1], ctx->stream));
           BLQH_TRY_CUDA(ctx, cudaEventSynchronize(b->ev[1]));
@@ -711,14 +1004,24 @@ void batch_create_impl(blqh_batch* b) {
   configure_shape(b, b->o.threads ? b->o.threads : 256,
                   b->o.lanes_per_row ? b->o.lanes_per_row : lpr_for(b->mean_row));
   // device storage per instance (instance_layout)
-  b->pool_off.assign(b->n, 0);
-  size_t total = 0;
-  for (int i = 0; i < b->n; i++) {
-    if (!b->csr[i]) continue;
-    b->pool_off[i] = total;
-    total += b->layout(i).total;
+  for (;;) {
+    b->pool_off.assign(b->n, 0);
+    size_t total = 0;
+    for (int i = 0; i < b->n; i++) {
+      if (!b->csr[i]) continue;
+      b->pool_off[i] = total;
+      total += b->layout(i).total;
+    }
+    try {
+      b->pool = dalloc<double>(ctx, total + 32);
+      break;
+    } catch (const BlqhError& e) {  // without room for the planes: the FP64 pass
+      if (e.code != BLQH_ERR_NOMEM || !b->planes) throw;
+      b->planes = false;
+      ctx->last_error.clear();
+    }
   }
-  b->pool = dalloc<double>(ctx, total + 32);
+  b->d_resall = dalloc<double>(ctx, 5 * (size_t)std::max(1, b->n));  // every instance's results, read back at once
   std::vector<BInst> hi;
   std::vector<double> cost;
   std::vector<double*> res_ptr;
@@ -741,8 +1044,12 @@ void batch_create_impl(blqh_batch* b) {
     I.w = p + L.w;
     I.psi = p + L.psi;
     I.ab = p + L.ab;
-    I.res = p + L.res;
-    I.xg = I.xsmem ? nullptr : p + L.xg;
+    I.res = b->d_resall + 5 * (size_t)i;
+    I.xg = I.xsmem && !I.cplx ? nullptr : p + L.xg;
+    if (b->planes && I.cplx) {
+      I.q1 = reinterpret_cast<int*>(p + L.q1);
+      I.q0 = reinterpret_cast<int*>(p + L.q0);
+    }
     hi.push_back(I);
     // cost: SpMV bytes and reorthogonalization work over lam steps
     cost.push_back((double)lam * ((double)M->nnz * (I.fp32 ? 8.0 : 12.0) * (I.cplx ? 1.5 : 1.0) +
@@ -761,6 +1068,19 @@ void batch_create_impl(blqh_batch* b) {
   }
   b->grid = std::max(1, std::min(b->nrun, ctx->num_sms * b->bps));
   if (b->o.threads == 0 && b->o.lanes_per_row == 0 && tune_enabled() && b->nrun > 0) tune_shape(b);
+  // Where one block per SM is all there is (by its registers and shared memory, or by
+  // the number of instances), the x area takes what shared memory is left, so that
+  // the gathers of larger complex instances stay in it.
+  if (b->nrun && (b->bps == 1 || b->nrun <= ctx->num_sms)) {
+    const int64_t cap = std::min<int64_t>(max_n * 8, smem_max - fixed - 64);
+    if (cap > b->x_cap) {
+      b->smem = fixed + (int)((cap + 15) / 16 * 16);
+      configure_shape(b, b->threads, b->lpr);
+      for (BInst& I : hi)
+        if (I.cplx) I.xsmem = I.dim * 16 <= cap;
+      BLQH_TRY_CUDA(ctx, cudaMemcpy(b->d_inst, hi.data(), hi.size() * sizeof(BInst), cudaMemcpyHostToDevice));
+    }
+  }
   // mixed precision: one regenerated Rayleigh quotient per instance
   b->rq.assign(b->n, nullptr);
   if (b->o.value_precision == BLQH_VAL_FP32) {
@@ -812,7 +1132,7 @@ void batch_enqueue(blqh_batch* b) {
   BLQH_TRY_CUDA(ctx, cudaMemsetAsync(b->d_counter, 0, sizeof(int), ctx->stream));
   record_ev(ctx, b->ev[0]);
   b->kern<<<b->grid, b->threads, b->smem, ctx->stream>>>(b->d_inst, b->d_order, b->nrun, b->o.lambda, b->o.seed,
-                                                         1e-13, b->d_counter);
+                                                         1e-13, 1, b->d_counter);
   BLQH_TRY_CUDA(ctx, cudaGetLastError());
   record_ev(ctx, b->ev[1]);
   count_launch(ctx, TM_SPMV);
@@ -918,6 +1238,12 @@ int blqh_batch_results(const blqh_batch* b, blqh_batch_result* out) {
     set_error(b->ctx, BLQH_ERR_STATE, "blqh_batch_results: call blqh_batch_solve first");
     return BLQH_ERR_STATE;
   }
+  std::vector<double> all(5 * (size_t)std::max(1, b->n));
+  if (b->nrun &&
+      cudaMemcpy(all.data(), b->d_resall, 5 * (size_t)b->n * sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess) {
+    set_error(b->ctx, BLQH_ERR_CUDA, "blqh_batch_results: copy failed");
+    return BLQH_ERR_CUDA;
+  }
   for (int i = 0; i < b->n; i++) {
     blqh_batch_result r{};
     const blqh_csr* M = b->csr[i];
@@ -926,12 +1252,7 @@ int blqh_batch_results(const blqh_batch* b, blqh_batch_result* out) {
       out[i] = r;
       continue;
     }
-    double res[5];
-    const double* d = b->pool + b->pool_off[i] + b->layout(i).res;
-    if (cudaMemcpy(res, d, sizeof(res), cudaMemcpyDeviceToHost) != cudaSuccess) {
-      set_error(b->ctx, BLQH_ERR_CUDA, "blqh_batch_results: copy failed");
-      return BLQH_ERR_CUDA;
-    }
+    const double* res = all.data() + 5 * (size_t)i;
     r.energy = res[0];
     r.ritz0 = res[1];
     r.resid = res[2];

@@ -332,19 +332,33 @@ __device__ __forceinline__ double fx_to_double(long long hi, unsigned long long 
   return __longlong_as_double((long long)(bits | (neg ? 1ULL << 63 : 0)));
 }
 
+// A 128-bit sum: three 64-bit sums hold 32 products (fx_add), longer ones are folded into it.
+struct Acc128 {
+  unsigned long long lo;
+  long long hi;
+  __device__ __forceinline__ void add(unsigned long long l, long long h) {
+    lo += l;
+    hi += h + (lo < l ? 1 : 0);
+  }
+  // + s[0] 2^58 + s[1] 2^29 + s[2]
+  __device__ __forceinline__ void fold(const long long* s) {
+    const __int128 t = ((__int128)s[0] << 58) + ((__int128)s[1] << 29) + s[2];
+    add((unsigned long long)t, (long long)(t >> 64));
+  }
+  // the sum over the warp, as FP64 times 2^e
+  __device__ __forceinline__ double warp_sum(int e) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      add(__shfl_xor_sync(0xffffffffu, lo, o), __shfl_xor_sync(0xffffffffu, hi, o));
+    return fx_to_double(hi, lo, e);
+  }
+};
+
 // The 128-bit sum over the warp as FP64 times 2^e.
 __device__ __forceinline__ double fx_warp_sum(const long long* s, int e) {
-  const __int128 t = ((__int128)s[0] << 58) + ((__int128)s[1] << 29) + s[2];
-  unsigned long long lo = (unsigned long long)t;
-  long long hi = (long long)(t >> 64);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const unsigned long long l2 = __shfl_xor_sync(0xffffffffu, lo, o);
-    const long long h2 = __shfl_xor_sync(0xffffffffu, hi, o);
-    lo += l2;
-    hi += h2 + (lo < l2 ? 1 : 0);
-  }
-  return fx_to_double(hi, lo, e);
+  Acc128 a{0, 0};
+  a.fold(s);
+  return a.warp_sum(e);
 }
 
 // Full pass, dots: h2[k] = conj(V_k) w' for k in [0, nk) from the planes. A block

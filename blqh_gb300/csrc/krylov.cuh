@@ -28,6 +28,51 @@ __device__ __forceinline__ void df_add_prod(float& ah, float& al, float v, float
   ah = s;
   al += e + t;
 }
+// Two FP32 values in one 64-bit register and the packed operations on them: each
+// half rounds as the scalar operation does, one issue slot for both.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+  return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 neg2(f32x2 a) { return a ^ 0x8000000080000000ULL; }
+// a - b, exact as the scalar difference: b times -1 added
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
+  return fma2(b, 0xBF800000BF800000ULL, a);  // (-1, -1)
+}
+// df_add_prod on both halves.
+__device__ __forceinline__ void df_add_prod2(f32x2& ah, f32x2& al, f32x2 v, f32x2 xh, f32x2 xl) {
+  const f32x2 p = mul2(v, xh);
+  const f32x2 pe = fma2(v, xh, neg2(p));
+  const f32x2 t = fma2(v, xl, pe);
+  const f32x2 s = add2(ah, p);
+  const f32x2 bb = sub2(s, ah);
+  const f32x2 e = add2(sub2(ah, sub2(s, bb)), sub2(p, bb));
+  ah = s;
+  al = add2(al, add2(e, t));
+}
+
 template <int LPR>
 __device__ __forceinline__ void df_seg_reduce(float& ah, float& al) {
 #pragma unroll

@@ -77,27 +77,6 @@ __global__ void k_fix_vector(const double* __restrict__ x, int2* __restrict__ xq
     xq[i] = fix_unit(x[i]);
 }
 
-struct Acc128 {
-  unsigned long long lo;
-  long long hi;
-  __device__ __forceinline__ void add(unsigned long long l, long long h) {
-    lo += l;
-    hi += h + (lo < l ? 1 : 0);
-  }
-  // + s[0] 2^58 + s[1] 2^29 + s[2]
-  __device__ __forceinline__ void fold(const long long* s) {
-    const __int128 t = ((__int128)s[0] << 58) + ((__int128)s[1] << 29) + s[2];
-    add((unsigned long long)t, (long long)(t >> 64));
-  }
-};
-
-__device__ __forceinline__ void fx_mul(long long* s, int a1, int a0, int b1, int b0) {
-  s[0] += (long long)a1 * b1;
-  s[1] += (long long)a1 * b0;
-  s[1] += (long long)a0 * b1;
-  s[2] += (long long)a0 * b0;
-}
-
 // LPR lanes per row. The real and imaginary sums are reduced together: after the
 // first exchange the lower half of a row's lanes carries the real part, the upper
 // half the imaginary part.
@@ -140,10 +119,10 @@ __global__ void __launch_bounds__(256, 3) k_spmv_fixed(const int64_t* __restrict
         }
 #pragma unroll
         for (int u = 0; u < 4; u++) {
-          fx_mul(sr, v[u].x, v[u].y, g[u].x, g[u].y);
-          fx_mul(sr, -v[u].z, -v[u].w, g[u].z, g[u].w);
-          fx_mul(si, v[u].x, v[u].y, g[u].z, g[u].w);
-          fx_mul(si, v[u].z, v[u].w, g[u].x, g[u].y);
+          fx_add(sr, v[u].x, v[u].y, g[u].x, g[u].y);
+          fx_add(sr, -v[u].z, -v[u].w, g[u].z, g[u].w);
+          fx_add(si, v[u].x, v[u].y, g[u].z, g[u].w);
+          fx_add(si, v[u].z, v[u].w, g[u].x, g[u].y);
         }
       }
       re.fold(sr);

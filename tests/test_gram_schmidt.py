@@ -112,3 +112,24 @@ def test_fixed_point_product(B, monkeypatch, sec, sharp):
     assert fixed <= max(native, 4 * np.finfo(float).eps * float(abs(a0) + b1)), (fixed, native)
     H.close()
     b.close()
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+def test_batched_complex_instances(B, prec):
+    """Complex instances of a batch (fixed-point pass, one exponent per vector): vectors of 2 x 11 .. 2 x 636 doubles,
+    some not a multiple of four, up to the whole Krylov space; energies as the dense matrix's (FP32 values finish
+    with the FP64 quotient of a 1e-7 vector: 1e-9)."""
+    secs = [s for s in SECTORS if s[4] not in (0, s[0] // 2) and s[0] <= 10 and s[1] == s[0]]
+    b = B.Batch([B.instance(*s, d) for s in secs for d in (0.6, 1.4)], lam=100,
+                precision=B.VAL_FP64 if prec == "f64" else B.VAL_FP32)
+    b.solve()
+    res = b.results()
+    for i, r in enumerate(res):
+        sec, d = secs[i // 2], (0.6, 1.4)[i % 2]
+        ref = _run(B, sec, B.VAL_FP64, 100, d)
+        assert r["dim"] == ref["dim"]
+        assert abs(r["energy"] - ref["dense"][0]) < (1e-10 if prec == "f64" else 1e-9)
+        psi = b.ground_state(i)
+        assert abs(np.linalg.norm(psi) - 1) < 1e-12
+        assert 1 - abs(np.vdot(psi, ref["psi"])) < 1e-10
+    b.close()
