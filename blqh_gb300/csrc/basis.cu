@@ -178,6 +178,114 @@ __global__ void k_lvl_pos(int64_t r, int64_t rn, const uint32_t* bkt, const int6
   }
 }
 
+// The first growth levels (up to LVL_SMALL buckets) in one block with everything in
+// shared memory (12 arrays of LVL_SMALL, the next level would not fit): a level of a
+// few hundred nodes is 16 launches, two of which the host waited for, of work that is
+// all latency. All of a basis: nphi 8, 0.59 -> 0.17 ms (75 -> 6 launches), nphi 12,
+// 1.2 -> 0.53 ms. The rules are those of the kernels above.
+constexpr int LVL_SMALL = 2400, LVL_THREADS = 1024, LVL_MAX = 12;
+struct SmallLevels {
+  int n;
+  uint32_t P[LVL_MAX];
+};
+
+// Exclusive scan of x[0..n), n <= 3 LVL_THREADS, into out (may be x).
+__device__ __forceinline__ void lvl_scan(const uint32_t* x, uint32_t* out, int n, uint32_t* wsum) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, i0 = threadIdx.x * 3;
+  uint32_t v[3], s = 0;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    v[k] = i0 + k < n ? x[i0 + k] : 0;
+    s += v[k];
+  }
+  uint32_t inc = s;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += y;
+  }
+  if (lane == 31) wsum[wid] = inc;
+  __syncthreads();
+  if (wid == 0) {
+    uint32_t w = wsum[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += y;
+    }
+    wsum[lane] = w;
+  }
+  __syncthreads();
+  uint32_t ex = (wid ? wsum[wid - 1] : 0) + inc - s;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    if (i0 + k < n) out[i0 + k] = ex;
+    ex += v[k];
+  }
+  __syncthreads();
+}
+
+__global__ void __launch_bounds__(LVL_THREADS) k_lvl_small(const uint64_t* keys, SmallLevels L, int N,
+                                                           uint32_t* pos_out) {
+  extern __shared__ uint32_t lv_sm[];
+  __shared__ uint32_t wsum[32];
+  uint32_t* a[12];
+  for (int i = 0; i < 12; i++) a[i] = lv_sm + i * LVL_SMALL;
+  uint32_t *pos = a[0], *npos = a[1];
+  uint32_t *bkt = a[2], *mem = a[3], *slot = a[4], *fo = a[5], *fn = a[6], *cnt = a[7], *cnew = a[8], *gs = a[9],
+           *cur = a[10], *bst = a[11];
+  int r = 0;
+  for (int lv = 0; lv < L.n; lv++) {
+    const uint32_t P = L.P[lv];
+    const int rn = min((int)P, N);
+    for (int b = threadIdx.x; b < (int)P; b += LVL_THREADS) {
+      fo[b] = fn[b] = NONE;
+      cnt[b] = cnew[b] = cur[b] = 0;
+      if (b < rn) slot[b] = 0;
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < rn; e += LVL_THREADS) {
+      const uint32_t b = (uint32_t)(keys[e] % P);
+      bkt[e] = b;
+      if (e < r) {
+        atomicMin(&fo[b], pos[e]);
+      } else {
+        atomicMin(&fn[b], (uint32_t)e);
+        atomicAdd(&cnew[b], 1u);
+      }
+      atomicAdd(&cnt[b], 1u);
+    }
+    __syncthreads();
+    for (int b = threadIdx.x; b < (int)P; b += LVL_THREADS)
+      if (cnt[b]) {
+        const int s = fo[b] != NONE ? (rn - r) + (r - 1 - (int)fo[b]) : rn - 1 - (int)fn[b];
+        slot[s] = cnt[b];
+        gs[b] = (uint32_t)s;
+      }
+    __syncthreads();
+    lvl_scan(slot, slot, rn, wsum);
+    lvl_scan(cnt, bst, (int)P, wsum);
+    for (int e = threadIdx.x; e < rn; e += LVL_THREADS) mem[bst[bkt[e]] + atomicAdd(&cur[bkt[e]], 1u)] = (uint32_t)e;
+    __syncthreads();
+    for (int e = threadIdx.x; e < rn; e += LVL_THREADS) {
+      const uint32_t b = bkt[e], s = bst[b], nb = cnt[b];
+      uint32_t rank = e >= r ? 0 : cnew[b];
+      const uint32_t pe = e >= r ? 0 : pos[e];
+      for (uint32_t k = 0; k < nb; k++) {
+        const uint32_t f = mem[s + k];
+        rank += e >= r ? (f >= (uint32_t)r && f > (uint32_t)e) : (f < (uint32_t)r && pos[f] > pe);
+      }
+      npos[e] = slot[gs[b]] + rank;
+    }
+    __syncthreads();
+    uint32_t* t = pos;
+    pos = npos;
+    npos = t;
+    r = rn;
+  }
+  for (int e = threadIdx.x; e < r; e += LVL_THREADS) pos_out[e] = pos[e];
+}
+
 // ---- survivor selection and compaction --------------------------------------
 constexpr int SEL_BLOCK = 256;
 constexpr int SEL_ITEMS = 8;
@@ -530,31 +638,39 @@ uint32_t* iteration_positions(blqh_ctx* ctx, const uint64_t* keys, int64_t N) {
   uint32_t* members = G.add(dalloc<uint32_t>(ctx, N));
   uint32_t* slot_size = G.add(dalloc<uint32_t>(ctx, N));
   int64_t* slot_off = G.add(dalloc<int64_t>(ctx, N));
-  uint32_t* first_old = G.add(dalloc<uint32_t>(ctx, Pmax));
-  uint32_t* first_new = G.add(dalloc<uint32_t>(ctx, Pmax));
-  uint32_t* cnt = G.add(dalloc<uint32_t>(ctx, Pmax));
-  uint32_t* cnt_new = G.add(dalloc<uint32_t>(ctx, Pmax));
+  // per level: [first_old | first_new] set to NONE, [cnt | cnt_new | cursor] to 0, each P entries
+  uint32_t* none = G.add(dalloc<uint32_t>(ctx, 2 * Pmax));
+  uint32_t* zero = G.add(dalloc<uint32_t>(ctx, 3 * Pmax));
   uint32_t* gslot = G.add(dalloc<uint32_t>(ctx, Pmax));
-  uint32_t* cursor = G.add(dalloc<uint32_t>(ctx, Pmax));
   int64_t* bstart = G.add(dalloc<int64_t>(ctx, Pmax));
+  int64_t* scratch = G.add(dalloc<int64_t>(ctx, scan_scratch((int64_t)Pmax)));
+  cudaStream_t st = ctx->stream;
   int64_t r = 0;
-  for (size_t lv = 0; lv < Ps.size() && r < N; lv++) {
+  size_t lv0 = 0;
+  SmallLevels L{};
+  while (lv0 < Ps.size() && Ps[lv0] <= LVL_SMALL && L.n < LVL_MAX) L.P[L.n++] = (uint32_t)Ps[lv0++];
+  if (L.n && N > 0) {
+    const int sm = 12 * LVL_SMALL * 4;
+    BLQH_TRY_CUDA(ctx, smem_attr_at_least(k_lvl_small, sm));
+    r = std::min<int64_t>(L.P[L.n - 1], N);
+    k_lvl_small<<<1, LVL_THREADS, sm, st>>>(keys, L, (int)r, pos);
+    BLQH_TRY_CUDA(ctx, cudaGetLastError());
+    count_launch(ctx, TM_BASIS, 1);
+  }
+  for (size_t lv = lv0; lv < Ps.size() && r < N; lv++) {
     const uint64_t Pl = Ps[lv];
     const int64_t rn = std::min<int64_t>((int64_t)Pl, N);
-    cudaStream_t st = ctx->stream;
-    BLQH_TRY_CUDA(ctx, cudaMemsetAsync(first_old, 0xFF, Pl * 4, st));
-    BLQH_TRY_CUDA(ctx, cudaMemsetAsync(first_new, 0xFF, Pl * 4, st));
-    BLQH_TRY_CUDA(ctx, cudaMemsetAsync(cnt, 0, Pl * 4, st));
-    BLQH_TRY_CUDA(ctx, cudaMemsetAsync(cnt_new, 0, Pl * 4, st));
-    BLQH_TRY_CUDA(ctx, cudaMemsetAsync(cursor, 0, Pl * 4, st));
+    uint32_t *first_old = none, *first_new = none + Pl, *cnt = zero, *cnt_new = zero + Pl, *cursor = zero + 2 * Pl;
+    BLQH_TRY_CUDA(ctx, cudaMemsetAsync(none, 0xFF, 2 * Pl * 4, st));
+    BLQH_TRY_CUDA(ctx, cudaMemsetAsync(zero, 0, 3 * Pl * 4, st));
     BLQH_TRY_CUDA(ctx, cudaMemsetAsync(slot_size, 0, rn * 4, st));
     k_lvl_bucket<<<grid_for(ctx, rn, BLK), BLK, 0, st>>>(keys, pos, r, rn, Pl, bkt, first_old, first_new, cnt,
                                                         cnt_new);
     k_lvl_slots<<<grid_for(ctx, (int64_t)Pl, BLK), BLK, 0, st>>>(r, rn, Pl, first_old, first_new, cnt, slot_size,
                                                                 gslot);
     BLQH_TRY_CUDA(ctx, cudaGetLastError());
-    scan_exclusive_u32_to_i64(ctx, slot_size, slot_off, rn, nullptr);
-    scan_exclusive_u32_to_i64(ctx, cnt, bstart, (int64_t)Pl, nullptr);
+    scan_enqueue_u32_to_i64(ctx, slot_size, slot_off, rn, scratch);
+    scan_enqueue_u32_to_i64(ctx, cnt, bstart, (int64_t)Pl, scratch);
     k_lvl_members<<<grid_for(ctx, rn, BLK), BLK, 0, st>>>(rn, bkt, bstart, cursor, members);
     k_lvl_pos<<<grid_for(ctx, rn, BLK), BLK, 0, st>>>(r, rn, bkt, bstart, cnt, cnt_new, members, gslot, slot_off,
                                                      pos, npos);

@@ -235,6 +235,9 @@ void fixed_spmv(blqh_ctx* ctx, const blqh_csr* M, const double* x, const int2* x
 
 void scan_exclusive_i64(blqh_ctx* ctx, const int64_t* in, int64_t* out, int64_t n, int64_t* total_host);
 void scan_exclusive_u32_to_i64(blqh_ctx* ctx, const uint32_t* in, int64_t* out, int64_t n, int64_t* total_host);
+// The same enqueued on the context's stream, in the caller's scratch of scan_scratch(n) values.
+int64_t scan_scratch(int64_t n);
+void scan_enqueue_u32_to_i64(blqh_ctx* ctx, const uint32_t* in, int64_t* out, int64_t n, int64_t* scratch);
 
 // tune.cu: shape choices timed once per problem class, cached in a JSON file.
 bool tune_enabled();

@@ -305,7 +305,24 @@ void scan_impl(blqh_ctx* ctx, const T* in, int64_t* out, int64_t n, int64_t* tot
   }
   dev_free(bs);
 }
+
+// One launch sequence without waiting: scratch holds scan_scratch(n) values.
+template <class T>
+void scan_enqueue(blqh_ctx* ctx, const T* in, int64_t* out, int64_t n, int64_t* scratch) {
+  if (n <= 0) return;
+  const int64_t nb = (n + SCAN_TILE - 1) / SCAN_TILE;
+  k_scan_reduce<T><<<(unsigned)nb, SCAN_BLOCK, 0, ctx->stream>>>(in, n, scratch);
+  k_scan_blocks<<<1, SCAN_BLOCK, 0, ctx->stream>>>(scratch, nb, scratch + nb);
+  k_scan_apply<T><<<(unsigned)nb, SCAN_BLOCK, 0, ctx->stream>>>(in, out, n, scratch);
+  BLQH_TRY_CUDA(ctx, cudaGetLastError());
+  count_launch(ctx, TM_MISC, 3);
+}
 }  // namespace
+
+int64_t scan_scratch(int64_t n) { return (n + SCAN_TILE - 1) / SCAN_TILE + 1; }
+void scan_enqueue_u32_to_i64(blqh_ctx* ctx, const uint32_t* in, int64_t* out, int64_t n, int64_t* scratch) {
+  scan_enqueue<uint32_t>(ctx, in, out, n, scratch);
+}
 
 void scan_exclusive_i64(blqh_ctx* ctx, const int64_t* in, int64_t* out, int64_t n, int64_t* total_host) {
   scan_impl<int64_t>(ctx, in, out, n, total_host);
