@@ -27,6 +27,7 @@
 #include "krylov.cuh"
 #include "gs_ordered.cuh"
 #include "sector.cuh"
+#include "tridiag.cuh"
 
 double rayleigh_regen_impl(blqh_ctx* ctx, const blqh_basis* B, const blqh_params& p, const double* d_psi,
                            bool want_complex);
@@ -291,69 +292,46 @@ __global__ void __launch_bounds__(256) k_rq_res(const int64_t* __restrict__ rp, 
 }
 
 // ---------------------------------------------------------------------------
-// K6: tridiagonal eigen-solve (Sturm count, bounds, inverse iteration in krylov.cuh).
-// Lowest eigenvalue by parallel multisection (one block); optional
-// convergence test against the previous check, which sets the stop flag.
-// One warp. FP64 on GB300 runs at a small fraction of the FP32 rate and a
-// block-wide multisection of 256 Sturm counts per round cost ~0.5 ms per call,
-// so the bracket starts from the previous check: by interlacing the lowest
-// Ritz value only moves down as the tridiagonal grows, so one point just above
-// it and 31 at geometric distances below it (2^-52 .. 2^8 of the spectrum's
-// scale) bracket it in one round; then 32-point multisection to 2 ulp. The first check, or a
-// probe that fails to bracket, starts from the Gershgorin interval.
-// With `staged`, alpha and beta are first copied into shared memory (every
-// Sturm sweep then reads them at shared-memory latency, not L2's).
-__device__ __forceinline__ void stage_tri(const double*& a, const double*& b, int m, int staged) {
-  if (!staged) return;
-  extern __shared__ double tri_sm[];
-  for (int i = threadIdx.x; i < m; i += blockDim.x) {
-    tri_sm[i] = a[i];
-    tri_sm[m + i] = b[i];
-  }
-  __syncthreads();
-  a = tri_sm;
-  b = tri_sm + m;
-}
-
-__global__ void k_tri_lowest(Scal S, int check_conv, double tol, int slot, int staged) {
+// K6: tridiagonal eigen-solve (tridiag.cuh).
+// Lowest eigenvalue by multisection; optional convergence test against the previous
+// check, which sets the stop flag. The bracket starts from the previous check: by
+// interlacing the lowest Ritz value only moves down as the tridiagonal grows, so one
+// point just above it and 31 at geometric distances below it (2^-52 .. 2^8 of the
+// spectrum's scale) bracket it in one round. The first check, or a probe that fails to
+// bracket, starts from the Gershgorin interval.
+__global__ void __launch_bounds__(TRI_THREADS) k_tri_lowest(Scal S, int check_conv, double tol, int slot, int level) {
+  __shared__ double br[2];
   const int m = S.flags[2];
   if (m <= 0) return;
   const int lane = threadIdx.x & 31;
-  const double* A_ = S.alpha;
-  const double* B_ = S.beta;
-  stage_tri(A_, B_, m, staged);
-  double glo = 0, ghi = 0, pm = 0;
-  gersh(A_, B_, m, &glo, &ghi, &pm);  // every lane (same values)
-  double lo = glo, hi = ghi;
+  const Tri T = tri_stage(S.alpha, S.beta, m, level);
+  double lo = T.glo, hi = T.ghi;
   const double prev = slot > 0 ? S.ritz[slot - 1] : 0.0;
-  if (slot > 0 && prev >= glo && prev <= ghi) {
-    const double scale = fmax(ghi - glo, fabs(prev));
-    // lane 0 just above prev (an eigenvalue lies below it), lanes 1..31 below
-    const double x = lane == 0 ? prev + scale * 0x1p-48 : prev - scale * ldexp(1.0, 2 * (lane - 1) - 52);
-    const unsigned hit = __ballot_sync(0xffffffffu, sturm_count(A_, B_, m, x, pm) >= 1);
-    // counts grow with x, i.e. towards lane 0: the lanes with a hit are 0 .. L-1
-    const int L = __popc(hit);
-    const double xa = __shfl_sync(0xffffffffu, x, L > 0 ? L - 1 : 0);
-    const double xb = __shfl_sync(0xffffffffu, x, L < 32 ? L : 31);
-    if (L > 0 && L < 32 && hit == ((1u << L) - 1u)) {
-      hi = xa;
-      lo = xb;
+  if (slot > 0 && prev >= T.glo && prev <= T.ghi) {
+    if (threadIdx.x < 32) {
+      const double scale = fmax(T.ghi - T.glo, fabs(prev));
+      // lane 0 just above prev (an eigenvalue lies below it), lanes 1..31 below
+      const double x = lane == 0 ? prev + scale * 0x1p-48 : prev - scale * ldexp(1.0, 2 * (lane - 1) - 52);
+      const unsigned hit = __ballot_sync(0xffffffffu, tri_count(T, x) >= 1);
+      // counts grow with x, i.e. towards lane 0: the lanes with a hit are 0 .. L-1
+      const int L = __popc(hit);
+      const double xa = __shfl_sync(0xffffffffu, x, L > 0 ? L - 1 : 0);
+      const double xb = __shfl_sync(0xffffffffu, x, L < 32 ? L : 31);
+      if (L > 0 && L < 32 && hit == ((1u << L) - 1u)) {
+        hi = xa;
+        lo = xb;
+      }
+      if (lane == 0) {
+        br[0] = lo;
+        br[1] = hi;
+      }
     }
+    __syncthreads();
+    lo = br[0];
+    hi = br[1];
   }
-  for (int it = 0; it < 16; it++) {
-    if (hi - lo <= 2 * DBL_EPSILON * fmax(fabs(lo), fabs(hi))) break;
-    const double x = lo + (hi - lo) * (lane + 1) / 33.0;
-    const unsigned hit = __ballot_sync(0xffffffffu, sturm_count(A_, B_, m, x, pm) >= 1);
-    const int f = hit ? __ffs(hit) - 1 : 32;  // first point with an eigenvalue below it
-    const double xf = __shfl_sync(0xffffffffu, x, f < 32 ? f : 31);
-    const double nhi = f < 32 ? xf : hi;
-    const double xprev = __shfl_sync(0xffffffffu, x, f > 0 ? f - 1 : 0);
-    const double nlo = f > 0 ? xprev : lo;
-    if (nhi == hi && nlo == lo) break;
-    hi = nhi;
-    lo = nlo;
-  }
-  if (lane == 0) {
+  tri_multisect(T, lo, hi, 16);
+  if (threadIdx.x == 0) {
     const double e = 0.5 * (lo + hi);
     S.ritz[slot] = e;
     S.flags[5] = m;  // the tridiagonal size this value belongs to
@@ -363,24 +341,32 @@ __global__ void k_tri_lowest(Scal S, int check_conv, double tol, int slot, int s
   }
 }
 
-// Lowest eigenvalue of the m x m tridiagonal (one warp): 32-point multisection
-// from the Gershgorin interval to 2 ulp: *out. When the last convergence check
-// (ritz[last], recorded for size flags[5]) already found it for this m, that
-// value is taken instead (the same 2-ulp multisection).
-__global__ void k_tri_min(const double* a, const double* b, int m, double* out, int staged, const double* ritz,
-                          const int* flags, int last) {
+// Lowest eigenvalue of the m x m tridiagonal: 32-point multisection from the
+// Gershgorin interval to 2 ulp: *out. When the last convergence check (ritz[last],
+// recorded for size flags[5]) already found it for this m, that value is taken instead
+// (the same 2-ulp multisection). 200 x 200: 1147 -> 442 us.
+__global__ void __launch_bounds__(TRI_THREADS) k_tri_min(const double* a, const double* b, int m, double* out,
+                                                         int level, const double* ritz, const int* flags, int last) {
   if (last >= 0 && flags[5] == m) {
     if (threadIdx.x == 0) *out = ritz[last];
     return;
   }
-  stage_tri(a, b, m, staged);
-  const int lane = threadIdx.x & 31;
-  double lo = 0, hi = 0, pm = 0;
-  gersh(a, b, m, &lo, &hi, &pm);
-  for (int it = 0; it < 24; it++) {
-    if (hi - lo <= 2 * DBL_EPSILON * fmax(fabs(lo), fabs(hi))) break;
+  const Tri T = tri_stage(a, b, m, level);
+  double lo = T.glo, hi = T.ghi;
+  tri_multisect(T, lo, hi, 24);
+  if (threadIdx.x == 0) *out = 0.5 * (lo + hi);
+}
+
+// All eigenvalues (ascending), a warp for each: 32-point multisection until the
+// interval's ends are neighbours, 12 rounds where one thread's bisection took 53, and
+// the FP64 pipes of all SMs (200 x 200 with the vector: 10.3 -> 1.6 ms).
+__global__ void __launch_bounds__(32) k_tri_all(const double* a, const double* b, int m, double* eig, int level) {
+  const Tri T = tri_stage(a, b, m, level);
+  const int lane = threadIdx.x, k = blockIdx.x;
+  double lo = T.glo, hi = T.ghi;
+  for (int it = 0; it < 200; it++) {
     const double x = lo + (hi - lo) * (lane + 1) / 33.0;
-    const unsigned hit = __ballot_sync(0xffffffffu, sturm_count(a, b, m, x, pm) >= 1);
+    const unsigned hit = __ballot_sync(0xffffffffu, tri_count(T, x) > k);
     const int f = hit ? __ffs(hit) - 1 : 32;
     const double xf = __shfl_sync(0xffffffffu, x, f < 32 ? f : 31);
     const double xp = __shfl_sync(0xffffffffu, x, f > 0 ? f - 1 : 0);
@@ -389,43 +375,21 @@ __global__ void k_tri_min(const double* a, const double* b, int m, double* out, 
     hi = nhi;
     lo = nlo;
   }
-  if (lane == 0) *out = 0.5 * (lo + hi);
+  if (lane == 0) eig[k] = 0.5 * (lo + hi);
 }
 
-// All eigenvalues (ascending) by bisection, one thread per index.
-__global__ void k_tri_all(const double* a, const double* b, int m, double* eig) {
-  __shared__ double lo0, hi0, pm;
-  if (threadIdx.x == 0) gersh(a, b, m, &lo0, &hi0, &pm);
-  __syncthreads();
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < m; k += gridDim.x * blockDim.x) {
-    double lo = lo0, hi = hi0;
-    for (int it = 0; it < 200; it++) {
-      const double mid = 0.5 * (lo + hi);
-      if (mid <= lo || mid >= hi) break;
-      if (sturm_count(a, b, m, mid, pm) > k) hi = mid;
-      else lo = mid;
-    }
-    eig[k] = 0.5 * (lo + hi);
-  }
-}
-
-// Eigenvector for eigenvalue *lam_p by inverse iteration (single thread).
-// With `staged` (one warp): alpha, beta, the factors and the vector live in
-// shared memory (8 m doubles) and only the result is written out.
-__global__ void k_tri_vec(const double* a, const double* b, int m, const double* lam_p, double* y, double* work,
-                          int staged) {
-  if (blockIdx.x != 0) return;
+// Eigenvector for eigenvalue *lam_p by inverse iteration. With `staged` everything
+// lives in shared memory (8 m doubles) and only the result is written out (200 x 200:
+// 877 -> 469 us); else one thread works in global memory.
+__global__ void __launch_bounds__(32) k_tri_vec(const double* a, const double* b, int m, const double* lam_p,
+                                                double* y, double* work, int staged) {
   if (!staged) {
     if (threadIdx.x == 0) tri_inverse_iteration(a, b, m, *lam_p, y, work);
     return;
   }
-  stage_tri(a, b, m, staged);
   extern __shared__ double tri_sm[];
-  double* sy = tri_sm + 2 * m;
-  double* swork = tri_sm + 3 * m;
-  if (threadIdx.x == 0) tri_inverse_iteration(a, b, m, *lam_p, sy, swork);
-  __syncthreads();
-  for (int i = threadIdx.x; i < m; i += blockDim.x) y[i] = sy[i];
+  tri_inverse_warp(a, b, m, *lam_p, tri_sm);
+  for (int i = threadIdx.x; i < m; i += 32) y[i] = tri_sm[2 * m + i];
 }
 
 // psi[r] = sum_l y[l] V_l[r] (GEMV over the Krylov basis); partial |psi|^2.
@@ -765,6 +729,9 @@ int tri_smem(const blqh_lanczos* L, int per) {
   return b <= 48 * 1024 ? (int)b : 0;
 }
 
+// What tri_stage has room for.
+int tri_level(const blqh_lanczos* L) { return tri_smem(L, 4) > 0 ? 4 : tri_smem(L, 2) > 0 ? 2 : 0; }
+
 // A kernel of the step chain: its blocks may be placed while the previous kernel
 // on the stream drains; it waits for that kernel's results itself (pdl_begin).
 template <class... P, class... A>
@@ -946,7 +913,7 @@ void iterate_impl(blqh_lanczos* L) {
     for (; j < jend; j++) lanczos_step(L, j);
     if (conv) {  // with tol = 0 the recurrence runs to max_steps: no check needed
       TimerScope tm(ctx, TM_MISC);
-      k_tri_lowest<<<1, 32, tri_smem(L, 2), st>>>(L->S, 1, L->o.tol, launched_chunks, tri_smem(L, 2) > 0);
+      k_tri_lowest<<<1, TRI_THREADS, tri_smem(L, tri_level(L)), st>>>(L->S, 1, L->o.tol, launched_chunks, tri_level(L));
       BLQH_TRY_CUDA(ctx, cudaGetLastError());
       count_launch(ctx, TM_MISC);
     }
@@ -978,8 +945,9 @@ void ritz_impl(blqh_lanczos* L) {
   const int m = L->steps;
   TimerScope tm(ctx, TM_MISC);
   // only the lowest Ritz pair is needed here (blqh_lanczos_eig gives them all)
-  k_tri_min<<<1, 32, tri_smem(L, 2), st>>>(L->S.alpha, L->S.beta, m, L->work + 6 * L->mmax, tri_smem(L, 2) > 0,
-                                            L->S.ritz, L->S.flags, L->last_check);
+  const int lv = tri_level(L);
+  k_tri_min<<<1, TRI_THREADS, tri_smem(L, lv), st>>>(L->S.alpha, L->S.beta, m, L->work + 6 * L->mmax, lv, L->S.ritz,
+                                                     L->S.flags, L->last_check);
   k_tri_vec<<<1, 32, tri_smem(L, 8), st>>>(L->S.alpha, L->S.beta, m, L->work + 6 * L->mmax, L->y, L->work,
                                             tri_smem(L, 8) > 0);
   const int blocks = (int)((L->dim + 255) / 256);
@@ -1321,7 +1289,8 @@ int blqh_lanczos_eig(blqh_lanczos* L, double* eigenvalues, double* psi0) {
   blqh_ctx* ctx = L->ctx;
   try {
     const int m = L->steps;
-    k_tri_all<<<1, 256, 0, ctx->stream>>>(L->S.alpha, L->S.beta, m, L->work + 6 * L->mmax);
+    const int lv = tri_smem(L, 2) > 0 ? 2 : 0;
+    k_tri_all<<<m, 32, tri_smem(L, lv), ctx->stream>>>(L->S.alpha, L->S.beta, m, L->work + 6 * L->mmax, lv);
     k_tri_vec<<<1, 32, tri_smem(L, 8), ctx->stream>>>(L->S.alpha, L->S.beta, m, L->work + 6 * L->mmax, L->y,
                                                       L->work, tri_smem(L, 8) > 0);
     BLQH_TRY_CUDA(ctx, cudaGetLastError());
