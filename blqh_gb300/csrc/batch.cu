@@ -1072,9 +1072,12 @@ void batch_create_impl(blqh_batch* b) {
   // the number of instances), the x area takes what shared memory is left, so that
   // the gathers of larger complex instances stay in it.
   if (b->nrun && (b->bps == 1 || b->nrun <= ctx->num_sms)) {
-    const int64_t cap = std::min<int64_t>(max_n * 8, smem_max - fixed - 64);
+    cudaFuncAttributes fa;  // the kernel's own static shared memory counts against the limit
+    BLQH_TRY_CUDA(ctx, cudaFuncGetAttributes(&fa, reinterpret_cast<const void*>(b->kern)));
+    const int64_t room = (smem_max - fixed - (int64_t)fa.sharedSizeBytes) / 16 * 16;
+    const int64_t cap = std::min<int64_t>((max_n * 8 + 15) / 16 * 16, room);
     if (cap > b->x_cap) {
-      b->smem = fixed + (int)((cap + 15) / 16 * 16);
+      b->smem = fixed + (int)cap;
       configure_shape(b, b->threads, b->lpr);
       for (BInst& I : hi)
         if (I.cplx) I.xsmem = I.dim * 16 <= cap;

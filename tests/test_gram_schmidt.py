@@ -133,3 +133,26 @@ def test_batched_complex_instances(B, prec):
         assert abs(np.linalg.norm(psi) - 1) < 1e-12
         assert 1 - abs(np.vdot(psi, ref["psi"])) < 1e-10
     b.close()
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+def test_batched_vectors_larger_than_shared_memory(B, prec):
+    """Batches whose largest vector is beyond (418 kB), within (174 kB) and far below a block's shared memory: the
+    area for it stops at what the kernel's own variables leave. 150 steps converge to 1e-10; FP32 values to 1e-9."""
+    secs = [(12, 10, 5, 9, 3), (12, 9, 4, 5, 3), (12, 8, 4, 5, 3)]
+    ref = []
+    for s in secs:
+        bas = B.Basis(*s)
+        H = B.Hamiltonian(bas, 0.9)
+        L = B.Lanczos(H, max_steps=200, tol=0.0)
+        L.iterate()
+        ref.append(L.eig()[0][0])
+        for x in (L, H, bas):
+            x.close()
+    for pick in ([0], [1], [0, 2], [0, 1, 2]):
+        b = B.Batch([B.instance(*secs[i], 0.9) for i in pick], lam=150,
+                    precision=B.VAL_FP64 if prec == "f64" else B.VAL_FP32)
+        b.solve()
+        for i, r in zip(pick, b.results()):
+            assert abs(r["energy"] - ref[i]) < (1e-10 if prec == "f64" else 1e-9)
+        b.close()
