@@ -540,7 +540,8 @@ def run_sweep_workload(args):
         "sweep_solve_s": run["solve_s"], "sweep_create_s": run["create_s"],
         "fp64_sweep_solve_s": r64["solve_s"], "fp64_over_mixed_solve": r64["solve_s"] / run["solve_s"],
         "max_abs_dE_mixed_vs_fp64": float(np.max(np.abs(e32[ok] - e64[ok]))),
-        "roofline": {"kernel": "k_batch_lanczos (reorthogonalization + Ritz vector in FP64)", "bound": "fp64",
+        "roofline": {"kernel": "k_batch_lanczos (reorthogonalization + Ritz vector as FP64 operations; complex instances "
+                               "do theirs in integers)", "bound": "fp64",
                      "achieved": achieved, "peak": peak, "unit": "GFLOP/s", "frac": achieved / peak,
                      "peak_source": "measured (cuBLAS FP64 GEMM through torch.matmul, 4096^3)",
                      "flops": flops, "lanczos_ms": run["lanczos_ms"], "finish_ms": run["finish_ms"]},
