@@ -723,14 +723,18 @@ void spmv_dev(blqh_ctx* ctx, const blqh_csr* M, const double* x, double* y, cons
 }
 
 // Dynamic shared memory of the tridiagonal kernels: `per` doubles per Lanczos
-// step when that fits in 48 KB, else 0 (they then read global memory).
-int tri_smem(const blqh_lanczos* L, int per) {
+// step when that and the kernel's `fixed` bytes of static shared memory fit in
+// 48 KB, else 0 (they then read global memory).
+int tri_smem(const blqh_lanczos* L, int per, size_t fixed = 0) {
   const size_t b = (size_t)per * (L->mmax + 1) * sizeof(double);
-  return b <= 48 * 1024 ? (int)b : 0;
+  return b + fixed <= 48 * 1024 ? (int)b : 0;
 }
 
-// What tri_stage has room for.
-int tri_level(const blqh_lanczos* L) { return tri_smem(L, 4) > 0 ? 4 : tri_smem(L, 2) > 0 ? 2 : 0; }
+// What tri_stage has room for next to k_tri_lowest's bracket.
+int tri_level(const blqh_lanczos* L) {
+  const size_t bracket = 2 * sizeof(double);
+  return tri_smem(L, 4, bracket) > 0 ? 4 : tri_smem(L, 2, bracket) > 0 ? 2 : 0;
+}
 
 // A kernel of the step chain: its blocks may be placed while the previous kernel
 // on the stream drains; it waits for that kernel's results itself (pdl_begin).
