@@ -73,8 +73,8 @@ MemberTable build_members(blqh_ctx* ctx, DevBufs& G, const blqh_basis* B, ROT ro
   const int64_t members = B->dim * (orbits ? per_orbit : 1);
   uint64_t slots = 1024;
   while (slots < (uint64_t)(2 * members)) slots <<= 1;
-  uint64_t* key = G.add(dalloc<uint64_t>(ctx, slots));
-  uint32_t* val = G.add(dalloc<uint32_t>(ctx, slots));
+  uint64_t* key = G.add(static_cast<uint64_t*>(dev_alloc(ctx, slots * (sizeof(uint64_t) + sizeof(uint32_t)))));
+  uint32_t* val = reinterpret_cast<uint32_t*>(key + slots);
   BLQH_TRY_CUDA(ctx, cudaMemsetAsync(key, 0xFF, slots * 8, ctx->stream));
   TimerScope tb(ctx, TM_BUILD);
   k_member_insert<<<grid_for(ctx, B->dim, 256), 256, 0, ctx->stream>>>(rot, B->d_id, B->d_period, B->dim, orbits, key,

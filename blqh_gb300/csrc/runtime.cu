@@ -6,6 +6,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "../../include/blqh_gpu_debug.h"
 #include "blqh_internal.h"
 
 static thread_local std::string g_thread_error;
@@ -71,6 +72,10 @@ void release_cached(blqh_ctx* only) {
 
 void* dev_alloc(blqh_ctx* ctx, size_t bytes) {
   const size_t b = bucket_bytes(bytes);
+  if (ctx && ctx->fail_alloc > 0 && --ctx->fail_alloc == 0) {
+    set_error(ctx, BLQH_ERR_NOMEM, "device allocation of " + std::to_string(bytes) + " bytes failed: on request");
+    throw BlqhError{BLQH_ERR_NOMEM, "fail_alloc"};
+  }
   {
     std::lock_guard<std::mutex> lk(g_mem_mu);
     auto it = g_cache.find({ctx, b});
@@ -333,6 +338,13 @@ void scan_exclusive_u32_to_i64(blqh_ctx* ctx, const uint32_t* in, int64_t* out, 
 
 // ---------------------------------------------------------------------------
 extern "C" {
+
+int64_t blqh_debug_fail_alloc(blqh_ctx* ctx, int64_t n) {
+  if (!ctx) return 0;
+  const int64_t left = ctx->fail_alloc;
+  ctx->fail_alloc = n;
+  return left;
+}
 
 int blqh_ctx_create(int device, blqh_ctx** out) {
   if (!out) return BLQH_ERR_ARG;

@@ -234,6 +234,30 @@ __device__ __forceinline__ int table_slot(const RowTable& T, int j) {
   return -1;
 }
 
+// Row of the representative of state c's orbit (-1: not in the basis) and how many
+// inverse translations away it is: from the orbit-member table (TAB) or, where that has
+// no memory or the basis more rows than its 32-bit entries hold, by a search per
+// translation.
+template <bool TAB>
+__device__ __forceinline__ int64_t orbit_row(const MemberTable& T, const uint64_t* id, int64_t dim, int nphi, int K,
+                                             uint64_t c, int* q) {
+  if (TAB) {
+    uint32_t v;
+    if (!member_find(T, c, &v)) return -1;
+    *q = (int)(v & 31);
+    return v >> 5;
+  }
+  for (int k = 0; k < (K < 0 ? 1 : nphi); k++) {
+    int par;
+    const int64_t j = find_key(id, dim, k ? rot4(c, k, nphi, 1, &par) : c);
+    if (j >= 0) {
+      *q = k;
+      return j;
+    }
+  }
+  return -1;
+}
+
 // Sum over the translates of a row state (period Dl) of sign * FT for a target
 // reached from the untranslated state, whose orbit (period Dr) has its
 // representative qr translations away: (re, im) without 1 / sqrt(Dl Dr).
@@ -266,12 +290,12 @@ __device__ __forceinline__ double2 translate_sum(const SpinGen& G, uint64_t rb0,
 }
 
 // Adds the contribution of target rbasis_0 (before the right-hand translations) to the row.
-template <bool CPLX>
+template <bool CPLX, bool TAB>
 __device__ __forceinline__ void add_target(const SpinGen& G, const RowTable& T, uint64_t rb0, int ql, int Dl, int parl,
                                            int parh, double amp_re, double amp_im) {
-  uint32_t mv;
-  if (!member_find(G.mem, rb0, &mv)) return;
-  const int j = (int)(mv >> 5), qr = (int)(mv & 31);
+  int qr;
+  const int j = (int)orbit_row<TAB>(G.mem, G.id, G.dim, G.nphi, G.K, rb0, &qr);
+  if (j < 0) return;
   const int Dr = G.K < 0 ? 1 : G.period[j];
   double2 f;
   if (G.literal) {
@@ -309,7 +333,7 @@ __device__ __forceinline__ int nth_bit(uint64_t c, int k) {
 // in column order, FP64, nothing stored.
 constexpr int SPIN_THREADS = 128;
 
-template <bool CPLX>
+template <bool CPLX, bool TAB>
 __global__ void __launch_bounds__(SPIN_THREADS)
     k_spin_rows(SpinGen G, int pass, int slots, int64_t stride, int64_t* __restrict__ row_nnz,
                 const int64_t* __restrict__ row_ptr, int32_t* __restrict__ col, double* __restrict__ val, int* overflow,
@@ -368,7 +392,7 @@ __global__ void __launch_bounds__(SPIN_THREADS)
           are = v * cos(G.theta_y * t / nphi);
           aim = v * sin(G.theta_y * t / nphi);
         }
-        add_target<CPLX>(G, acc, mt_mask | b, ql, Dl, parl, pair_parity(lb, n, m, nt, mt), are, aim);
+        add_target<CPLX, TAB>(G, acc, mt_mask | b, ql, Dl, parl, pair_parity(lb, n, m, nt, mt), are, aim);
       } else {
         w -= hop_items;
         const int kind = w / nphi, r = w % nphi;
@@ -389,7 +413,7 @@ __global__ void __launch_bounds__(SPIN_THREADS)
         const uint64_t rb0 = lb - kn + (kn ^ mask);
         double cr = 1.0, ci = 0.0;
         if (CPLX && ph != 0.0) sincos(ph, &ci, &cr);
-        add_target<CPLX>(G, acc, rb0, ql, Dl, parl, empties_between(lb, lo, hi), amp * cr, amp * ci);
+        add_target<CPLX, TAB>(G, acc, rb0, ql, Dl, parl, empties_between(lb, lo, hi), amp * cr, amp * ci);
       }
     }
     __syncthreads();
@@ -508,6 +532,7 @@ __constant__ int c_move_pairs[8][2] = {{0, 2}, {2, 0}, {1, 3}, {3, 1}, {0, 3}, {
 
 // One warp per state: for each move pair the lanes take (translate, orbital), the
 // target's representative comes from the orbit-member table.
+template <bool TAB>
 __global__ void __launch_bounds__(256) k_spin_observables(const uint64_t* __restrict__ id,
                                                           const uint8_t* __restrict__ period, MemberTable mem,
                                                           const double2* __restrict__ FT,
@@ -552,10 +577,10 @@ __global__ void __launch_bounds__(256) k_spin_observables(const uint64_t* __rest
         const uint64_t kn = lb & mask;
         if (kn == mask || kn == 0) continue;
         const uint64_t rb0 = lb ^ mask;
-        uint32_t mv;
-        if (!member_find(mem, rb0, &mv)) continue;
-        const int64_t jj = mv >> 5;
-        const int qr = (int)(mv & 31), Dr = K < 0 ? 1 : period[jj];
+        int qr;
+        const int64_t jj = orbit_row<TAB>(mem, id, dim, nphi, K, rb0, &qr);
+        if (jj < 0) continue;
+        const int Dr = K < 0 ? 1 : period[jj];
         int parr = 0;
         if (qr) rot4(rb0, qr, nphi, 1, &parr);
         const int hpar = empties_between(lb, n < nt ? n : nt, n < nt ? nt : n);
@@ -714,7 +739,12 @@ SpinTables spin_tables(blqh_ctx* ctx, const blqh_basis* B, DevBufs& G, int* derr
   SpinTables T;
   T.FT = reinterpret_cast<const double2*>(d);
   T.isq = d + 2 * (2 * nphi - 1);
-  T.mem = build_members(ctx, G, B, SpinRot{nphi}, s.K >= 0, nphi, derr);
+  if (B->dim < ((int64_t)1 << 27)) try {
+      T.mem = build_members(ctx, G, B, SpinRot{nphi}, s.K >= 0, nphi, derr);
+    } catch (const BlqhError& e) {
+      if (e.code != BLQH_ERR_NOMEM) throw;
+      ctx->last_error.clear();  // T.mem stays empty: orbit_row searches
+    }
   return T;
 }
 
@@ -725,7 +755,7 @@ struct SpinSetup {
   int slots = 0;
   int64_t stride = 0;  // a row's largest number of entries
   size_t smem = 0;
-  decltype(&k_spin_rows<true>) rows = nullptr;
+  decltype(&k_spin_rows<true, true>) rows = nullptr;
   int grid = 0;
 };
 
@@ -782,7 +812,8 @@ SpinSetup spin_setup(blqh_ctx* ctx, const blqh_basis* B, const blqh_params_spin&
     throw BlqhError{BLQH_ERR_UNSUPPORTED, "spin row table"};
   }
   S.stride = moves;
-  S.rows = S.cplx ? k_spin_rows<true> : k_spin_rows<false>;
+  if (T.mem.key) S.rows = S.cplx ? k_spin_rows<true, true> : k_spin_rows<false, true>;
+  else S.rows = S.cplx ? k_spin_rows<true, false> : k_spin_rows<false, false>;
   BLQH_TRY_CUDA(ctx, smem_attr_at_least(S.rows, (int)S.smem));
   S.grid = (int)std::min<int64_t>(B->dim, (int64_t)ctx->num_sms * 16);
   return S;
@@ -829,29 +860,42 @@ void build_spin_hamil(blqh_ctx* ctx, const blqh_basis* B, const blqh_params_spin
   M->precision = BLQH_VAL_FP64;
   M->d_row_ptr = dalloc<int64_t>(ctx, dim + 1);
   // rows are generated once into a staging buffer that holds any row when it fits
-  // in 8 GB, else twice (counted, then written)
-  const bool staged = (double)dim * S.stride * (4 + 8 * vw) <= 8.0 * (1ULL << 30);
-  int32_t* scol = staged ? G.add(dalloc<int32_t>(ctx, (size_t)dim * S.stride)) : nullptr;
-  double* sval = staged ? G.add(dalloc<double>(ctx, (size_t)dim * S.stride * vw)) : nullptr;
+  // in 8 GB and the device has that memory, else twice (counted, then written)
   TimerScope ts(ctx, TM_BUILD);
-  S.rows<<<S.grid, SPIN_THREADS, S.smem, ctx->stream>>>(S.g, staged ? 3 : 0, S.slots, S.stride, M->d_row_ptr, nullptr,
-                                                        scol, sval, over, nullptr, nullptr);
-  BLQH_TRY_CUDA(ctx, cudaGetLastError());
   int64_t nnz = 0;
-  scan_exclusive_i64(ctx, M->d_row_ptr, M->d_row_ptr, dim, &nnz);
-  BLQH_TRY_CUDA(ctx, cudaMemcpyAsync(M->d_row_ptr + dim, &nnz, 8, cudaMemcpyHostToDevice, ctx->stream));
-  M->nnz = nnz;
-  M->mean_row = dim ? (double)nnz / dim : 0;
-  M->d_col = dalloc<int32_t>(ctx, std::max<int64_t>(1, nnz));
-  M->d_val = dev_alloc(ctx, std::max<int64_t>(1, nnz) * (cplx ? 16 : 8) + 16);
-  double* val = reinterpret_cast<double*>(M->d_val);
-  if (staged)
-    k_spin_unstage<<<grid_for(ctx, dim * 32, 256), 256, 0, ctx->stream>>>(scol, sval, S.stride, vw, M->d_row_ptr, dim,
-                                                                          M->d_col, val);
-  else
-    S.rows<<<S.grid, SPIN_THREADS, S.smem, ctx->stream>>>(S.g, 1, S.slots, S.stride, nullptr, M->d_row_ptr, M->d_col,
-                                                          val, over, nullptr, nullptr);
-  BLQH_TRY_CUDA(ctx, cudaGetLastError());
+  auto passes = [&](bool staged) {
+    DevBufs stage;
+    int32_t* scol = staged ? stage.add(dalloc<int32_t>(ctx, (size_t)dim * S.stride)) : nullptr;
+    double* sval = staged ? stage.add(dalloc<double>(ctx, (size_t)dim * S.stride * vw)) : nullptr;
+    S.rows<<<S.grid, SPIN_THREADS, S.smem, ctx->stream>>>(S.g, staged ? 3 : 0, S.slots, S.stride, M->d_row_ptr,
+                                                          nullptr, scol, sval, over, nullptr, nullptr);
+    BLQH_TRY_CUDA(ctx, cudaGetLastError());
+    scan_exclusive_i64(ctx, M->d_row_ptr, M->d_row_ptr, dim, &nnz);
+    BLQH_TRY_CUDA(ctx, cudaMemcpyAsync(M->d_row_ptr + dim, &nnz, 8, cudaMemcpyHostToDevice, ctx->stream));
+    M->nnz = nnz;
+    M->mean_row = dim ? (double)nnz / dim : 0;
+    M->d_col = dalloc<int32_t>(ctx, std::max<int64_t>(1, nnz));
+    M->d_val = dev_alloc(ctx, std::max<int64_t>(1, nnz) * (cplx ? 16 : 8) + 16);
+    double* val = reinterpret_cast<double*>(M->d_val);
+    if (staged)
+      k_spin_unstage<<<grid_for(ctx, dim * 32, 256), 256, 0, ctx->stream>>>(scol, sval, S.stride, vw, M->d_row_ptr,
+                                                                            dim, M->d_col, val);
+    else
+      S.rows<<<S.grid, SPIN_THREADS, S.smem, ctx->stream>>>(S.g, 1, S.slots, S.stride, nullptr, M->d_row_ptr,
+                                                            M->d_col, val, over, nullptr, nullptr);
+    BLQH_TRY_CUDA(ctx, cudaGetLastError());
+  };
+  bool done = false;
+  if ((double)dim * S.stride * (4 + 8 * vw) <= 8.0 * (1ULL << 30)) try {
+      passes(true);
+      done = true;
+    } catch (const BlqhError& e) {
+      if (e.code != BLQH_ERR_NOMEM) throw;
+      dev_free(M->d_col);
+      M->d_col = nullptr;
+      ctx->last_error.clear();
+    }
+  if (!done) passes(false);
   count_launch(ctx, TM_BUILD, 2);
   check_overflow(ctx, over);
   if (prec == BLQH_VAL_FP32) {  // FP32 values, rounded from the FP64 sums
@@ -882,8 +926,9 @@ void spin_observables_impl(blqh_ctx* ctx, const blqh_basis* B, const double* psi
   const SpinTables T = spin_tables(ctx, B, G, derr);
   {
     TimerScope tm(ctx, TM_MISC);
-    k_spin_observables<<<grid, 256, 0, ctx->stream>>>(B->d_id, B->d_period, T.mem, T.FT, T.isq, B->dim, nphi,
-                                                      B->ssector.K, psi, cplx, part);
+    auto kern = T.mem.key ? k_spin_observables<true> : k_spin_observables<false>;
+    kern<<<grid, 256, 0, ctx->stream>>>(B->d_id, B->d_period, T.mem, T.FT, T.isq, B->dim, nphi, B->ssector.K, psi, cplx,
+                                        part);
     BLQH_TRY_CUDA(ctx, cudaGetLastError());
     count_launch(ctx, TM_MISC);
   }

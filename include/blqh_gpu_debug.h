@@ -1,7 +1,7 @@
-/* blqh_gpu_debug.h — host-only inspection entry points of libblqh_gpu.so.
+/* blqh_gpu_debug.h — inspection entry points of libblqh_gpu.so.
  *
- * They run on the CPU (no device needed) and expose internals that the tests
- * check against the oracle. Not part of the reference's interface.
+ * They expose internals that the tests check. Not part of the reference's
+ * interface. blqh_debug_sector_index needs no device.
  */
 #ifndef BLQH_GPU_DEBUG_H
 #define BLQH_GPU_DEBUG_H
@@ -26,6 +26,11 @@ int blqh_debug_sector_index(const blqh_sector* s, int64_t n, const uint64_t* sta
  * table; real matrices with few distinct values), 0 when the row-wise CSR
  * kernels are used; -1 for a null matrix. */
 int blqh_debug_spmv_layout(const blqh_csr* M);
+
+/* The n-th device allocation that the library makes for this context from now
+ * on fails with BLQH_ERR_NOMEM, once (n = 0: none). Returns what was left of
+ * the previous request: 0 when it has been met (or none was made). */
+int64_t blqh_debug_fail_alloc(blqh_ctx* ctx, int64_t n);
 
 #ifdef __cplusplus
 }

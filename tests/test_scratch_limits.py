@@ -1,0 +1,95 @@
+"""Calls whose fast route needs more device memory than their plain one take the plain one where the memory is not
+there. Every allocation of a call is made to fail in turn: the call then either reports BLQH_ERR_NOMEM or returns what
+it returns otherwise, and the context stays usable."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+NOMEM = -3
+
+
+@pytest.fixture()
+def ctx():
+    import blqh_gb300 as B
+
+    c = B.Context(0)
+    yield c
+    c.close()
+
+
+def sweep(ctx, call, limit=400):
+    """Results of `call` with its 1st, 2nd, ... allocation failing (None: NOMEM), until none is left to fail."""
+    from blqh_gb300._lib import BlqhError, lib
+
+    out = []
+    for n in range(1, limit):
+        lib().blqh_debug_fail_alloc(ctx.h, n)
+        try:
+            r = call()
+        except BlqhError as e:
+            assert e.code == NOMEM, e
+            r = None
+        if lib().blqh_debug_fail_alloc(ctx.h, 0):
+            assert r is not None
+            return out
+        out.append(r)
+    raise AssertionError("more allocations than expected")
+
+
+SPIN = [  # even and odd nphi, with and without translation symmetry, real and complex, every route of the generator
+    ((4, 4, 2, 2, 0, 0), dict(delta_v=0.01, delta_z=0.02)), ((4, 4, -1, -1, 0, 1), dict(delta_sas=0.2)),
+    ((6, 6, 3, 3, 1, 2), {}), ((5, 3, 1, 1, 2, 1), {}), ((4, 3, 1, 1, 2, -1), dict(delta_v=0.01)),
+]
+
+
+@pytest.mark.parametrize("sec,kw", SPIN, ids=str)
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+def test_spinful_build(ctx, sec, kw, prec):
+    """The row generator's staging (two buffers) and its orbit-member table each fail over: rows counted, then written,
+    and targets searched. Same columns; values are sums of at most ~60 terms of size <= 2 in another order, 2e-14
+    (FP32 values: one rounding of entries below 16 apart, 1e-6)."""
+    import blqh_gb300 as B
+
+    p = B.VAL_FP64 if prec == "f64" else B.VAL_FP32
+    b = B.basis_spin(*sec, ctx=ctx)
+
+    def build():
+        H = B.hamiltonian_spin(b, 0.8, precision=p, **kw)
+        r = H.csr()
+        H.close()
+        return r
+
+    rp, col, val = build()
+    got = sweep(ctx, build)
+    assert sum(r is not None for r in got) >= 5  # table, two staging buffers, the CSR's two arrays
+    for r in got:
+        if r is not None:
+            assert np.array_equal(r[0], rp) and np.array_equal(r[1], col)
+            assert np.max(np.abs(r[2] - val)) < (2e-14 if prec == "f64" else 1e-6)
+    b.close()
+
+
+@pytest.mark.parametrize("sec,kw", SPIN, ids=str)
+def test_spinful_observables_and_regenerated_energy(ctx, sec, kw):
+    import blqh_gb300 as B
+
+    b = B.basis_spin(*sec, ctx=ctx)
+    H = B.hamiltonian_spin(b, 0.8, **kw)
+    L = B.Lanczos(H, max_steps=60)
+    L.iterate()
+    L.ritz_vector(copy=False)
+
+    def values():
+        o = L.observables_spin(b)
+        return np.concatenate([[v for k, v in sorted(o.items()) if k != "occupation"], o["occupation"].ravel()])
+
+    for call in (values, lambda: np.array([L.rayleigh_fp64()])):
+        ref = call()
+        got = sweep(ctx, call)
+        assert any(r is not None for r in got)  # the table
+        for r in got:
+            if r is not None:
+                assert np.max(np.abs(r - ref)) < 1e-12  # sums of a few thousand terms below 10 in another order
+    for x in (L, H, b):
+        x.close()
