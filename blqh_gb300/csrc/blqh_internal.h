@@ -48,7 +48,7 @@ struct blqh_ctx {
   std::vector<std::pair<int, std::pair<cudaEvent_t, cudaEvent_t>>> pending;
   // small pinned host buffer for scalar read-backs
   double* pinned = nullptr;
-  int64_t fail_alloc = 0;  // allocations until one is made to fail (blqh_debug_fail_alloc), 0: none
+  int fail_alloc = 0;  // allocations until one is made to fail (blqh_debug_fail_alloc), 0: none
 };
 
 // Device allocation that throws BlqhError on failure. Blocks are cached per

@@ -339,9 +339,9 @@ void scan_exclusive_u32_to_i64(blqh_ctx* ctx, const uint32_t* in, int64_t* out, 
 // ---------------------------------------------------------------------------
 extern "C" {
 
-int64_t blqh_debug_fail_alloc(blqh_ctx* ctx, int64_t n) {
+int blqh_debug_fail_alloc(blqh_ctx* ctx, int n) {
   if (!ctx) return 0;
-  const int64_t left = ctx->fail_alloc;
+  const int left = ctx->fail_alloc;
   ctx->fail_alloc = n;
   return left;
 }

@@ -30,7 +30,7 @@ int blqh_debug_spmv_layout(const blqh_csr* M);
 /* The n-th device allocation that the library makes for this context from now
  * on fails with BLQH_ERR_NOMEM, once (n = 0: none). Returns what was left of
  * the previous request: 0 when it has been met (or none was made). */
-int64_t blqh_debug_fail_alloc(blqh_ctx* ctx, int64_t n);
+int blqh_debug_fail_alloc(blqh_ctx* ctx, int n);
 
 #ifdef __cplusplus
 }
