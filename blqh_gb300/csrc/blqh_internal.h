@@ -137,10 +137,6 @@ struct blqh_csr {
   // element to 2^-48 for the final Rayleigh quotient; null otherwise
   void* d_res = nullptr;
   int lanes_per_row = 32;        // SpMV shape chosen by the tuner
-  // fixed-point copy of a complex FP64 matrix (spmv_fixed.cu), or null
-  void* d_qval = nullptr;        // [nnz] int4: (re, im) in two limbs each, 0 on the diagonal
-  int* d_qexp = nullptr;         // [dim] row exponents
-  double* d_qdiag = nullptr;     // [2 dim] diagonal
   double mean_row = 0;
   // blocked SpMV (spmv_blocked.cu): per (row block, column tile) slices of 32
   // rows sorted by entry count, stored column-major; blk_state 0 untried,
@@ -227,12 +223,19 @@ void blocked_spmv(blqh_ctx* ctx, const blqh_csr* M, const float2* xs, double* y,
                   const double* xprev, const int* stop);
 int blocked_error(blqh_ctx* ctx, const blqh_csr* M);
 
-// Fixed-point SpMV of complex FP64 matrices (spmv_fixed.cu).
-bool fixed_prepare(blqh_ctx* ctx, blqh_csr* M);
-void fixed_release(blqh_csr* M);
+// Fixed-point SpMV of complex FP64 matrices (spmv_fixed.cu). The split copy belongs to
+// the object that multiplies with it and is used on that object's stream only, so
+// that contexts, streams and threads can share a matrix; it goes with the object.
+struct FixedMatrix {
+  void* val = nullptr;     // [nnz] int4: (re, im) in two limbs each, 0 on the diagonal
+  int* row_exp = nullptr;  // [dim] row exponents
+  double* diag = nullptr;  // [2 dim] diagonal
+};
+bool fixed_prepare(blqh_ctx* ctx, const blqh_csr* M, FixedMatrix* F);
+void fixed_release(FixedMatrix* F);
 void fixed_vector(blqh_ctx* ctx, const double* x, int2* xq, int64_t n, const int* stop);
-void fixed_spmv(blqh_ctx* ctx, const blqh_csr* M, const double* x, const int2* xq, double* y, const double* bptr,
-                const double* xprev, const int* stop);
+void fixed_spmv(blqh_ctx* ctx, const blqh_csr* M, const FixedMatrix& F, const double* x, const int2* xq, double* y,
+                const double* bptr, const double* xprev, const int* stop);
 
 void scan_exclusive_i64(blqh_ctx* ctx, const int64_t* in, int64_t* out, int64_t n, int64_t* total_host);
 void scan_exclusive_u32_to_i64(blqh_ctx* ctx, const uint32_t* in, int64_t* out, int64_t n, int64_t* total_host);

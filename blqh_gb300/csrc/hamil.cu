@@ -1186,7 +1186,6 @@ void free_csr(blqh_csr* m) {
   dev_free(m->d_val);
   dev_free(m->d_res);
   blocked_release(m);
-  fixed_release(m);
   delete m;
 }
 

@@ -580,7 +580,8 @@ struct blqh_lanczos {
   double* work = nullptr;  // tridiagonal work [5*mmax + ...]
   double* y = nullptr;     // [mmax] Ritz coefficients
   float2* xs = nullptr;    // [dim * vw] (hi, lo) split of the SpMV input (double-float accumulation)
-  int2* xq = nullptr;      // [dim * 2] the same in fixed point (complex FP64 matrices)
+  FixedMatrix fx;          // the matrix in fixed point (complex FP64 matrices)
+  int2* xq = nullptr;      // [dim * 2] the SpMV input in fixed point
   // complex sectors: fixed-point planes of V and, in the last row, of w (or null)
   int* Q1 = nullptr;       // [(mmax+2) * pld]
   int* Q0 = nullptr;
@@ -602,6 +603,7 @@ namespace {
 void free_lanczos(blqh_lanczos* L) {
   if (!L) return;
   dev_free(L->xs);
+  fixed_release(&L->fx);
   dev_free(L->xq);
   dev_free(L->Q1);
   dev_free(L->Q0);
@@ -683,11 +685,11 @@ void spmv_df_t(blqh_ctx* ctx, const blqh_csr* M, const float2* xs, double* y, co
 }
 
 // y = H x - b xprev. With an FP32-valued CSR and a split buffer xs, the product
-// accumulates in double-float (k_spmv_df); with a fixed-point copy of the matrix and
+// accumulates in double-float (k_spmv_df); with a fixed-point copy fx of the matrix and
 // a buffer xq (|x| <= 1) in integers (k_spmv_fixed); otherwise in native FP64 (k_spmv).
 void spmv_dev(blqh_ctx* ctx, const blqh_csr* M, const double* x, double* y, const double* bptr = nullptr,
               const double* xprev = nullptr, const int* stop = nullptr, float2* xs = nullptr,
-              bool xs_ready = false, int2* xq = nullptr) {
+              bool xs_ready = false, const FixedMatrix* fx = nullptr, int2* xq = nullptr) {
   if (xs && M->precision == BLQH_VAL_FP32) {
     const int64_t n = M->dim * (M->is_complex ? 2 : 1);
     if (!xs_ready) {  // else the caller's previous kernel left x's split in xs
@@ -705,7 +707,7 @@ void spmv_dev(blqh_ctx* ctx, const blqh_csr* M, const double* x, double* y, cons
   if (xq) {  // fixed point (complex FP64)
     if (!xs_ready) fixed_vector(ctx, x, xq, M->dim * 2, stop);
     TimerScope ts(ctx, TM_SPMV);
-    fixed_spmv(ctx, M, x, xq, y, bptr, xprev, stop);
+    fixed_spmv(ctx, M, *fx, x, xq, y, bptr, xprev, stop);
     BLQH_TRY_CUDA(ctx, cudaGetLastError());
     count_launch(ctx, TM_SPMV);
     return;
@@ -856,7 +858,7 @@ void lanczos_step(blqh_lanczos* L, int j) {
   const double* vprev = j > 0 ? L->V + (int64_t)(j - 1) * n : nullptr;
   // from the second step on, the previous step left v_j's split in xs
   spmv_dev(ctx, L->M, vj, L->w, j > 0 ? L->S.beta + j : nullptr, vprev, L->S.flags, L->xs, j > 0,
-           L->xq);
+           &L->fx, L->xq);
   // three-term step: the SpMV removed beta_j v_{j-1}; remove the v_j component
   // (alpha_j). With reorth, one classical Gram-Schmidt pass against every stored
   // vector follows; taking the local step first keeps that pass from having to
@@ -1144,7 +1146,7 @@ blqh_lanczos* create_impl(blqh_ctx* ctx, const blqh_csr* M, const blqh_lanczos_o
     L->work = dalloc<double>(ctx, 8 * (size_t)m + 16);
     L->y = dalloc<double>(ctx, m + 1);
     if (M->precision == BLQH_VAL_FP32 && o.accumulate == 0) L->xs = dalloc<float2>(ctx, n + 2);
-    if (fixed_prepare(ctx, const_cast<blqh_csr*>(M))) L->xq = dalloc<int2>(ctx, n + 2);
+    if (fixed_prepare(ctx, M, &L->fx)) L->xq = dalloc<int2>(ctx, n + 2);
     if (o.reorth && gs_planes_enabled()) {
       // the planes take up to the Krylov basis' memory again; without room for
       // them the run works on the FP64 vectors

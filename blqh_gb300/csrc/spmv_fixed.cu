@@ -157,37 +157,34 @@ __global__ void __launch_bounds__(256, 3) k_spmv_fixed(const int64_t* __restrict
 
 // The split copy of a complex FP64 matrix; false (and the FP64 kernel stays) without
 // room for it or with BLQH_SPMV_FIXED=0.
-bool fixed_prepare(blqh_ctx* ctx, blqh_csr* M) {
+bool fixed_prepare(blqh_ctx* ctx, const blqh_csr* M, FixedMatrix* F) {
   if (!M->is_complex || M->precision != BLQH_VAL_FP64) return false;
   const char* env = getenv("BLQH_SPMV_FIXED");
   if (env && env[0] == '0') return false;
-  if (M->d_qval) return true;
   try {
-    M->d_qval = dev_alloc(ctx, std::max<int64_t>(1, M->nnz) * sizeof(int4));
-    M->d_qexp = dalloc<int>(ctx, M->dim);
-    M->d_qdiag = dalloc<double>(ctx, 2 * M->dim);
+    F->val = dev_alloc(ctx, std::max<int64_t>(1, M->nnz) * sizeof(int4));
+    F->row_exp = dalloc<int>(ctx, M->dim);
+    F->diag = dalloc<double>(ctx, 2 * M->dim);
   } catch (const BlqhError& e) {
     if (e.code != BLQH_ERR_NOMEM) throw;
-    fixed_release(M);
+    fixed_release(F);
     ctx->last_error.clear();
     return false;
   }
   TimerScope ts(ctx, TM_MISC);
   k_fix_matrix<<<grid_for(ctx, M->dim * 32, 256, 16), 256, 0, ctx->stream>>>(
-      M->d_row_ptr, M->d_col, reinterpret_cast<const double2*>(M->d_val), M->dim, reinterpret_cast<int4*>(M->d_qval),
-      M->d_qexp, reinterpret_cast<double2*>(M->d_qdiag));
+      M->d_row_ptr, M->d_col, reinterpret_cast<const double2*>(M->d_val), M->dim, static_cast<int4*>(F->val), F->row_exp,
+      reinterpret_cast<double2*>(F->diag));
   BLQH_TRY_CUDA(ctx, cudaGetLastError());
   count_launch(ctx, TM_MISC);
   return true;
 }
 
-void fixed_release(blqh_csr* M) {
-  dev_free(M->d_qval);
-  dev_free(M->d_qexp);
-  dev_free(M->d_qdiag);
-  M->d_qval = nullptr;
-  M->d_qexp = nullptr;
-  M->d_qdiag = nullptr;
+void fixed_release(FixedMatrix* F) {
+  dev_free(F->val);
+  dev_free(F->row_exp);
+  dev_free(F->diag);
+  *F = FixedMatrix{};
 }
 
 void fixed_vector(blqh_ctx* ctx, const double* x, int2* xq, int64_t n, const int* stop) {
@@ -198,15 +195,15 @@ void fixed_vector(blqh_ctx* ctx, const double* x, int2* xq, int64_t n, const int
 }
 
 // y = H x - b xprev; xq: x in fixed point (|x| <= 1, as Krylov vectors are).
-void fixed_spmv(blqh_ctx* ctx, const blqh_csr* M, const double* x, const int2* xq, double* y, const double* bptr,
-                const double* xprev, const int* stop) {
+void fixed_spmv(blqh_ctx* ctx, const blqh_csr* M, const FixedMatrix& F, const double* x, const int2* xq, double* y,
+                const double* bptr, const double* xprev, const int* stop) {
   // 8 lanes per row (four rows per warp): 84 us at 60,096 rows of 256 nonzeros, against
   // 92 with 4 lanes, 95 with 16 and 121 with 32 (longer reductions per row)
   constexpr int LPR = 8;
   const int64_t blocks = std::min<int64_t>((M->dim * LPR + 255) / 256, (int64_t)ctx->num_sms * 16);
   k_spmv_fixed<LPR><<<(int)std::max<int64_t>(1, blocks), 256, 0, ctx->stream>>>(
-      M->d_row_ptr, M->d_col, reinterpret_cast<const int4*>(M->d_qval), M->d_qexp,
-      reinterpret_cast<const double2*>(M->d_qdiag), reinterpret_cast<const int4*>(xq),
+      M->d_row_ptr, M->d_col, static_cast<const int4*>(F.val), F.row_exp, reinterpret_cast<const double2*>(F.diag),
+      reinterpret_cast<const int4*>(xq),
       reinterpret_cast<const double2*>(x), reinterpret_cast<double2*>(y), M->dim, bptr,
       reinterpret_cast<const double2*>(xprev), stop);
 }
