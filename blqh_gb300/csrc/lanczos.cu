@@ -1146,7 +1146,13 @@ blqh_lanczos* create_impl(blqh_ctx* ctx, const blqh_csr* M, const blqh_lanczos_o
     L->work = dalloc<double>(ctx, 8 * (size_t)m + 16);
     L->y = dalloc<double>(ctx, m + 1);
     if (M->precision == BLQH_VAL_FP32 && o.accumulate == 0) L->xs = dalloc<float2>(ctx, n + 2);
-    if (fixed_prepare(ctx, M, &L->fx)) L->xq = dalloc<int2>(ctx, n + 2);
+    if (fixed_prepare(ctx, M, &L->fx)) try {
+        L->xq = dalloc<int2>(ctx, n + 2);
+      } catch (const BlqhError& e) {  // without room for it: the FP64 product
+        if (e.code != BLQH_ERR_NOMEM) throw;
+        fixed_release(&L->fx);
+        ctx->last_error.clear();
+      }
     if (o.reorth && gs_planes_enabled()) {
       // the planes take up to the Krylov basis' memory again; without room for
       // them the run works on the FP64 vectors

@@ -93,3 +93,39 @@ def test_spinful_observables_and_regenerated_energy(ctx, sec, kw):
                 assert np.max(np.abs(r - ref)) < 1e-12  # sums of a few thousand terms below 10 in another order
     for x in (L, H, b):
         x.close()
+
+
+RUNS = [  # sector, values, allocations that a run can do without
+    ((8, 8, 4, 0, 1), "f64", 7),   # complex FP64: split matrix (3), split vector, planes (3)
+    ((12, 10, 5, 3, 1), "f64", 7),
+    ((12, 10, 5, 3, 1), "f32", 3),  # complex FP32: planes
+    ((12, 10, 5, 5, 0), "f64", 1),  # real FP64: FP32 plane
+    ((12, 10, 5, 5, 0), "f32", 2),  # real FP32: two FP32 planes
+]
+
+
+@pytest.mark.parametrize("sec,prec,spare", RUNS, ids=str)
+def test_lanczos(ctx, monkeypatch, sec, prec, spare):
+    """A run that lacks one of its spare buffers returns the bits of the run that does without what it belongs to."""
+    import blqh_gb300 as B
+
+    b = B.Basis(*sec, ctx=ctx)
+    H = B.Hamiltonian(b, 0.9, precision=B.VAL_FP64 if prec == "f64" else B.VAL_FP32)
+
+    def run():
+        L = B.Lanczos(H, max_steps=40, tol=0.0, seed=3)
+        L.iterate()
+        r = np.concatenate([*L.coeffs(), L.ritz_vector().view(np.float64)])
+        L.close()
+        return r
+
+    modes = [run()]
+    for var, val in (("BLQH_SPMV_FIXED", "0"), ("BLQH_GS_FP64", "1")):
+        monkeypatch.setenv(var, val)
+        modes.append(run())
+        monkeypatch.delenv(var)
+    got = [r for r in sweep(ctx, run) if r is not None]
+    assert len(got) == spare
+    assert all(any(np.array_equal(r, m) for m in modes) for r in got)
+    H.close()
+    b.close()
