@@ -1146,14 +1146,15 @@ blqh_lanczos* create_impl(blqh_ctx* ctx, const blqh_csr* M, const blqh_lanczos_o
     L->work = dalloc<double>(ctx, 8 * (size_t)m + 16);
     L->y = dalloc<double>(ctx, m + 1);
     if (M->precision == BLQH_VAL_FP32 && o.accumulate == 0) L->xs = dalloc<float2>(ctx, n + 2);
-    if (fixed_prepare(ctx, M, &L->fx)) try {
+    if (!o.accumulate && fixed_prepare(ctx, M, &L->fx)) try {
         L->xq = dalloc<int2>(ctx, n + 2);
       } catch (const BlqhError& e) {  // without room for it: the FP64 product
         if (e.code != BLQH_ERR_NOMEM) throw;
         fixed_release(&L->fx);
         ctx->last_error.clear();
       }
-    if (o.reorth && gs_planes_enabled()) {
+    // (real sectors with accumulate = 1 keep the FP32 plane for the correction, not for the dots)
+    if (o.reorth && gs_planes_enabled() && !(L->cplx && o.accumulate)) {
       // the planes take up to the Krylov basis' memory again; without room for
       // them the run works on the FP64 vectors
       try {

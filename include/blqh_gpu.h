@@ -34,7 +34,7 @@ extern "C" {
 #define BLQH_REP_REFERENCE 0 /* survivor of the reference's unordered_map orbit filter (basis.cpp:82-99) */
 #define BLQH_REP_MIN 1       /* numerically smallest member of each orbit */
 
-/* Precision of the stored CSR values. Products always accumulate in FP64. */
+/* Precision of the stored CSR values (what products accumulate in: blqh_lanczos_opts.accumulate). */
 #define BLQH_VAL_FP64 0
 #define BLQH_VAL_FP32 1
 
@@ -95,17 +95,23 @@ typedef struct {
 /* Lanczos options. */
 typedef struct {
   int max_steps;      /* lambda: upper bound on Krylov steps (lanczos_hamiltonian.h:15) */
-  int reorth;         /* 1: full FP64 reorthogonalization (three-term step, then one classical Gram-Schmidt
-                         pass against every stored vector); 0: plain three-term recurrence */
+  int reorth;         /* 1: full reorthogonalization of the FP64 vectors (three-term step, then one classical
+                         Gram-Schmidt pass against every stored vector); 0: plain three-term recurrence */
   double tol;         /* stop when the lowest Ritz value moves less than tol between checks (0: run max_steps) */
   int check_every;    /* steps between convergence checks (>= 1) */
   uint64_t seed;      /* start-vector seed */
   int rng;            /* start vector: 0 = std::mt19937 stream as matrix.cpp:54-75 (host);
                          1 = mt19937-64 genrand64_real3 (host); 2 = counter-based generator on
                          the device (splitmix64 of seed and index), no host work */
-  int accumulate;     /* SpMV with FP32 values: 0 = double-float accumulation (FP32 pairs with error-free
-                         transformations, ~2^-48 per product; keeps the per-nonzero work off GB300's
-                         slow FP64 pipe); 1 = native FP64 FMA. FP64 values always use native FP64. */
+  int accumulate;     /* arithmetic of the products and of the reorthogonalization's dots (its correction is
+                         summed in FP32 while every coefficient is below 2^-30 of the vector). 1: native FP64.
+                         0: off GB300's slow FP64 pipe where that is faster. Products with FP32 values in
+                         double-float (FP32 pairs with error-free transformations, ~2^-48 per product);
+                         products with complex FP64 values in fixed point (57 bits below the largest
+                         off-diagonal entry of each row, 60 below the vector's norm, exact integer
+                         sums); complex sectors' dots in fixed point (57 bits below the largest of each
+                         1024 or 256 entries, exact integer sums), real sectors' with FP32 values in
+                         double-float. Products with real FP64 values are native FP64 either way. */
 } blqh_lanczos_opts;
 
 /* ---- context ------------------------------------------------------------ */
