@@ -233,9 +233,9 @@ struct FixedMatrix {
 };
 bool fixed_prepare(blqh_ctx* ctx, const blqh_csr* M, FixedMatrix* F);
 void fixed_release(FixedMatrix* F);
-void fixed_vector(blqh_ctx* ctx, const double* x, int2* xq, int64_t n, const int* stop);
-void fixed_spmv(blqh_ctx* ctx, const blqh_csr* M, const FixedMatrix& F, const double* x, const int2* xq, double* y,
-                const double* bptr, const double* xprev, const int* stop);
+void fixed_vector(blqh_ctx* ctx, const double* x, int2* xq, int* xe, unsigned* xmax, int64_t n, const int* stop);
+void fixed_spmv(blqh_ctx* ctx, const blqh_csr* M, const FixedMatrix& F, const double* x, const int2* xq, const int* xe,
+                double* y, const double* bptr, const double* xprev, const int* stop);
 
 void scan_exclusive_i64(blqh_ctx* ctx, const int64_t* in, int64_t* out, int64_t n, int64_t* total_host);
 void scan_exclusive_u32_to_i64(blqh_ctx* ctx, const uint32_t* in, int64_t* out, int64_t n, int64_t* total_host);

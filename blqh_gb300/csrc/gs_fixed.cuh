@@ -130,15 +130,15 @@ __device__ __forceinline__ void quantize(double x, int E, int& q1, int& q0) {
   q0 = (int)(q - ((long long)q1 << 29));
 }
 
-// x = (q.x 2^29 + q.y) 2^-59, |x| <= 1, rounded to nearest (the vector operand of
-// the fixed-point SpMV). Larger and non-finite values give zero (the SpMV's FP64
+// x = (q.x 2^29 + q.y) 2^(xe - 59), |x| <= 2^xe, rounded to nearest (the vector operand
+// of the fixed-point SpMV). Larger and non-finite values give zero (the SpMV's FP64
 // diagonal term carries them on).
-__device__ __forceinline__ int2 fix_unit(double x) {
+__device__ __forceinline__ int2 fix_scaled(double x, int xe) {
   const long long b = __double_as_longlong(x);
   const int ex = (int)((b >> 52) & 0x7FF) - 1023;
   long long m = (b & 0xFFFFFFFFFFFFFLL) | 0x10000000000000LL;
-  const int sh = ex + 7;  // m 2^(ex - 52) in units of 2^-59
-  if (ex > 0 || sh < -60) m = 0;
+  const int sh = ex - xe + 7;  // m 2^(ex - 52) in units of 2^(xe - 59)
+  if (sh > 7 || sh < -60) m = 0;
   else if (sh >= 0) m <<= sh;
   else m = (m + (1LL << (-sh - 1))) >> -sh;
   const long long q = b < 0 ? -m : m;
@@ -146,17 +146,32 @@ __device__ __forceinline__ int2 fix_unit(double x) {
   return make_int2(hi, (int)(q - ((long long)hi << 29)));
 }
 
-// Exponent E of the largest |x| over the block, from each thread's largest high
-// word (sign cleared). All zero (or denormal): -1023.
-__device__ __forceinline__ int block_exponent(unsigned hw, unsigned* red) {
+// Largest value over the block, in every thread.
+__device__ __forceinline__ unsigned block_max(unsigned hw, unsigned* red) {
   hw = __reduce_max_sync(0xffffffffu, hw);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = hw;
   __syncthreads();
   unsigned m = 0;
   for (int i = 0; i < (int)(blockDim.x >> 5); i++) m = max(m, red[i]);
-  return (int)(m >> 20) - 1023;
+  return m;
 }
+
+// High word of |x|, and the exponent E of the value it is the high word of (zero and
+// denormals: -1023).
 __device__ __forceinline__ unsigned abs_high_word(double x) { return (unsigned)__double2hiint(x) & 0x7FFFFFFFu; }
+__device__ __forceinline__ int word_exponent(unsigned hw) { return (int)(hw >> 20) - 1023; }
+
+// Exponent E of the largest |x| over the block, from each thread's largest high word.
+__device__ __forceinline__ int block_exponent(unsigned hw, unsigned* red) { return word_exponent(block_max(hw, red)); }
+
+// xe of a normalized vector v = (w - c) inv for fix_scaled, 2^E <= max |w| < 2^(E+1),
+// |c| <= sqrt(cc): the least power of two above a bound on |v| (at most 4 times the
+// largest entry for negligible c), and no more than 2^0.
+__device__ __forceinline__ int scaled_exponent(int E, double cc, double inv) {
+  const double a = __hiloint2double((E + 1 + 1023) << 20, 0);
+  const double c = __hiloint2double((((word_exponent(abs_high_word(cc)) + 2) >> 1) + 1023) << 20, 0);
+  return min(word_exponent(abs_high_word((a + c) * inv * (1 + 0x1p-20))) + 1, 0);
+}
 
 // Sum of a pair over the warp, in every lane. (One warp sums what a block needs: an
 // FP64 instruction takes the SM's FP64 pipe 16 clocks, so the same sum spread over
@@ -385,7 +400,7 @@ struct WTile {
   int na;
   const int* w1;
   const int* w0;
-  const int* we;
+  int* we;               // [ntile] exponents of w' (LOCAL writes them)
   double* npart;         // [ntile] partials of |w'|^2 (LOCAL writes them)
 };
 
@@ -456,7 +471,10 @@ __global__ void __launch_bounds__(256, DOT_MINB)
     sw[1][threadIdx.x] = q0;
     if (g == 0) {
       const double nn = block_sum_256(x * x, red);  // the whole block
-      if (threadIdx.x == 0) W.npart[tile] = nn;
+      if (threadIdx.x == 0) {
+        W.npart[tile] = nn;
+        W.we[tile] = ew;
+      }
     }
     __syncthreads();
     a1 = reinterpret_cast<const int4*>(sw[0]) + lane;
@@ -554,11 +572,12 @@ __device__ __forceinline__ float2 split_f64(double x) {
   return make_float2((float)hi * sh, (float)lo * sl);
 }
 
-// One vector entry: V_{j+1} and its split for the next SpMV (double-float xs, or fixed point xq).
-__device__ __forceinline__ void store_entry(double v, int64_t i, double* vout, float2* xs, int2* xq) {
+// One vector entry: V_{j+1} and its split for the next SpMV (double-float xs, or fixed
+// point xq below 2^xe).
+__device__ __forceinline__ void store_entry(double v, int64_t i, double* vout, float2* xs, int2* xq, int xe) {
   vout[i] = v;
   if (xs) xs[i] = split_f64(v);
-  if (xq) xq[i] = fix_unit(v);
+  if (xq) xq[i] = fix_scaled(v, xe);
 }
 
 // Where v_{j+1} goes: its row of V, of the planes, and the SpMV's split input.
@@ -566,6 +585,7 @@ struct NextVec {
   double* v;
   float2* xs;
   int2* xq;
+  int* xe;  // the exponent xq is below
   int* q1;
   int* q0;
   int* E;
@@ -596,6 +616,7 @@ __global__ void __launch_bounds__(KS * TILE / 4) k_update_q(const double* V, con
   __shared__ double s_inv, s_hh, s_nn;
   __shared__ double2 s_h;
   __shared__ int s_hexp;  // exponent of the largest coefficient
+  __shared__ int s_wexp, s_xe;  // of the largest |w'|; of the next SpMV's input
   const int tile = (int)(gridDim.x - 1 - blockIdx.x);
   const int64_t r0 = (int64_t)tile * TILE;
   const int stop = S.flags[0];
@@ -638,6 +659,11 @@ __global__ void __launch_bounds__(KS * TILE / 4) k_update_q(const double* V, con
   } else if (wid == 1) {
     const double nn = sum_partials(W.npart, ntile);
     if (lane == 0) s_nn = nn;
+  } else if (wid == 3) {
+    int e = -1023;
+    for (int t = lane; t < ntile && nx.xq; t += 32) e = max(e, __ldcg(W.we + t));
+    e = __reduce_max_sync(0xffffffffu, e);
+    if (lane == 0) s_wexp = e;
   } else if (LOCAL && wid == 2) {
     const double2 h = sum_partials(W.apart, W.na);
     if (lane == 0) s_h = h;
@@ -665,6 +691,10 @@ __global__ void __launch_bounds__(KS * TILE / 4) k_update_q(const double* V, con
     if (threadIdx.x == 0) {
       const double b2 = s_nn - s_hh;
       s_inv = rsqrt(b2);
+      if (nx.xq) {
+        s_xe = scaled_exponent(s_wexp, s_hh, s_inv);
+        if (tile == 0) *nx.xe = s_xe;
+      }
       if (tile == 0) beta_from(S, j, b2, breakdown_tol);
     }
     const int sl = (int)threadIdx.x / TP, pos = (int)threadIdx.x % TP;
@@ -692,6 +722,7 @@ __global__ void __launch_bounds__(KS * TILE / 4) k_update_q(const double* V, con
     *reinterpret_cast<float4*>(sred + sl * TILE + pos * 4) = make_float4(d[0], d[1], d[2], d[3]);
     __syncthreads();
     const double inv = s_inv;
+    const int xe = s_xe;
     unsigned hw = 0;
 #pragma unroll
     for (int q = 0; q < NE; q++) {
@@ -701,7 +732,7 @@ __global__ void __launch_bounds__(KS * TILE / 4) k_update_q(const double* V, con
 #pragma unroll
         for (int z = 0; z < KS; z++) c += sred[z * TILE + i];
         a[q] = (a[q] - (double)c) * inv;
-        store_entry(a[q], r0 + i, nx.v, nx.xs, nx.xq);
+        store_entry(a[q], r0 + i, nx.v, nx.xs, nx.xq, xe);
         hw = max(hw, abs_high_word(a[q]));
       }
     }
@@ -709,6 +740,7 @@ __global__ void __launch_bounds__(KS * TILE / 4) k_update_q(const double* V, con
     return;
   }
   double nn = 0;
+  unsigned hw = 0;
 #pragma unroll
   for (int q = 0; q < NE; q++) {
     const int64_t r = r0 + q * NT + threadIdx.x;
@@ -724,28 +756,41 @@ __global__ void __launch_bounds__(KS * TILE / 4) k_update_q(const double* V, con
     }
     nx.v[r] = a[q];  // not yet scaled (w is still read by other blocks' three-term step)
     nn += a[q] * a[q];
+    hw = max(hw, abs_high_word(a[q]));
   }
   nn = block_sum_256(nn, red1);
-  if (threadIdx.x == 0) part[tile] = nn;
+  hw = block_max(hw, ured);
+  if (threadIdx.x == 0) {
+    part[tile] = nn;
+    nx.E[tile] = (int)hw;  // the tile's exponent goes here at the end
+  }
   if (!last_block(S.cnt + CNT_UPDATE, gridDim.x)) return;
   double s = 0;
-  for (int t = threadIdx.x; t < (int)gridDim.x; t += NT) s += __ldcg(part + t);
+  hw = 0;
+  for (int t = threadIdx.x; t < (int)gridDim.x; t += NT) {
+    s += __ldcg(part + t);
+    hw = max(hw, (unsigned)__ldcg(nx.E + t));
+  }
   s = block_sum_256(s, red1);
+  hw = block_max(hw, ured);
   if (threadIdx.x == 0) {
     s_inv = rsqrt(s);
+    s_xe = scaled_exponent(word_exponent(hw), 0.0, s_inv);
+    if (nx.xq) *nx.xe = s_xe;
     beta_from(S, j, s, breakdown_tol);
   }
   __syncthreads();
   const double inv = s_inv;
+  const int xe = s_xe;
   for (int t = 0; t < ntile; t++) {
-    unsigned hw = 0;
+    hw = 0;
 #pragma unroll
     for (int q = 0; q < NE; q++) {
       const int64_t i = (int64_t)t * TILE + q * NT + threadIdx.x;
       a[q] = 0.0;
       if (q * NT + (int)threadIdx.x < TILE && i < n) {
         a[q] = __ldcg(nx.v + i) * inv;
-        store_entry(a[q], i, nx.v, nx.xs, nx.xq);
+        store_entry(a[q], i, nx.v, nx.xs, nx.xq, xe);
         hw = max(hw, abs_high_word(a[q]));
       }
     }

@@ -90,13 +90,16 @@ __global__ void __launch_bounds__(32) k_alpha_o(const double* vj, const double* 
 // |w|^2 per 256 EPT entries. EPT = 4 (four consecutive entries per thread) in the
 // runs with double-float planes, else 1. Every block sums h_j itself, so large
 // sectors take a few blocks per SM with several groups of entries each (2,528
-// blocks at 647,079 rows: 25 us, 608: 18 us).
+// blocks at 647,079 rows: 25 us, 608: 18 us). pmax (complex): the group's largest
+// high word of |w|, for the fixed-point product's scale, or null.
 template <bool CPLX, int EPT>
 __global__ void __launch_bounds__(256) k_local_o(const double* vj, double* w, int64_t dim, const double* apart,
-                                                 int ntile, double* pnorm, int ngroups, Scal S, int j) {
+                                                 int ntile, double* pnorm, unsigned* pmax, int ngroups, Scal S,
+                                                 int j) {
   pdl_begin();
   static_assert(!CPLX || EPT == 1, "complex rows one per thread");
   __shared__ double red[8];
+  __shared__ unsigned ured[8];
   __shared__ double s_h[2];
   const int stop = S.flags[0];
   double a[EPT], b[EPT], v[EPT], u[EPT];
@@ -137,6 +140,7 @@ __global__ void __launch_bounds__(256) k_local_o(const double* vj, double* w, in
     const int64_t i0 = ((int64_t)g * 256 + threadIdx.x) * EPT;
     if (g != (int)blockIdx.x) load(i0);
     double nn = 0;
+    unsigned hw = 0;
 #pragma unroll
     for (int q = 0; q < EPT; q++) {
       const int64_t i = i0 + q;
@@ -146,6 +150,7 @@ __global__ void __launch_bounds__(256) k_local_o(const double* vj, double* w, in
           b[q] -= hr * u[q] + hi * v[q];
           reinterpret_cast<double2*>(w)[i] = make_double2(a[q], b[q]);
           nn += a[q] * a[q] + b[q] * b[q];
+          hw = max(abs_high_word(a[q]), abs_high_word(b[q]));
         } else {
           a[q] -= hr * v[q];
           w[i] = a[q];
@@ -155,6 +160,11 @@ __global__ void __launch_bounds__(256) k_local_o(const double* vj, double* w, in
     }
     nn = block_sum_256(nn, red);
     if (threadIdx.x == 0) pnorm[g] = nn;
+    if (CPLX && pmax) {
+      hw = block_max(hw, ured);
+      if (threadIdx.x == 0) pmax[g] = hw;
+      __syncthreads();  // ured is written again
+    }
   }
 }
 
@@ -329,16 +339,17 @@ __global__ void __launch_bounds__(256) k_reduce_o(const double* part, int ntile,
   if (k == j) S.alpha[j] += a;
 }
 
-// Full pass, correction: w -= sum_k h2[k] V_k, partials of |w|^2 as in k_local_o.
+// Full pass, correction: w -= sum_k h2[k] V_k, partials of |w|^2 (and pmax) as in k_local_o.
 // In FP32 from FP32-truncated coefficients and entries (the Vh plane where there
 // is one, PL, else V truncated here; relative error ~2^-22 of a correction <=
 // 2^-30 |w|, below FP64's rounding of w), subtracted in FP64. A flagged pass uses
 // FP64 FMAs on V. BATCH vectors' loads are in flight per thread.
 template <bool CPLX, int EPT, bool PL>
 __global__ void __launch_bounds__(256) k_update_o(const double* V, const float* Vh, int64_t ld, int64_t dim, int nk,
-                                                  double* w, double* pnorm, Scal S) {
+                                                  double* w, double* pnorm, unsigned* pmax, Scal S) {
   pdl_begin();
   static_assert(!CPLX || (EPT == 1 && !PL), "complex rows one per thread, from V");
+  __shared__ unsigned ured[8];
   if (S.flags[0]) return;
   extern __shared__ double hs[];  // [2 nk] coefficients, then [2 nk] floats
   __shared__ double red[8];
@@ -453,6 +464,10 @@ __global__ void __launch_bounds__(256) k_update_o(const double* V, const float* 
   }
   nn = block_sum_256(nn, red);
   if (threadIdx.x == 0) pnorm[blockIdx.x] = nn;
+  if (CPLX && pmax) {
+    const unsigned hw = block_max(max(abs_high_word(a[0]), abs_high_word(b)), ured);
+    if (threadIdx.x == 0) pmax[blockIdx.x] = hw;
+  }
 }
 
 // Where v_{j+1} goes: V, the SpMV's split input, the planes (rows padded with zeros to ld floats).
@@ -460,24 +475,38 @@ struct NextPlanes {
   double* v;
   float2* xs;
   int2* xq;
+  int* xe;  // the exponent xq is below
   float* vh;
   float* vl;
   int64_t ld;
 };
 
-// v_{j+1} = w / beta_{j+1}, beta from the partials of |w|^2 (summed by every block,
-// so there are few of them, grid-stride). start: src is the start vector, only its
+// v_{j+1} = w / beta_{j+1}, beta from the partials of |w|^2 and, for the fixed-point
+// product, the scale of its input from pmax (taken together by every block, so there
+// are few of them, grid-stride). start: src is the start vector, only its
 // planes are written.
-__global__ void __launch_bounds__(256) k_scale_o(const double* src, int64_t n, int start, const double* pnorm, int npn,
-                                                 Scal S, int j, double breakdown_tol, NextPlanes nx) {
+__global__ void __launch_bounds__(256) k_scale_o(const double* src, int64_t n, int start, const double* pnorm,
+                                                 const unsigned* pmax, int npn, Scal S, int j, double breakdown_tol,
+                                                 NextPlanes nx) {
   pdl_begin();
   if (S.flags[0]) return;
   __shared__ double red[8];
+  __shared__ unsigned ured[8];
   __shared__ double s_inv;
+  __shared__ int s_xe;
   if (!start) {
     const double s = ordered_sum(pnorm, 1, npn, red);
+    unsigned hw = 0;
+    if (nx.xq) {
+      for (int t = threadIdx.x; t < npn; t += 256) hw = max(hw, __ldcg(pmax + t));
+      hw = block_max(hw, ured);
+    }
     if (threadIdx.x == 0) {
       s_inv = 1.0 / sqrt(s);
+      if (nx.xq) {
+        s_xe = scaled_exponent(word_exponent(hw), 0.0, s_inv);
+        if (blockIdx.x == 0) *nx.xe = s_xe;
+      }
       if (blockIdx.x == 0) beta_from(S, j, s, breakdown_tol);
     }
   }
@@ -490,7 +519,7 @@ __global__ void __launch_bounds__(256) k_scale_o(const double* src, int64_t n, i
       v = src[i];
       if (!start) {
         v *= inv;
-        store_entry(v, i, nx.v, nx.xs, nx.xq);
+        store_entry(v, i, nx.v, nx.xs, nx.xq, s_xe);
       }
     }
     if (nx.vh) {

@@ -581,7 +581,9 @@ struct blqh_lanczos {
   double* y = nullptr;     // [mmax] Ritz coefficients
   float2* xs = nullptr;    // [dim * vw] (hi, lo) split of the SpMV input (double-float accumulation)
   FixedMatrix fx;          // the matrix in fixed point (complex FP64 matrices)
-  int2* xq = nullptr;      // [dim * 2] the SpMV input in fixed point
+  int2* xq = nullptr;      // [dim * 2] the SpMV input in fixed point, then xe and pmax in the same buffer
+  int* xe = nullptr;       // the exponent that its entries are below
+  unsigned* pmax = nullptr;  // [nblk_upd] block maxima of |w| (high words), where its scale comes from
   // complex sectors: fixed-point planes of V and, in the last row, of w (or null)
   int* Q1 = nullptr;       // [(mmax+2) * pld]
   int* Q0 = nullptr;
@@ -686,10 +688,11 @@ void spmv_df_t(blqh_ctx* ctx, const blqh_csr* M, const float2* xs, double* y, co
 
 // y = H x - b xprev. With an FP32-valued CSR and a split buffer xs, the product
 // accumulates in double-float (k_spmv_df); with a fixed-point copy fx of the matrix and
-// a buffer xq (|x| <= 1) in integers (k_spmv_fixed); otherwise in native FP64 (k_spmv).
+// buffers xq, xe, pmax (|x| <= 1) in integers (k_spmv_fixed); otherwise in native FP64 (k_spmv).
 void spmv_dev(blqh_ctx* ctx, const blqh_csr* M, const double* x, double* y, const double* bptr = nullptr,
               const double* xprev = nullptr, const int* stop = nullptr, float2* xs = nullptr,
-              bool xs_ready = false, const FixedMatrix* fx = nullptr, int2* xq = nullptr) {
+              bool xs_ready = false, const FixedMatrix* fx = nullptr, int2* xq = nullptr, int* xe = nullptr,
+              unsigned* pmax = nullptr) {
   if (xs && M->precision == BLQH_VAL_FP32) {
     const int64_t n = M->dim * (M->is_complex ? 2 : 1);
     if (!xs_ready) {  // else the caller's previous kernel left x's split in xs
@@ -705,9 +708,9 @@ void spmv_dev(blqh_ctx* ctx, const blqh_csr* M, const double* x, double* y, cons
     return;
   }
   if (xq) {  // fixed point (complex FP64)
-    if (!xs_ready) fixed_vector(ctx, x, xq, M->dim * 2, stop);
+    if (!xs_ready) fixed_vector(ctx, x, xq, xe, pmax, M->dim * 2, stop);
     TimerScope ts(ctx, TM_SPMV);
-    fixed_spmv(ctx, M, *fx, x, xq, y, bptr, xprev, stop);
+    fixed_spmv(ctx, M, *fx, x, xq, xe, y, bptr, xprev, stop);
     BLQH_TRY_CUDA(ctx, cudaGetLastError());
     count_launch(ctx, TM_SPMV);
     return;
@@ -762,7 +765,7 @@ int* qe_row(const blqh_lanczos* L, int k) { return L->QE ? L->QE + (int64_t)k * 
 
 NextVec next_vec(const blqh_lanczos* L, int k) {
   return {L->V + (int64_t)k * L->dim * L->vw, L->M->precision == BLQH_VAL_FP32 ? L->xs : nullptr, L->xq,
-          q1_row(L, k), q0_row(L, k), qe_row(L, k)};
+          L->xe, q1_row(L, k), q0_row(L, k), qe_row(L, k)};
 }
 
 // The step after the SpMV on the fixed-point planes (complex sectors).
@@ -795,7 +798,7 @@ void gs_step_q(blqh_lanczos* L, int j) {
 
 NextPlanes next_planes(const blqh_lanczos* L, int k) {
   return {L->V + (int64_t)k * L->dim * L->vw, L->M->precision == BLQH_VAL_FP32 ? L->xs : nullptr, L->xq,
-          L->Vh ? L->Vh + (int64_t)k * L->vld : nullptr, L->Vl ? L->Vl + (int64_t)k * L->vld : nullptr, L->vld};
+          L->xe, L->Vh ? L->Vh + (int64_t)k * L->vld : nullptr, L->Vl ? L->Vl + (int64_t)k * L->vld : nullptr, L->vld};
 }
 
 // The step after the SpMV in the fixed order of operations (real sectors, and
@@ -811,9 +814,11 @@ void gs_step_o(blqh_lanczos* L, int j) {
   launch_chained(ctx, k_alpha_o<CPLX>, nt, 32, 0, vj, L->w, L->dim, apart, L->S);
   const int lg = std::min(nu, 4 * ctx->num_sms);
   if (df)
-    launch_chained(ctx, k_local_o<false, 4>, lg, 256, 0, vj, L->w, L->dim, apart, nt, L->pnorm, nu, L->S, j);
+    launch_chained(ctx, k_local_o<false, 4>, lg, 256, 0, vj, L->w, L->dim, apart, nt, L->pnorm, L->pmax, nu, L->S,
+                   j);
   else
-    launch_chained(ctx, k_local_o<CPLX, 1>, lg, 256, 0, vj, L->w, L->dim, apart, nt, L->pnorm, nu, L->S, j);
+    launch_chained(ctx, k_local_o<CPLX, 1>, lg, 256, 0, vj, L->w, L->dim, apart, nt, L->pnorm, L->pmax, nu, L->S,
+                   j);
   if (L->o.reorth) {
     const int nk = j + 1;
     // up to 64 tiles: 8 vectors per block (one per warp), summed by each group's last block; beyond, a
@@ -830,7 +835,7 @@ void gs_step_o(blqh_lanczos* L, int j) {
     };
     const size_t hsm = 2 * nk * (sizeof(double) + sizeof(float));
     auto update = [&](auto kern) {
-      launch_chained(ctx, kern, nu, 256, hsm, L->V, L->Vh, L->vld, L->dim, nk, L->w, L->pnorm, L->S);
+      launch_chained(ctx, kern, nu, 256, hsm, L->V, L->Vh, L->vld, L->dim, nk, L->w, L->pnorm, L->pmax, L->S);
     };
     if constexpr (CPLX) {
       dots(k_dots_o<true, false, 1>);
@@ -846,7 +851,7 @@ void gs_step_o(blqh_lanczos* L, int j) {
     }
     count_launch(ctx, TM_REORTH, finish ? 2 : 3);
   }
-  launch_chained(ctx, k_scale_o, grid_for(ctx, n, 256, 2), 256, 0, L->w, n, 0, L->pnorm, nu, L->S, j, 1e-13,
+  launch_chained(ctx, k_scale_o, grid_for(ctx, n, 256, 2), 256, 0, L->w, n, 0, L->pnorm, L->pmax, nu, L->S, j, 1e-13,
                  next_planes(L, j + 1));
   count_launch(ctx, TM_REORTH, 3);
 }
@@ -858,7 +863,7 @@ void lanczos_step(blqh_lanczos* L, int j) {
   const double* vprev = j > 0 ? L->V + (int64_t)(j - 1) * n : nullptr;
   // from the second step on, the previous step left v_j's split in xs
   spmv_dev(ctx, L->M, vj, L->w, j > 0 ? L->S.beta + j : nullptr, vprev, L->S.flags, L->xs, j > 0,
-           &L->fx, L->xq);
+           &L->fx, L->xq, L->xe, L->pmax);
   // three-term step: the SpMV removed beta_j v_{j-1}; remove the v_j component
   // (alpha_j). With reorth, one classical Gram-Schmidt pass against every stored
   // vector follows; taking the local step first keeps that pass from having to
@@ -900,8 +905,8 @@ void iterate_impl(blqh_lanczos* L) {
       launch_chained(ctx, L->tile == 1024 ? k_planes_q<1024> : k_planes_q<256>, L->ntile, L->tile / 4, 0, L->V, n,
                      next_vec(L, 0));
     else
-      launch_chained(ctx, k_scale_o, grid_for(ctx, n, 256, 2), 256, 0, L->V, n, 1, nullptr, 0, L->S, 0, 0.0,
-                     next_planes(L, 0));
+      launch_chained(ctx, k_scale_o, grid_for(ctx, n, 256, 2), 256, 0, L->V, n, 1, nullptr, nullptr, 0, L->S, 0,
+                     0.0, next_planes(L, 0));
     count_launch(ctx, TM_MISC);
   }
   BLQH_TRY_CUDA(ctx, cudaMemsetAsync(L->S.beta, 0, sizeof(double), st));
@@ -1147,7 +1152,9 @@ blqh_lanczos* create_impl(blqh_ctx* ctx, const blqh_csr* M, const blqh_lanczos_o
     L->y = dalloc<double>(ctx, m + 1);
     if (M->precision == BLQH_VAL_FP32 && o.accumulate == 0) L->xs = dalloc<float2>(ctx, n + 2);
     if (!o.accumulate && fixed_prepare(ctx, M, &L->fx)) try {
-        L->xq = dalloc<int2>(ctx, n + 2);
+        L->xq = dalloc<int2>(ctx, n + 2 + L->nblk_upd);
+        L->xe = reinterpret_cast<int*>(L->xq + n);
+        L->pmax = reinterpret_cast<unsigned*>(L->xq + n + 2);
       } catch (const BlqhError& e) {  // without room for it: the FP64 product
         if (e.code != BLQH_ERR_NOMEM) throw;
         fixed_release(&L->fx);
@@ -1493,6 +1500,27 @@ int blqh_lanczos_observables_spin(blqh_lanczos* L, const blqh_basis* b, double* 
   }
   try {
     spin_observables_impl(L->ctx, b, L->psi, L->cplx, out);
+  } catch (const BlqhError& e) {
+    return e.code;
+  }
+  return BLQH_OK;
+}
+
+int blqh_debug_lanczos_product(blqh_lanczos* L, double* x, double* y) {
+  if (!L || !x || !y) return BLQH_ERR_ARG;
+  blqh_ctx* ctx = L->ctx;
+  try {
+    const int64_t n = L->dim * L->vw;
+    const int m = L->iterated ? L->steps : 0;
+    if (!L->started) {
+      set_error(ctx, BLQH_ERR_STATE, "blqh_debug_lanczos_product: no start vector yet");
+      return BLQH_ERR_STATE;
+    }
+    const double* v = L->V + (int64_t)m * n;
+    spmv_dev(ctx, L->M, v, L->w, nullptr, nullptr, nullptr, L->xs, m > 0, &L->fx, L->xq, L->xe, L->pmax);
+    BLQH_TRY_CUDA(ctx, cudaMemcpyAsync(x, v, n * 8, cudaMemcpyDeviceToHost, ctx->stream));
+    BLQH_TRY_CUDA(ctx, cudaMemcpyAsync(y, L->w, n * 8, cudaMemcpyDeviceToHost, ctx->stream));
+    BLQH_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   } catch (const BlqhError& e) {
     return e.code;
   }

@@ -5,15 +5,21 @@
 // row on a pipe of ~1.6 lane operations per clock per SM: that pipe, not memory,
 // sets its time. Here both operands are integers, split once: the matrix per row (57
 // bits below the row's largest off-diagonal entry; the diagonal stays FP64 and
-// apart), the vector on one scale (|x| <= 1, unit 2^-59),
-//   v = (v1 2^29 + v0) 2^(E - 56), |v1|, |v0| <= 2^28,
-//   x = (x1 2^29 + x0) 2^-59,      |x1| <= 2^30, |x0| <= 2^28,
+// apart), the vector on the scale of its largest entry (|x| <= 2^xe, at most 4 times
+// that entry),
+//   v = (v1 2^29 + v0) 2^(E - 56),   |v1|, |v0| <= 2^28,
+//   x = (x1 2^29 + x0) 2^(xe - 59),  |x1| <= 2^30, |x0| <= 2^28,
 // and a row's sum is exact integer arithmetic: four IMAD.WIDE (27 lanes per clock
 // per SM) per real product into three 64-bit sums, folded into 128 bits every
 // eight nonzeros (the largest sum, of 2 x 8 cross products below 1.25 x 2^58, stays
 // below 2^63), one conversion to FP64 per row. What is lost is the operands'
-// rounding to 2^-57 of the row's largest entry and 2^-60 of the vector's norm,
-// below the 2^-53 an FP64 product rounds to.
+// rounding, 2^-57 of the row's and 2^-58 of the vector's largest entry: entries far
+// below those keep fewer bits than FP64's 53, but a row's sum is not rounded at every
+// addition. Error against extended precision, root mean square over rows, Krylov
+// vectors of 79 to 100,141 states: 0.27 to 0.66 of the FP64 kernel's; rows of states
+// where the vector is zero, which leave the FP64 diagonal term out: 0.28 to 0.36
+// (tests/test_fixed_product.py; with the unit at 2^-59 of the vector's norm the latter
+// were 0.41 to 1.003, growing with the number of states).
 //
 // The split matrix takes 16 bytes per nonzero next to the CSR values. What is left
 // is the latency of the column, then the gather behind it (long-scoreboard stalls,
@@ -70,11 +76,25 @@ __global__ void __launch_bounds__(256) k_fix_matrix(const int64_t* __restrict__ 
   }
 }
 
-// x in the vector's fixed point, for products whose previous kernel did not leave it.
-__global__ void k_fix_vector(const double* __restrict__ x, int2* __restrict__ xq, int64_t n, const int* stop) {
+// x in the vector's fixed point, for products whose previous kernel did not leave it:
+// the largest entry's high word (*xmax zero before), then the entries and their scale.
+__global__ void __launch_bounds__(256) k_fix_max(const double* __restrict__ x, unsigned* xmax, int64_t n,
+                                                 const int* stop) {
   if (stop && *stop) return;
+  __shared__ unsigned red[8];
+  unsigned hw = 0;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    xq[i] = fix_unit(x[i]);
+    hw = max(hw, abs_high_word(x[i]));
+  hw = block_max(hw, red);
+  if (threadIdx.x == 0) atomicMax(xmax, hw);
+}
+__global__ void k_fix_vector(const double* __restrict__ x, int2* __restrict__ xq, int* xe, const unsigned* xmax,
+                             int64_t n, const int* stop) {
+  if (stop && *stop) return;
+  const int e = min(word_exponent(*xmax) + 1, 0);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *xe = e;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    xq[i] = fix_scaled(x[i], e);
 }
 
 // LPR lanes per row. The real and imaginary sums are reduced together: after the
@@ -84,6 +104,7 @@ template <int LPR>
 __global__ void __launch_bounds__(256, 3) k_spmv_fixed(const int64_t* __restrict__ rp, const int32_t* __restrict__ col,
                                                     const int4* __restrict__ qv, const int* __restrict__ qe,
                                                     const double2* __restrict__ diag, const int4* xq,
+                                                    const int* __restrict__ xe,
                                                     const double2* x, double2* __restrict__ y, int64_t dim,
                                                     const double* bptr, const double2* xprev, const int* stop) {
   if (stop && *stop) return;
@@ -138,7 +159,8 @@ __global__ void __launch_bounds__(256, 3) k_spmv_fixed(const int64_t* __restrict
 #pragma unroll
     for (int d = LPR / 4; d > 0; d >>= 1)
       a.add(__shfl_xor_sync(0xffffffffu, a.lo, d), __shfl_xor_sync(0xffffffffu, a.hi, d));
-    const double part = ok ? fx_to_double(a.hi, a.lo, __ldg(qe + r) - 115) : 0.0;
+    // 2^(E - 56) of the matrix times 2^(xe - 59) of the vector
+    const double part = ok ? fx_to_double(a.hi, a.lo, __ldg(qe + r) + __ldg(xe) - 115) : 0.0;
     const double other = __shfl_xor_sync(0xffffffffu, part, LPR / 2);
     if (ok && sub == 0) {
       const double2 d = __ldg(diag + r), xr = x[r];
@@ -187,23 +209,27 @@ void fixed_release(FixedMatrix* F) {
   *F = FixedMatrix{};
 }
 
-void fixed_vector(blqh_ctx* ctx, const double* x, int2* xq, int64_t n, const int* stop) {
+// x (|x| <= 1, as Krylov vectors are) in fixed point; xmax: scratch.
+void fixed_vector(blqh_ctx* ctx, const double* x, int2* xq, int* xe, unsigned* xmax, int64_t n, const int* stop) {
   TimerScope tm(ctx, TM_MISC);
-  k_fix_vector<<<grid_for(ctx, n, 256, 8), 256, 0, ctx->stream>>>(x, xq, n, stop);
+  const int grid = grid_for(ctx, n, 256, 8);
+  BLQH_TRY_CUDA(ctx, cudaMemsetAsync(xmax, 0, sizeof(unsigned), ctx->stream));
+  k_fix_max<<<grid, 256, 0, ctx->stream>>>(x, xmax, n, stop);
+  k_fix_vector<<<grid, 256, 0, ctx->stream>>>(x, xq, xe, xmax, n, stop);
   BLQH_TRY_CUDA(ctx, cudaGetLastError());
-  count_launch(ctx, TM_MISC);
+  count_launch(ctx, TM_MISC, 2);
 }
 
-// y = H x - b xprev; xq: x in fixed point (|x| <= 1, as Krylov vectors are).
-void fixed_spmv(blqh_ctx* ctx, const blqh_csr* M, const FixedMatrix& F, const double* x, const int2* xq, double* y,
-                const double* bptr, const double* xprev, const int* stop) {
+// y = H x - b xprev; xq, xe: x in fixed point.
+void fixed_spmv(blqh_ctx* ctx, const blqh_csr* M, const FixedMatrix& F, const double* x, const int2* xq, const int* xe,
+                double* y, const double* bptr, const double* xprev, const int* stop) {
   // 8 lanes per row (four rows per warp): 84 us at 60,096 rows of 256 nonzeros, against
   // 92 with 4 lanes, 95 with 16 and 121 with 32 (longer reductions per row)
   constexpr int LPR = 8;
   const int64_t blocks = std::min<int64_t>((M->dim * LPR + 255) / 256, (int64_t)ctx->num_sms * 16);
   k_spmv_fixed<LPR><<<(int)std::max<int64_t>(1, blocks), 256, 0, ctx->stream>>>(
       M->d_row_ptr, M->d_col, static_cast<const int4*>(F.val), F.row_exp, reinterpret_cast<const double2*>(F.diag),
-      reinterpret_cast<const int4*>(xq),
+      reinterpret_cast<const int4*>(xq), xe,
       reinterpret_cast<const double2*>(x), reinterpret_cast<double2*>(y), M->dim, bptr,
       reinterpret_cast<const double2*>(xprev), stop);
 }

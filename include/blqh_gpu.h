@@ -108,7 +108,7 @@ typedef struct {
                          0: off GB300's slow FP64 pipe where that is faster. Products with FP32 values in
                          double-float (FP32 pairs with error-free transformations, ~2^-48 per product);
                          products with complex FP64 values in fixed point (57 bits below the largest
-                         off-diagonal entry of each row, 60 below the vector's norm, exact integer
+                         off-diagonal entry of each row and the largest of the vector, exact integer
                          sums); complex sectors' dots in fixed point (57 bits below the largest of each
                          1024 or 256 entries, exact integer sums), real sectors' with FP32 values in
                          double-float. Products with real FP64 values are native FP64 either way. */

@@ -27,6 +27,12 @@ int blqh_debug_sector_index(const blqh_sector* s, int64_t n, const uint64_t* sta
  * kernels are used; -1 for a null matrix. */
 int blqh_debug_spmv_layout(const blqh_csr* M);
 
+/* The product of the Lanczos recurrence: x receives the vector after the last
+ * step (the start vector before the first one) and y = H x, computed as the
+ * next step would, from the split input that the last step left. Host arrays
+ * of dim doubles, 2 dim when complex. */
+int blqh_debug_lanczos_product(blqh_lanczos* L, double* x, double* y);
+
 /* The n-th device allocation that the library makes for this context from now
  * on fails with BLQH_ERR_NOMEM, once (n = 0: none). Returns what was left of
  * the previous request: 0 when it has been met (or none was made). */
