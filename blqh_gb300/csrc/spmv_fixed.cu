@@ -37,7 +37,9 @@
 
 namespace {
 
-// Row exponents, split off-diagonal values and the diagonal: one warp per row.
+// Row exponents, split off-diagonal values and the diagonal: one warp per row. The
+// exponent is raised until the row's sum of |q| stays below 2^67 (rows of up to 512
+// nonzeros always do), so that a product with |x| <= 2^59 units stays below 2^127.
 __global__ void __launch_bounds__(256) k_fix_matrix(const int64_t* __restrict__ rp, const int32_t* __restrict__ col,
                                                     const double2* __restrict__ val, int64_t dim,
                                                     int4* __restrict__ qv, int* __restrict__ qe,
@@ -59,19 +61,26 @@ __global__ void __launch_bounds__(256) k_fix_matrix(const int64_t* __restrict__ 
     }
     hw = __reduce_max_sync(0xffffffffu, hw);
     has = __any_sync(0xffffffffu, has);
-    const int E = (int)(hw >> 20) - 1023;
+    int E = word_exponent(hw);
+    for (;; E++) {
+      long long sum = 0;  // of |q| / 2^29, rounded up
+      for (int64_t k = s + lane; k < e; k += 32) {
+        int4 q = make_int4(0, 0, 0, 0);
+        if (col[k] != r) {
+          const double2 v = val[k];
+          quantize(v.x, E, q.x, q.y);
+          quantize(v.y, E, q.z, q.w);
+          sum += abs(q.x) + abs(q.z) + 2;
+        }
+        qv[k] = q;
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      if (sum <= 1LL << 38) break;
+    }
     if (lane == 0) {
       qe[r] = E;
       if (!has) diag[r] = make_double2(0.0, 0.0);
-    }
-    for (int64_t k = s + lane; k < e; k += 32) {
-      int4 q = make_int4(0, 0, 0, 0);
-      if (col[k] != r) {
-        const double2 v = val[k];
-        quantize(v.x, E, q.x, q.y);
-        quantize(v.y, E, q.z, q.w);
-      }
-      qv[k] = q;
     }
   }
 }

@@ -118,3 +118,25 @@ def test_rows_without_their_diagonal_term(B, kind, sec):
     assert err[0] <= err[1], err
     H.close()
     b.close()
+
+
+@pytest.mark.parametrize("kind,sec", [("mono", (24, 12, 0, 1)), ("spin", (8, 8, 4, 4, 1, 3)), ("ground", (14, 14, 7, 0, 3))],
+                         ids=str)
+def test_even_vectors_and_long_rows(B, kind, sec):
+    """Every entry of the vector as large as the largest one, each with the sign that makes one row's terms add up:
+    the largest sums that the row's 128 bits can meet."""
+    b, H = build(B, kind, sec)
+    csr = H.csr()
+    rp, col, val = csr
+    long = int(np.argmax(np.diff(rp)))
+    r = np.full(H.dim, 1 + 1j)
+    k = slice(rp[long], rp[long + 1])
+    r.real[col[k]] = np.where(val[k].real < 0, -1, 1)
+    r.imag[col[k]] = np.where(val[k].imag > 0, -1, 1)
+    L = B.Lanczos(H, max_steps=1, tol=0.0, start=r)
+    x, y = product(L, H.dim)
+    rows = np.unique(np.append(np.linspace(0, H.dim - 1, 2000).astype(int), long))
+    e, bound = errors(H, csr, x, y, rows)
+    assert np.all(e <= bound), float(np.max(e / bound))
+    for o in (L, H, b):
+        o.close()
