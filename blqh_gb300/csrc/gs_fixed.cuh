@@ -328,7 +328,7 @@ __device__ __forceinline__ void fx_add(long long* s, int a1, int a0, int b1, int
 
 // hi 2^64 + lo (signed) times 2^e, rounded to FP64 with integer operations (an
 // FP64 conversion by one lane takes the FP64 pipe as long as a full warp's).
-// Results below FP64's normal range are zero.
+// Results below FP64's normal range are zero, those above it infinite.
 __device__ __forceinline__ double fx_to_double(long long hi, unsigned long long lo, int e) {
   const bool neg = hi < 0;
   if (neg) {
@@ -342,6 +342,7 @@ __device__ __forceinline__ double fx_to_double(long long hi, unsigned long long 
   else top = lz ? ((unsigned long long)hi << lz) | (lo >> (64 - lz)) : (unsigned long long)hi;
   const int be = 127 - lz + e + 1023;
   if (be <= 0) return 0.0;
+  if (be >= 2047) return __longlong_as_double(0x7FF0000000000000LL | (neg ? 1LL << 63 : 0));
   const unsigned long long m = (top >> 11) + ((top >> 10) & 1);  // in [2^52, 2^53]
   const unsigned long long bits = ((unsigned long long)be << 52) + (m - (1ULL << 52));
   return __longlong_as_double((long long)(bits | (neg ? 1ULL << 63 : 0)));

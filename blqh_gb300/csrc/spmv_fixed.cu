@@ -39,7 +39,9 @@ namespace {
 
 // Row exponents, split off-diagonal values and the diagonal: one warp per row. The
 // exponent is raised until the row's sum of |q| stays below 2^67 (rows of up to 512
-// nonzeros always do), so that a product with |x| <= 2^59 units stays below 2^127.
+// nonzeros always do), so that a product with |x| <= 2^59 units stays below 2^127. A row
+// with an infinite or NaN entry, which has no integers, gets a NaN diagonal: its
+// product is then NaN.
 __global__ void __launch_bounds__(256) k_fix_matrix(const int64_t* __restrict__ rp, const int32_t* __restrict__ col,
                                                     const double2* __restrict__ val, int64_t dim,
                                                     int4* __restrict__ qv, int* __restrict__ qe,
@@ -81,6 +83,7 @@ __global__ void __launch_bounds__(256) k_fix_matrix(const int64_t* __restrict__ 
     if (lane == 0) {
       qe[r] = E;
       if (!has) diag[r] = make_double2(0.0, 0.0);
+      if (word_exponent(hw) == 1024) diag[r].x = diag[r].y = __longlong_as_double(0x7FF8000000000000LL);
     }
   }
 }

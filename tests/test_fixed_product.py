@@ -140,3 +140,24 @@ def test_even_vectors_and_long_rows(B, kind, sec):
     assert np.all(e <= bound), float(np.max(e / bound))
     for o in (L, H, b):
         o.close()
+
+
+def test_infinite_elements_stay_visible(B):
+    """A tunnelling amplitude at the end of FP64's range, which short orbits multiply beyond it: a row with an infinite
+    element has no finite product, and the recurrence no finite coefficient."""
+    b = B.basis_spin(4, 4, -1, -1, 0, 1)
+    H = B.hamiltonian_spin(b, 0.9, delta_sas=1.79e308)
+    assert H.is_complex
+    rp, col, val = H.csr()
+    row = np.repeat(np.arange(H.dim), np.diff(rp))
+    rows = np.unique(row[~(np.isfinite(val.real) & np.isfinite(val.imag)) & (col != row)])
+    assert len(rows)
+    for accumulate in (0, 1):
+        L = B.Lanczos(H, max_steps=1, tol=0.0, start=np.ones(H.dim), accumulate=accumulate)
+        y = product(L, H.dim)[1][rows]
+        assert not np.any(np.isfinite(y.real) & np.isfinite(y.imag))
+        L.iterate()
+        assert not np.isfinite(L.coeffs()[0][0])
+        L.close()
+    H.close()
+    b.close()
