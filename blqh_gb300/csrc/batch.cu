@@ -19,8 +19,9 @@
 // Daniel-Gragg-Kaufman-Stewart criterion). Real instances run the pass in FP64, in
 // a fixed order of operations (their ground states can be degenerate, see
 // gs_ordered.cuh, and then depend on it); complex instances take it on fixed-point
-// planes of the Krylov basis (gs_fixed.cuh), one exponent per vector: exact integer
-// dots, and the correction in FP32 while every coefficient is below 2^-30 |w|. The
+// planes of the Krylov basis (gs_fixed.cuh), one exponent per vector (57 bits below its
+// largest entry): exact integer dots (error against extended precision, random vectors
+// of 79 to 100,141 complex entries: 0.18 to 0.42 of the FP64 dots'), and the correction in FP32 while every coefficient is below 2^-30 |w|. The
 // FP64 pass of a complex instance took the SM's FP64 pipe 8 FMAs per entry and
 // vector; 96 instances of 5,940 states, 150 steps: 348 -> 134 ms. The lowest Ritz pair comes from
 // Sturm multisection and inverse iteration; the finisher is the FP64
@@ -383,16 +384,17 @@ __device__ __forceinline__ double cgs_update(const double* __restrict__ V, int64
 }
 
 // ---- the full pass of complex instances on fixed-point planes --------------------
-// Extra bits of headroom of an N-entry vector's exponent: 2 (57 - s) + log2 N + 1 bits
-// of a whole vector's sum stay below 2^126.
-__device__ __forceinline__ int plane_headroom(int64_t N) {
+// Bits that partial sums of an N-entry dot drop at their lower end so that the whole
+// of it (N products below 2^114) stays below 2^127: 2^-101 of its largest product
+// and less, nothing against the operands' 2^-57.
+__device__ __forceinline__ int sum_shift(int64_t N) {
   const int lg = 64 - __clzll(N);
-  return lg > 11 ? (lg - 10) / 2 : 0;
+  return lg > 12 ? lg - 12 : 0;
 }
 
-// Exponent of the block's largest |x| plus the headroom (in every thread).
+// Exponent of the block's largest |x| (in every thread).
 template <int NT>
-__device__ __forceinline__ int plane_exponent(unsigned hw, int64_t N, double* red) {
+__device__ __forceinline__ int plane_exponent(unsigned hw, double* red) {
   unsigned* ur = reinterpret_cast<unsigned*>(red);
   hw = __reduce_max_sync(0xffffffffu, hw);
   if ((threadIdx.x & 31) == 0) ur[threadIdx.x >> 5] = hw;
@@ -401,7 +403,7 @@ __device__ __forceinline__ int plane_exponent(unsigned hw, int64_t N, double* re
 #pragma unroll
   for (int i = 0; i < NT / 32; i++) m = max(m, ur[i]);
   __syncthreads();
-  return (int)(m >> 20) - 1023 + plane_headroom(N);
+  return word_exponent(m);
 }
 
 // Planes of x (N entries, FP64, written by this block) with exponent E; zeros up to NP.
@@ -422,7 +424,7 @@ template <int NT>
 __device__ __forceinline__ void cgs_dots_q(const int* __restrict__ q1, const int* __restrict__ q0, int64_t NP,
                                            const int* qe, int nk, const int* w1, const int* w0, int we, double* h) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int n4 = (int)(NP / 4);
+  const int n4 = (int)(NP / 4), shift = sum_shift(NP);
   for (int k = 2 * wid; k < nk; k += 2 * (NT / 32)) {
     const int kb = min(k + 1, nk - 1);  // a missing second vector repeats the first
     const int4* a1 = reinterpret_cast<const int4*>(q1 + k * NP);
@@ -453,9 +455,9 @@ __device__ __forceinline__ void cgs_dots_q(const int* __restrict__ q1, const int
         one(s[2], s[3], z1, z0, y1, y0);
       }
 #pragma unroll
-      for (int c = 0; c < 4; c++) t[c].fold(s[c]);
+      for (int c = 0; c < 4; c++) t[c].fold(s[c], shift);
     }
-    const int ea = qe[k] + we - 112, eb = qe[kb] + we - 112;
+    const int ea = qe[k] + we - 112 + shift, eb = qe[kb] + we - 112 + shift;
     const double ar = t[0].warp_sum(ea), ai = t[1].warp_sum(ea), br = t[2].warp_sum(eb), bi = t[3].warp_sum(eb);
     if (lane == 0) {
       h[2 * k] = ar;
@@ -583,7 +585,7 @@ __device__ void run_instance(const BInst& I, int lam, uint64_t seed, double bd_t
           hw = max(hw, abs_high_word(v));
         });
     if (planes) {
-      const int E = plane_exponent<NT>(hw, N, red);
+      const int E = plane_exponent<NT>(hw, red);
       if (threadIdx.x == 0) qe[0] = E;
       write_planes<NT>(I.V, N, NP, E, I.q1, I.q0);
     }
@@ -621,7 +623,7 @@ __device__ void run_instance(const BInst& I, int lam, uint64_t seed, double bd_t
       unsigned hw = 0;
       sweep<NT, 4>(
           N, [&](int i) { return I.w[i]; }, [&](int, double v) { hw = max(hw, abs_high_word(v)); });
-      const int we = plane_exponent<NT>(hw, N, red);
+      const int we = plane_exponent<NT>(hw, red);
       write_planes<NT>(I.w, N, NP, we, w1, w0);
       __syncthreads();
       cgs_dots_q<NT>(I.q1, I.q0, NP, qe, j + 1, w1, w0, we, hs);
@@ -674,7 +676,7 @@ __device__ void run_instance(const BInst& I, int lam, uint64_t seed, double bd_t
           hw = max(hw, abs_high_word(v));
         });
     if (planes) {
-      const int E = plane_exponent<NT>(hw, N, red);
+      const int E = plane_exponent<NT>(hw, red);
       if (threadIdx.x == 0) qe[j + 1] = E;
       write_planes<NT>(vn, N, NP, E, I.q1 + (int64_t)(j + 1) * NP, I.q0 + (int64_t)(j + 1) * NP);
     }
@@ -792,6 +794,24 @@ __global__ void k_rq_reduce(const double* __restrict__ part, const int64_t* __re
     for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += red[w];
     res[i][0] = t;
   }
+}
+
+// The instances' fixed-point dots of one vector w against nk others (blqh_debug_dots).
+constexpr int DEBUG_NT = 256;
+__global__ void __launch_bounds__(DEBUG_NT) k_debug_dots(const double* V, const double* w, int64_t N, int nk, int* q1,
+                                                         int* q0, int* qe, double* h) {
+  __shared__ double red[RED];
+  const int64_t NP = (N + 3) / 4 * 4;
+  for (int k = 0; k <= nk; k++) {
+    const double* x = k < nk ? V + k * N : w;
+    unsigned hw = 0;
+    for (int64_t i = threadIdx.x; i < N; i += DEBUG_NT) hw = max(hw, abs_high_word(x[i]));
+    const int E = plane_exponent<DEBUG_NT>(hw, red);
+    if (threadIdx.x == 0) qe[k] = E;
+    write_planes<DEBUG_NT>(x, N, NP, E, q1 + k * NP, q0 + k * NP);
+    __syncthreads();
+  }
+  cgs_dots_q<DEBUG_NT>(q1, q0, NP, qe, nk, q1 + nk * NP, q0 + nk * NP, qe[nk], h);
 }
 
 using KFn = void (*)(const BInst*, const int*, int, int, uint64_t, double, int, int*);
@@ -1191,6 +1211,17 @@ void batch_solve_impl(blqh_batch* b) {
 }
 
 }  // namespace
+
+// Complex vectors of N doubles, device pointers (see blqh_debug_dots).
+void debug_batch_dots(blqh_ctx* ctx, const double* V, const double* w, int64_t N, int nk, double* h) {
+  DevBufs G;
+  const size_t NP = (size_t)(N + 3) / 4 * 4;
+  int* q1 = G.add(dalloc<int>(ctx, NP * (nk + 1)));
+  int* q0 = G.add(dalloc<int>(ctx, NP * (nk + 1)));
+  int* qe = G.add(dalloc<int>(ctx, nk + 1));
+  k_debug_dots<<<1, DEBUG_NT, 0, ctx->stream>>>(V, w, N, nk, q1, q0, qe, h);
+  BLQH_TRY_CUDA(ctx, cudaGetLastError());
+}
 
 extern "C" {
 

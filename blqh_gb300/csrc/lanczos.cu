@@ -35,6 +35,7 @@ void spin_observables_impl(blqh_ctx* ctx, const blqh_basis* B, const double* psi
 double spin_rayleigh_regen_impl(blqh_ctx* ctx, const blqh_basis* B, const blqh_params_spin& p, const double* x);
 int hamil_build_impl(blqh_ctx* ctx, const blqh_basis* B, const blqh_params& p, int prec, blqh_csr* M);
 void free_csr(blqh_csr* m);
+void debug_batch_dots(blqh_ctx* ctx, const double* V, const double* w, int64_t N, int nk, double* h);
 
 namespace {
 
@@ -1196,9 +1197,74 @@ blqh_lanczos* create_impl(blqh_ctx* ctx, const blqh_csr* M, const blqh_lanczos_o
   return L;
 }
 
+// blqh_debug_dots on device pointers; part, S as in a Lanczos object of nk steps.
+template <int TILE>
+void debug_dots_q(blqh_ctx* ctx, DevBufs& G, const double* V, const double* w, int64_t n, int nk, double* part, Scal S) {
+  constexpr bool LOCAL = TILE == 256;
+  const int ntile = (int)((n + TILE - 1) / TILE), ng = (nk + DOT_GROUP - 1) / DOT_GROUP;
+  const int64_t pld = (int64_t)ntile * TILE;
+  int* q1 = G.add(dalloc<int>(ctx, pld * (nk + 1)));
+  int* q0 = G.add(dalloc<int>(ctx, pld * (nk + 1)));
+  int* qe = G.add(dalloc<int>(ctx, (size_t)ntile * (nk + 1)));
+  double2* apart = G.add(dalloc<double2>(ctx, 1));
+  double* npart = G.add(dalloc<double>(ctx, ntile));
+  BLQH_TRY_CUDA(ctx, cudaMemsetAsync(apart, 0, sizeof(double2), ctx->stream));
+  for (int k = 0; k <= nk; k++)
+    launch_chained(ctx, k_planes_q<TILE>, ntile, TILE / 4, 0, k < nk ? V + k * n : w, n,
+                   NextVec{nullptr, nullptr, nullptr, nullptr, q1 + k * pld, q0 + k * pld, qe + (int64_t)k * ntile});
+  const WTile W{w, w, apart, 1, q1 + nk * pld, q0 + nk * pld, qe + (int64_t)nk * ntile, npart};
+  launch_chained(ctx, k_dots_q<true, TILE, LOCAL>, ng * ntile, 256, 0, q1, q0, qe, pld, ntile, n, nk, ng, W, part, S,
+                 0);
+}
+
+void debug_dots_impl(blqh_ctx* ctx, int64_t n, int nk, const double* V, const double* w, int form, double* h) {
+  DevBufs G;
+  const int64_t dim = n / 2;
+  const int nt = (int)((dim + GS_ROWS - 1) / GS_ROWS);
+  double* dV = G.add(dalloc<double>(ctx, n * nk));
+  double* dw = G.add(dalloc<double>(ctx, n));
+  double* part = G.add(dalloc<double>(ctx, (size_t)(n / 256 + 1) * 2 * nk));
+  const size_t ns = 4 * nk + 16;
+  double* p = G.add(dalloc<double>(ctx, ns));
+  BLQH_TRY_CUDA(ctx, cudaMemsetAsync(p, 0, ns * 8, ctx->stream));
+  Scal S{};
+  S.alpha = p;
+  S.h2 = p + nk;
+  S.flags = reinterpret_cast<int*>(p + 3 * nk);
+  S.cnt = reinterpret_cast<unsigned*>(p + 3 * nk + 4);
+  double* pnorm = p + ns - 1;
+  BLQH_TRY_CUDA(ctx, cudaMemcpyAsync(dV, V, n * nk * 8, cudaMemcpyHostToDevice, ctx->stream));
+  BLQH_TRY_CUDA(ctx, cudaMemcpyAsync(dw, w, n * 8, cudaMemcpyHostToDevice, ctx->stream));
+  if (form == 0) {
+    launch_chained(ctx, k_dots_o<true, false, 1>, (nk + 7) / 8 * nt, 256, 0, dV, nullptr, nullptr, 0, dim, nt, nk, 8,
+                   (nk + 7) / 8, dw, part, pnorm, 1, 0, S, 0);
+    launch_chained(ctx, k_reduce_o<true>, nk, 256, 0, part, nt, pnorm, 1, S, 0);
+  } else if (form == 1) {
+    debug_dots_q<1024>(ctx, G, dV, dw, n, nk, part, S);
+  } else if (form == 2) {
+    debug_dots_q<256>(ctx, G, dV, dw, n, nk, part, S);
+  } else {
+    debug_batch_dots(ctx, dV, dw, n, nk, S.h2);
+  }
+  BLQH_TRY_CUDA(ctx, cudaMemcpyAsync(h, S.h2, 2 * nk * 8, cudaMemcpyDeviceToHost, ctx->stream));
+  BLQH_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+}
+
 }  // namespace
 
 extern "C" {
+
+int blqh_debug_dots(blqh_ctx* ctx, int64_t n, int nk, const double* V, const double* w, int form, double* h) {
+  if (!ctx || !V || !w || !h || n < 2 || n % 2 || n > (1 << 30) || nk < 1 || nk > BLQH_MAX_LAMBDA || form < 0 ||
+      form > 3)
+    return BLQH_ERR_ARG;
+  try {
+    debug_dots_impl(ctx, n, nk, V, w, form, h);
+  } catch (const BlqhError& e) {
+    return e.code;
+  }
+  return BLQH_OK;
+}
 
 int blqh_spmv(blqh_ctx* ctx, const blqh_csr* m, const double* x, double* y) {
   if (!ctx || !m || !x || !y) return BLQH_ERR_ARG;

@@ -33,6 +33,12 @@ int blqh_debug_spmv_layout(const blqh_csr* M);
  * of dim doubles, 2 dim when complex. */
 int blqh_debug_lanczos_product(blqh_lanczos* L, double* x, double* y);
 
+/* The Gram-Schmidt dots of complex sectors: h[k] = sum_i conj(V_k[i]) w[i] for
+ * nk vectors of n doubles (n even, host arrays). form: 0 = FP64, in the order
+ * of the plain pass; 1, 2 = fixed-point planes in tiles of 1024 and of 256
+ * doubles; 3 = fixed-point planes of the batched instances. */
+int blqh_debug_dots(blqh_ctx* ctx, int64_t n, int nk, const double* V, const double* w, int form, double* h);
+
 /* The n-th device allocation that the library makes for this context from now
  * on fails with BLQH_ERR_NOMEM, once (n = 0: none). Returns what was left of
  * the previous request: 0 when it has been met (or none was made). */
