@@ -21,7 +21,7 @@
 // gs_ordered.cuh, and then depend on it); complex instances take it on fixed-point
 // planes of the Krylov basis (gs_fixed.cuh), one exponent per vector (57 bits below its
 // largest entry): exact integer dots (error against extended precision, random vectors
-// of 79 to 100,141 complex entries: 0.18 to 0.42 of the FP64 dots'), and the correction in FP32 while every coefficient is below 2^-30 |w|. The
+// of 79 to 100,141 complex entries: 0.18 to 0.42 of the FP64 dots'), and the correction in FP32 while every coefficient is below 2^-36 |w|. The
 // FP64 pass of a complex instance took the SM's FP64 pipe 8 FMAs per entry and
 // vector; 96 instances of 5,940 states, 150 steps: 348 -> 134 ms. The lowest Ritz pair comes from
 // Sturm multisection and inverse iteration; the finisher is the FP64
@@ -470,8 +470,11 @@ __device__ __forceinline__ void cgs_dots_q(const int* __restrict__ q1, const int
   }
 }
 
-// Whether every coefficient is below 2^-30 of |w| (|w|^2 = nn), by exponents, and the
+// Whether every coefficient is below 2^-36 of |w| (|w|^2 = nn), by exponents, and the
 // coefficients times the planes' scale as FP32: value = q1 2^(E - 27). One flag in *ok.
+// The FP32 sum is good to about 2^-22 of itself, so below that line it errs by no more
+// than 2^-58 sqrt(nk) |w| over the vector; the FP64 form, which rounds w at every
+// vector, by about 2^-55 sqrt(nk) |w|.
 template <int NT>
 __device__ __forceinline__ void plane_coefs(const double* h, const int* qe, int nk, double nn, float2* hf, int* ok) {
   if (threadIdx.x == 0) *ok = 1;
@@ -480,7 +483,7 @@ __device__ __forceinline__ void plane_coefs(const double* h, const int* qe, int 
   bool small = true;
   for (int k = threadIdx.x; k < nk; k += NT) {
     const int eh = (int)(max(abs_high_word(h[2 * k]), abs_high_word(h[2 * k + 1])) >> 20) - 1023;
-    small = small && 2 * (eh + 2) <= en - 60;
+    small = small && 2 * (eh + 2) <= en - 72;
     const int e = qe[k] - 27;
     const float sc = e < -126 ? 0.0f : __uint_as_float((unsigned)(e + 127) << 23);
     hf[k] = make_float2(f64_lead_f32(h[2 * k]) * sc, f64_lead_f32(h[2 * k + 1]) * sc);
@@ -796,10 +799,11 @@ __global__ void k_rq_reduce(const double* __restrict__ part, const int64_t* __re
   }
 }
 
-// The instances' fixed-point dots of one vector w against nk others (blqh_debug_dots).
+// The instances' fixed-point dots of one vector w against nk others into h (blqh_debug_dots)
+// or, with hf, their correction of w by given coefficients h (blqh_debug_batch_update).
 constexpr int DEBUG_NT = 256;
-__global__ void __launch_bounds__(DEBUG_NT) k_debug_dots(const double* V, const double* w, int64_t N, int nk, int* q1,
-                                                         int* q0, int* qe, double* h) {
+__global__ void __launch_bounds__(DEBUG_NT) k_debug_pass(const double* V, double* w, int64_t N, int nk, int* q1,
+                                                         int* q0, int* qe, double* h, float2* hf) {
   __shared__ double red[RED];
   const int64_t NP = (N + 3) / 4 * 4;
   for (int k = 0; k <= nk; k++) {
@@ -811,7 +815,17 @@ __global__ void __launch_bounds__(DEBUG_NT) k_debug_dots(const double* V, const 
     write_planes<DEBUG_NT>(x, N, NP, E, q1 + k * NP, q0 + k * NP);
     __syncthreads();
   }
-  cgs_dots_q<DEBUG_NT>(q1, q0, NP, qe, nk, q1 + nk * NP, q0 + nk * NP, qe[nk], h);
+  if (!hf) {
+    cgs_dots_q<DEBUG_NT>(q1, q0, NP, qe, nk, q1 + nk * NP, q0 + nk * NP, qe[nk], h);
+    return;
+  }
+  __shared__ int ok;
+  double nn = 0.0, z = 0.0;
+  for (int64_t i = threadIdx.x; i < N; i += DEBUG_NT) nn += w[i] * w[i];
+  block_sum2<DEBUG_NT>(nn, z, red);
+  plane_coefs<DEBUG_NT>(h, qe, nk, nn, hf, &ok);
+  if (ok) cgs_update_q<DEBUG_NT>(q1, NP, nk, hf, w, N);
+  else cgs_update<DEBUG_NT, true>(V, N, nk, h, w);
 }
 
 using KFn = void (*)(const BInst*, const int*, int, int, uint64_t, double, int, int*);
@@ -1212,14 +1226,15 @@ void batch_solve_impl(blqh_batch* b) {
 
 }  // namespace
 
-// Complex vectors of N doubles, device pointers (see blqh_debug_dots).
-void debug_batch_dots(blqh_ctx* ctx, const double* V, const double* w, int64_t N, int nk, double* h) {
+// Complex vectors of N doubles, device pointers (see blqh_debug_dots and, with update, blqh_debug_batch_update).
+void debug_batch_pass(blqh_ctx* ctx, const double* V, double* w, int64_t N, int nk, double* h, bool update) {
   DevBufs G;
   const size_t NP = (size_t)(N + 3) / 4 * 4;
   int* q1 = G.add(dalloc<int>(ctx, NP * (nk + 1)));
   int* q0 = G.add(dalloc<int>(ctx, NP * (nk + 1)));
   int* qe = G.add(dalloc<int>(ctx, nk + 1));
-  k_debug_dots<<<1, DEBUG_NT, 0, ctx->stream>>>(V, w, N, nk, q1, q0, qe, h);
+  float2* hf = update ? G.add(dalloc<float2>(ctx, nk)) : nullptr;
+  k_debug_pass<<<1, DEBUG_NT, 0, ctx->stream>>>(V, w, N, nk, q1, q0, qe, h, hf);
   BLQH_TRY_CUDA(ctx, cudaGetLastError());
 }
 

@@ -35,7 +35,7 @@ void spin_observables_impl(blqh_ctx* ctx, const blqh_basis* B, const double* psi
 double spin_rayleigh_regen_impl(blqh_ctx* ctx, const blqh_basis* B, const blqh_params_spin& p, const double* x);
 int hamil_build_impl(blqh_ctx* ctx, const blqh_basis* B, const blqh_params& p, int prec, blqh_csr* M);
 void free_csr(blqh_csr* m);
-void debug_batch_dots(blqh_ctx* ctx, const double* V, const double* w, int64_t N, int nk, double* h);
+void debug_batch_pass(blqh_ctx* ctx, const double* V, double* w, int64_t N, int nk, double* h, bool update);
 
 namespace {
 
@@ -1244,7 +1244,7 @@ void debug_dots_impl(blqh_ctx* ctx, int64_t n, int nk, const double* V, const do
   } else if (form == 2) {
     debug_dots_q<256>(ctx, G, dV, dw, n, nk, part, S);
   } else {
-    debug_batch_dots(ctx, dV, dw, n, nk, S.h2);
+    debug_batch_pass(ctx, dV, dw, n, nk, S.h2, false);
   }
   BLQH_TRY_CUDA(ctx, cudaMemcpyAsync(h, S.h2, 2 * nk * 8, cudaMemcpyDeviceToHost, ctx->stream));
   BLQH_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -1253,6 +1253,25 @@ void debug_dots_impl(blqh_ctx* ctx, int64_t n, int nk, const double* V, const do
 }  // namespace
 
 extern "C" {
+
+int blqh_debug_batch_update(blqh_ctx* ctx, int64_t n, int nk, const double* V, double* w, const double* h) {
+  if (!ctx || !V || !w || !h || n < 2 || n % 2 || n > (1 << 30) || nk < 1 || nk > BLQH_MAX_LAMBDA) return BLQH_ERR_ARG;
+  try {
+    DevBufs G;
+    double* dV = G.add(dalloc<double>(ctx, n * nk));
+    double* dw = G.add(dalloc<double>(ctx, n));
+    double* dh = G.add(dalloc<double>(ctx, 2 * nk));
+    BLQH_TRY_CUDA(ctx, cudaMemcpyAsync(dV, V, n * nk * 8, cudaMemcpyHostToDevice, ctx->stream));
+    BLQH_TRY_CUDA(ctx, cudaMemcpyAsync(dw, w, n * 8, cudaMemcpyHostToDevice, ctx->stream));
+    BLQH_TRY_CUDA(ctx, cudaMemcpyAsync(dh, h, 2 * nk * 8, cudaMemcpyHostToDevice, ctx->stream));
+    debug_batch_pass(ctx, dV, dw, n, nk, dh, true);
+    BLQH_TRY_CUDA(ctx, cudaMemcpyAsync(w, dw, n * 8, cudaMemcpyDeviceToHost, ctx->stream));
+    BLQH_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  } catch (const BlqhError& e) {
+    return e.code;
+  }
+  return BLQH_OK;
+}
 
 int blqh_debug_dots(blqh_ctx* ctx, int64_t n, int nk, const double* V, const double* w, int form, double* h) {
   if (!ctx || !V || !w || !h || n < 2 || n % 2 || n > (1 << 30) || nk < 1 || nk > BLQH_MAX_LAMBDA || form < 0 ||

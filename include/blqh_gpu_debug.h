@@ -39,6 +39,10 @@ int blqh_debug_lanczos_product(blqh_lanczos* L, double* x, double* y);
  * doubles; 3 = fixed-point planes of the batched instances. */
 int blqh_debug_dots(blqh_ctx* ctx, int64_t n, int nk, const double* V, const double* w, int form, double* h);
 
+/* The Gram-Schmidt correction of the batched complex instances, w -= sum_k h_k V_k,
+ * in the form that the coefficients' size selects there (host arrays as above). */
+int blqh_debug_batch_update(blqh_ctx* ctx, int64_t n, int nk, const double* V, double* w, const double* h);
+
 /* The n-th device allocation that the library makes for this context from now
  * on fails with BLQH_ERR_NOMEM, once (n = 0: none). Returns what was left of
  * the previous request: 0 when it has been met (or none was made). */

@@ -93,3 +93,30 @@ def test_krylov_vectors(sec, d):
     assert all(err[f] <= err[0] for f in FORMS), err
     H.close()
     b.close()
+
+
+@pytest.mark.parametrize("size", [2.0 ** -29, 2.0 ** -31, 2.0 ** -33, 2.0 ** -35, 2.0 ** -38, 2.0 ** -46])
+@pytest.mark.parametrize("dim", [79, 5940, 60096])
+def test_batched_correction(dim, size):
+    """w - sum_k h_k V_k of 64 random vectors, coefficients of about `size` of |w|: no further off than the plain FP64
+    sum, which subtracts vector by vector (restated here), whichever form the instances take."""
+    import blqh_gb300 as B
+    from blqh_gb300._lib import lib
+
+    rng = np.random.default_rng(dim)
+    V = rng.standard_normal((64, 2 * dim)).view(np.complex128)
+    V /= np.linalg.norm(V, axis=1, keepdims=True)
+    w = rng.standard_normal(2 * dim).view(np.complex128)
+    w /= np.linalg.norm(w)
+    h = rng.choice([-1, 1], 128).view() * size * rng.uniform(0.5, 1.0, 128)
+    h = h.view(np.complex128)
+    ref = w.astype(np.clongdouble) - np.sum(h.astype(np.clongdouble)[:, None] * V.astype(np.clongdouble), axis=0)
+    plain = w.copy()
+    for k in range(64):
+        plain -= h[k] * V[k]
+    ctx = B.Context.default()
+    out = w.copy()
+    ctx.check(lib().blqh_debug_batch_update(ctx.h, 2 * dim, 64, *(a.ctypes.data_as(ctypes.c_void_p) for a in (V, out, h))))
+    err, native = rms(out, ref), rms(plain, ref)
+    print("update", dim, size, "%.3f" % (err / native))
+    assert err <= native * (1 + 1e-3), (err, native)  # (the FP64 form is the same sum up to fused operations)
