@@ -164,6 +164,7 @@ DEBUG_SIGNATURES = [
     ("blqh_debug_lanczos_product", _i, [_vp, _vp, _vp]),
     ("blqh_debug_dots", _i, [_vp, _i64, _i, _vp, _vp, _i, _vp]),
     ("blqh_debug_batch_update", _i, [_vp, _i64, _i, _vp, _vp, _vp]),
+    ("blqh_debug_free_bytes", _i, [_vp, _i64]),
     ("blqh_debug_fail_alloc", _i, [_vp, _i]),
 ]
 

@@ -48,6 +48,7 @@ struct blqh_ctx {
   std::vector<std::pair<int, std::pair<cudaEvent_t, cudaEvent_t>>> pending;
   // small pinned host buffer for scalar read-backs
   double* pinned = nullptr;
+  int64_t free_bytes = -1;  // what optional_room takes for the free device memory (blqh_debug_free_bytes), -1: ask
   int fail_alloc = 0;  // allocations until one is made to fail (blqh_debug_fail_alloc), 0: none
 };
 
@@ -55,6 +56,10 @@ struct blqh_ctx {
 // context after dev_free (see runtime.cu); dev_forget_ctx releases a context's.
 void* dev_alloc(blqh_ctx* ctx, size_t bytes);
 void dev_free(void* p);
+// Device memory that a call may take on top of what it needs: half of what is free, so
+// that later calls find the rest. (Below 64 MB it makes no difference and is not asked.)
+size_t optional_bytes(blqh_ctx* ctx);
+bool optional_room(blqh_ctx* ctx, size_t bytes);
 void dev_forget_ctx(blqh_ctx* ctx);
 template <class T>
 T* dalloc(blqh_ctx* ctx, size_t n) {

@@ -1152,7 +1152,11 @@ blqh_lanczos* create_impl(blqh_ctx* ctx, const blqh_csr* M, const blqh_lanczos_o
     L->work = dalloc<double>(ctx, 8 * (size_t)m + 16);
     L->y = dalloc<double>(ctx, m + 1);
     if (M->precision == BLQH_VAL_FP32 && o.accumulate == 0) L->xs = dalloc<float2>(ctx, n + 2);
-    if (!o.accumulate && fixed_prepare(ctx, M, &L->fx)) try {
+    // a fixed-point copy and planes of FP64-valued runs come on top of what those need, FP32-valued
+    // runs count on theirs
+    const bool fp64 = M->precision == BLQH_VAL_FP64;
+    const size_t copy = (size_t)M->nnz * 16 + (size_t)M->dim * 20 + (size_t)n * 8;
+    if (!o.accumulate && optional_room(ctx, copy) && fixed_prepare(ctx, M, &L->fx)) try {
         L->xq = dalloc<int2>(ctx, n + 2 + L->nblk_upd);
         L->xe = reinterpret_cast<int*>(L->xq + n);
         L->pmax = reinterpret_cast<unsigned*>(L->xq + n + 2);
@@ -1162,7 +1166,8 @@ blqh_lanczos* create_impl(blqh_ctx* ctx, const blqh_csr* M, const blqh_lanczos_o
         ctx->last_error.clear();
       }
     // (real sectors with accumulate = 1 keep the FP32 plane for the correction, not for the dots)
-    if (o.reorth && gs_planes_enabled() && !(L->cplx && o.accumulate)) {
+    const size_t planes = (size_t)(m + 2) * n * (L->cplx ? 8 : 4);
+    if (o.reorth && gs_planes_enabled() && !(L->cplx && o.accumulate) && (!fp64 || optional_room(ctx, planes))) {
       // the planes take up to the Krylov basis' memory again; without room for
       // them the run works on the FP64 vectors
       try {

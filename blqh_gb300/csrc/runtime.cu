@@ -133,6 +133,21 @@ void dev_free(void* p) {
   g_cached_bytes += l.bytes;
 }
 
+size_t optional_bytes(blqh_ctx* ctx) {
+  if (ctx->free_bytes >= 0) return (size_t)ctx->free_bytes / 2;
+  size_t free = 0, total = 0;
+  if (cudaMemGetInfo(&free, &total) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  std::lock_guard<std::mutex> lk(g_mem_mu);
+  return (free + g_cached_bytes) / 2;
+}
+
+bool optional_room(blqh_ctx* ctx, size_t bytes) {
+  return (ctx->free_bytes < 0 && bytes < ((size_t)64 << 20)) || bytes <= optional_bytes(ctx);
+}
+
 // On context destruction: cached blocks are freed, live ones lose their context.
 void dev_forget_ctx(blqh_ctx* ctx) {
   std::lock_guard<std::mutex> lk(g_mem_mu);
@@ -338,6 +353,12 @@ void scan_exclusive_u32_to_i64(blqh_ctx* ctx, const uint32_t* in, int64_t* out, 
 
 // ---------------------------------------------------------------------------
 extern "C" {
+
+int blqh_debug_free_bytes(blqh_ctx* ctx, int64_t bytes) {
+  if (!ctx) return BLQH_ERR_ARG;
+  ctx->free_bytes = bytes;
+  return BLQH_OK;
+}
 
 int blqh_debug_fail_alloc(blqh_ctx* ctx, int n) {
   if (!ctx) return 0;

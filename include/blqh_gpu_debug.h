@@ -48,6 +48,10 @@ int blqh_debug_batch_update(blqh_ctx* ctx, int64_t n, int nk, const double* V, d
  * the previous request: 0 when it has been met (or none was made). */
 int blqh_debug_fail_alloc(blqh_ctx* ctx, int n);
 
+/* Device memory that this context takes to be free when it decides on storage
+ * that a call can do without (-1: what the device says). */
+int blqh_debug_free_bytes(blqh_ctx* ctx, int64_t bytes);
+
 #ifdef __cplusplus
 }
 #endif

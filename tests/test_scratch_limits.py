@@ -129,3 +129,43 @@ def test_lanczos(ctx, monkeypatch, sec, prec, spare):
     assert all(any(np.array_equal(r, m) for m in modes) for r in got)
     H.close()
     b.close()
+
+
+@pytest.mark.parametrize("sec,prec", [r[:2] for r in RUNS], ids=str)
+def test_lanczos_leaves_memory_to_later_calls(ctx, monkeypatch, sec, prec):
+    """FP64-valued runs take their copies and planes only while half of the free memory holds them: with none of it
+    they return the bits of the run without either. FP32-valued runs count on theirs."""
+    import blqh_gb300 as B
+    from blqh_gb300._lib import lib
+
+    b = B.Basis(*sec, ctx=ctx)
+    H = B.Hamiltonian(b, 0.9, precision=B.VAL_FP64 if prec == "f64" else B.VAL_FP32)
+
+    def run():
+        L = B.Lanczos(H, max_steps=40, tol=0.0, seed=3)
+        L.iterate()
+        r = np.concatenate([*L.coeffs(), L.ritz_vector().view(np.float64)])
+        L.close()
+        return r
+
+    full = run()
+    monkeypatch.setenv("BLQH_SPMV_FIXED", "0")
+    monkeypatch.setenv("BLQH_GS_FP64", "1")
+    bare = run()
+    monkeypatch.undo()
+
+    def allocations():
+        lib().blqh_debug_fail_alloc(ctx.h, 100000)
+        r = run()
+        return r, 100000 - lib().blqh_debug_fail_alloc(ctx.h, 0)
+
+    _, most = allocations()
+    lib().blqh_debug_free_bytes(ctx.h, 1000)
+    r, least = allocations()
+    assert np.array_equal(r, bare if prec == "f64" else full)
+    assert (least < most) == (prec == "f64")
+    lib().blqh_debug_free_bytes(ctx.h, 1 << 40)
+    r, n = allocations()
+    assert n == most and np.array_equal(r, full)
+    H.close()
+    b.close()
