@@ -68,9 +68,9 @@ __host__ __device__ inline int batch_fixed_doubles(int lam) {
 
 // Per-instance device storage, in doubles from the instance's block (each array 256-byte aligned).
 struct Lay {
-  size_t V, w, psi, ab, xg, q1, q0, total;
+  size_t V, w, psi, ab, xg, total;
 };
-inline Lay instance_layout(int64_t N, int lam, bool xsmem, bool planes) {
+inline Lay instance_layout(int64_t N, int lam, bool xsmem) {
   auto up = [](size_t v) { return (v + 31) / 32 * 32; };
   Lay L;
   L.V = 0;
@@ -78,12 +78,11 @@ inline Lay instance_layout(int64_t N, int lam, bool xsmem, bool planes) {
   L.psi = up(L.w + N);
   L.ab = up(L.psi + N);
   L.xg = up(L.ab + 2 * lam + 1);
-  const size_t q = planes ? up((size_t)(lam + 2) * (size_t)((N + 3) / 4 * 4) / 2 + 1) : 0;  // ints
-  L.q1 = up(L.xg + (xsmem ? 0 : (size_t)N));
-  L.q0 = L.q1 + q;
-  L.total = L.q0 + q;
+  L.total = up(L.xg + (xsmem ? 0 : (size_t)N));
   return L;
 }
+// One plane of a complex instance: w's after the lam + 1 vectors' (ints, 256-byte aligned).
+inline size_t plane_ints(int64_t N, int lam) { return ((size_t)(lam + 2) * (size_t)((N + 3) / 4 * 4) + 63) / 64 * 64; }
 
 template <int NT>
 __device__ __forceinline__ void block_sum2(double& a, double& b, double* red) {
@@ -853,6 +852,7 @@ struct blqh_batch {
   std::vector<int64_t> N;            // doubles per vector
   std::vector<size_t> pool_off;      // doubles from the pool start
   double* pool = nullptr;
+  int* qpool = nullptr;              // fixed-point planes of the complex instances (of as many as there is room for)
   double* d_resall = nullptr;        // [n][5] results
   BInst* d_inst = nullptr;
   int* d_order = nullptr;
@@ -870,11 +870,10 @@ struct blqh_batch {
   cudaGraphExec_t gexec = nullptr;
   cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};  // before the Lanczos launch, after it, after the finisher
   bool solved = false;
-  bool planes = true;                // fixed-point planes for complex instances
   Lay layout(int i) const {
     const bool cplx = csr[i]->is_complex;
     // (the x area may grow after the tuning, so complex instances keep a global one)
-    return instance_layout(N[i], o.lambda, !cplx && N[i] * 8 <= x_cap, planes && cplx);
+    return instance_layout(N[i], o.lambda, !cplx && N[i] * 8 <= x_cap);
   }
 };
 
@@ -890,6 +889,7 @@ void batch_free(blqh_batch* b) {
   for (auto* m : b->csr) free_csr(m);
   for (auto* s : b->bases) blqh_basis_destroy(s);
   dev_free(b->pool);
+  dev_free(b->qpool);
   dev_free(b->d_resall);
   dev_free(b->d_inst);
   dev_free(b->d_order);
@@ -1038,23 +1038,31 @@ void batch_create_impl(blqh_batch* b) {
   configure_shape(b, b->o.threads ? b->o.threads : 256,
                   b->o.lanes_per_row ? b->o.lanes_per_row : lpr_for(b->mean_row));
   // device storage per instance (instance_layout)
-  for (;;) {
-    b->pool_off.assign(b->n, 0);
-    size_t total = 0;
-    for (int i = 0; i < b->n; i++) {
-      if (!b->csr[i]) continue;
-      b->pool_off[i] = total;
-      total += b->layout(i).total;
-    }
-    try {
-      b->pool = dalloc<double>(ctx, total + 32);
-      break;
-    } catch (const BlqhError& e) {  // without room for the planes: the FP64 pass
-      if (e.code != BLQH_ERR_NOMEM || !b->planes) throw;
-      b->planes = false;
+  b->pool_off.assign(b->n, 0);
+  size_t total = 0;
+  for (int i = 0; i < b->n; i++) {
+    if (!b->csr[i]) continue;
+    b->pool_off[i] = total;
+    total += b->layout(i).total;
+  }
+  b->pool = dalloc<double>(ctx, total + 32);
+  // planes (as much again) for the first complex instances that half of the free memory
+  // holds; the others take the FP64 pass
+  std::vector<size_t> plane_at(b->n, SIZE_MAX);
+  size_t ints = 0;
+  const size_t room = optional_bytes(ctx) / sizeof(int);
+  for (int i = 0; i < b->n; i++) {
+    const size_t need = b->csr[i] && b->csr[i]->is_complex ? 2 * plane_ints(b->N[i], lam) : 0;
+    if (!need || ints + need > room) continue;
+    plane_at[i] = ints;
+    ints += need;
+  }
+  if (ints) try {
+      b->qpool = dalloc<int>(ctx, ints);
+    } catch (const BlqhError& e) {
+      if (e.code != BLQH_ERR_NOMEM) throw;
       ctx->last_error.clear();
     }
-  }
   b->d_resall = dalloc<double>(ctx, 5 * (size_t)std::max(1, b->n));  // every instance's results, read back at once
   std::vector<BInst> hi;
   std::vector<double> cost;
@@ -1080,9 +1088,9 @@ void batch_create_impl(blqh_batch* b) {
     I.ab = p + L.ab;
     I.res = b->d_resall + 5 * (size_t)i;
     I.xg = I.xsmem && !I.cplx ? nullptr : p + L.xg;
-    if (b->planes && I.cplx) {
-      I.q1 = reinterpret_cast<int*>(p + L.q1);
-      I.q0 = reinterpret_cast<int*>(p + L.q0);
+    if (b->qpool && plane_at[i] != SIZE_MAX) {
+      I.q1 = b->qpool + plane_at[i];
+      I.q0 = I.q1 + plane_ints(Ni, lam);
     }
     hi.push_back(I);
     // cost: SpMV bytes and reorthogonalization work over lam steps

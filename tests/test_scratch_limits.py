@@ -169,3 +169,46 @@ def test_lanczos_leaves_memory_to_later_calls(ctx, monkeypatch, sec, prec):
     assert n == most and np.array_equal(r, full)
     H.close()
     b.close()
+
+
+def _batch(ctx, prec="f64"):
+    import blqh_gb300 as B
+
+    b = B.Batch([B.instance(8, 8, 4, 0, k, 0.9) for k in (1, 0, 2, 3)], lam=40, threads=256, lanes_per_row=8, ctx=ctx,
+                precision=B.VAL_FP64 if prec == "f64" else B.VAL_FP32)
+    b.solve()
+    r = [np.concatenate([[x["energy"], x["ritz0"]], b.ground_state(i).view(np.float64)])
+         for i, x in enumerate(b.results())]
+    b.close()
+    return r
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+def test_batch(ctx, prec):
+    """Each allocation of a batch fails in turn: without the planes' buffer its complex instances take the FP64 pass
+    (energies and, up to the convergence of 40 steps, vectors agree), the real one the bits it always has."""
+    full = _batch(ctx, prec)
+    got = [r for r in sweep(ctx, lambda: _batch(ctx, prec), 2000) if r is not None]
+    assert len(got) >= 1
+    for r in got:
+        assert np.array_equal(r[1], full[1])
+        for a, f in zip(r, full):
+            assert abs(a[0] - f[0]) < 1e-10 and np.max(abs(a - f)) < 1e-6
+
+
+def test_batch_with_planes_for_some_instances(ctx):
+    """As many complex instances as half of the free memory holds planes for take the fixed-point pass, the others the
+    FP64 pass; the real instance (the second) is not concerned. 79 states, 158 doubles: two planes of 42 rows of 160."""
+    from blqh_gb300._lib import lib
+
+    full = _batch(ctx)
+    out = {}
+    for n in range(4):
+        lib().blqh_debug_free_bytes(ctx.h, 2 * n * (2 * 42 * 160 * 4))
+        out[n] = _batch(ctx)
+    lib().blqh_debug_free_bytes(ctx.h, -1)
+    for n in range(4):
+        for i, rank in ((0, 1), (2, 2), (3, 3)):
+            assert np.array_equal(out[n][i], full[i] if n >= rank else out[0][i])
+        assert np.array_equal(out[n][1], full[1])
+    assert any(not np.array_equal(out[0][i], full[i]) for i in (0, 2, 3))
