@@ -49,8 +49,7 @@
 struct Scal {
   double* alpha;  // [mmax]
   double* beta;   // [mmax+1]; beta[0] = 0 internally
-  double* h;      // [2*(mmax+1)] Gram-Schmidt coefficients (re, im)
-  double* h2;     // [2*(mmax+1)] full pass
+  double* h2;     // [2*(mmax+1)] coefficients of the full pass (re, im)
   double* nrm;    // [4]: [2], [3] scratch
   double* ritz;   // [mmax] lowest Ritz value at checks
   int* flags;     // [8]: stop, -, steps, breakdown, a coefficient of the ordered full pass not small,
@@ -208,37 +207,31 @@ __device__ __forceinline__ double sum_partials(const double* p, int n) {
 }
 
 // Block partials (re, im) of h_j = conj(V_j) w, w after the SpMV.
-template <bool CPLX>
-__global__ void __launch_bounds__(256) k_alpha(const double* vj, const double* w, int64_t dim, double2* part, Scal S) {
+static __global__ void __launch_bounds__(256) k_alpha(const double* vj, const double* w, int64_t dim, double2* part, Scal S) {
   pdl_begin();
   __shared__ double red[8];
   double sr = 0, si = 0;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < dim; i += stride) {
-    if (CPLX) {
-      const double2 a = reinterpret_cast<const double2*>(vj)[i], b = reinterpret_cast<const double2*>(w)[i];
-      sr += a.x * b.x + a.y * b.y;
-      si += a.x * b.y - a.y * b.x;
-    } else {
-      sr += vj[i] * w[i];
-    }
+    const double2 a = reinterpret_cast<const double2*>(vj)[i], b = reinterpret_cast<const double2*>(w)[i];
+    sr += a.x * b.x + a.y * b.y;
+    si += a.x * b.y - a.y * b.x;
   }
   if (S.flags[0]) return;
   sr = block_sum_256(sr, red);
-  if (CPLX) si = block_sum_256(si, red);
+  si = block_sum_256(si, red);
   if (threadIdx.x == 0) part[blockIdx.x] = make_double2(sr, si);
 }
 
-// w' = w - h v for one entry (real), and for one complex entry.
-__device__ __forceinline__ double three_term(double w, double v, double2 h) { return w - h.x * v; }
+// w' = w - h v for one complex entry.
 __device__ __forceinline__ double2 three_term(double2 w, double2 v, double2 h) {
   return make_double2(w.x - (h.x * v.x - h.y * v.y), w.y - (h.x * v.y + h.y * v.x));
 }
 
 // Three-term step: w -= h_j V_j (the SpMV removed beta_j v_{j-1}), partials of
-// |w|^2 per tile, and w's fixed-point planes for the full pass when w1 is set. One
-// block of TILE / 4 threads per tile.
-template <bool CPLX, int TILE>
+// |w|^2 per tile, and w's fixed-point planes for the full pass. One block of TILE / 4
+// threads per tile.
+template <int TILE>
 __global__ void __launch_bounds__(TILE / 4) k_local(const double* vj, double* w, int64_t n, const double2* apart,
                                                     int na, int* w1, int* w0, int* we, double* part, Scal S, int j) {
   pdl_begin();
@@ -250,21 +243,15 @@ __global__ void __launch_bounds__(TILE / 4) k_local(const double* vj, double* w,
   const int stop = S.flags[0];
   double a[4], v[4];
 #pragma unroll
-  for (int q = 0; q < 4; q += CPLX ? 2 : 1) {
-    if (CPLX) {
-      const int64_t i = e0 + 2 * ((q >> 1) * T + threadIdx.x);
-      const bool in = i < n;
-      const double2 x = in ? *reinterpret_cast<const double2*>(w + i) : make_double2(0.0, 0.0);
-      const double2 y = in ? *reinterpret_cast<const double2*>(vj + i) : make_double2(0.0, 0.0);
-      a[q] = x.x;
-      a[q + 1] = x.y;
-      v[q] = y.x;
-      v[q + 1] = y.y;
-    } else {
-      const int64_t i = e0 + q * T + threadIdx.x;
-      a[q] = i < n ? w[i] : 0.0;
-      v[q] = i < n ? vj[i] : 0.0;
-    }
+  for (int q = 0; q < 4; q += 2) {
+    const int64_t i = e0 + 2 * ((q >> 1) * T + threadIdx.x);
+    const bool in = i < n;
+    const double2 x = in ? *reinterpret_cast<const double2*>(w + i) : make_double2(0.0, 0.0);
+    const double2 y = in ? *reinterpret_cast<const double2*>(vj + i) : make_double2(0.0, 0.0);
+    a[q] = x.x;
+    a[q + 1] = x.y;
+    v[q] = y.x;
+    v[q + 1] = y.y;
   }
   if (stop) return;
   if (threadIdx.x < 32) {
@@ -279,42 +266,25 @@ __global__ void __launch_bounds__(TILE / 4) k_local(const double* vj, double* w,
   double nn = 0;
   unsigned hw = 0;
 #pragma unroll
-  for (int q = 0; q < 4; q += CPLX ? 2 : 1) {
-    if (CPLX) {
-      const int64_t i = e0 + 2 * ((q >> 1) * T + threadIdx.x);
-      const double2 x = three_term(make_double2(a[q], a[q + 1]), make_double2(v[q], v[q + 1]), h);
-      if (i < n) *reinterpret_cast<double2*>(w + i) = x;
-      a[q] = x.x;
-      a[q + 1] = x.y;
-      nn += x.x * x.x + x.y * x.y;
-      hw = max(hw, max(abs_high_word(x.x), abs_high_word(x.y)));
-    } else {
-      const int64_t i = e0 + q * T + threadIdx.x;
-      a[q] = three_term(a[q], v[q], h);
-      if (i < n) w[i] = a[q];
-      nn += a[q] * a[q];
-      hw = max(hw, abs_high_word(a[q]));
-    }
+  for (int q = 0; q < 4; q += 2) {
+    const int64_t i = e0 + 2 * ((q >> 1) * T + threadIdx.x);
+    const double2 x = three_term(make_double2(a[q], a[q + 1]), make_double2(v[q], v[q + 1]), h);
+    if (i < n) *reinterpret_cast<double2*>(w + i) = x;
+    a[q] = x.x;
+    a[q + 1] = x.y;
+    nn += x.x * x.x + x.y * x.y;
+    hw = max(hw, max(abs_high_word(x.x), abs_high_word(x.y)));
   }
-  if (w1) {
-    const int E = block_exponent(hw, ured);
-    if (threadIdx.x == 0) we[blockIdx.x] = E;
+  const int E = block_exponent(hw, ured);
+  if (threadIdx.x == 0) we[blockIdx.x] = E;
 #pragma unroll
-    for (int q = 0; q < 4; q += CPLX ? 2 : 1) {
-      int q1, q0;
-      quantize(a[q], E, q1, q0);
-      if (CPLX) {
-        int p1, p0;
-        quantize(a[q + 1], E, p1, p0);
-        const int64_t i = e0 / 2 + (q >> 1) * T + threadIdx.x;
-        reinterpret_cast<int2*>(w1)[i] = make_int2(q1, p1);
-        reinterpret_cast<int2*>(w0)[i] = make_int2(q0, p0);
-      } else {
-        const int64_t i = e0 + q * T + threadIdx.x;
-        w1[i] = q1;
-        w0[i] = q0;
-      }
-    }
+  for (int q = 0; q < 4; q += 2) {
+    int q1, q0, p1, p0;
+    quantize(a[q], E, q1, q0);
+    quantize(a[q + 1], E, p1, p0);
+    const int64_t i = e0 / 2 + (q >> 1) * T + threadIdx.x;
+    reinterpret_cast<int2*>(w1)[i] = make_int2(q1, p1);
+    reinterpret_cast<int2*>(w0)[i] = make_int2(q0, p0);
   }
   nn = block_sum_256(nn, red);
   if (threadIdx.x == 0) part[blockIdx.x] = nn;
@@ -407,7 +377,7 @@ struct WTile {
   double* npart;         // [ntile] partials of |w'|^2 (LOCAL writes them)
 };
 
-template <bool CPLX, int TILE, bool LOCAL>
+template <int TILE, bool LOCAL>
 __global__ void __launch_bounds__(256, DOT_MINB)
     k_dots_q(const int* Q1, const int* Q0, const int* E, int64_t ld, int ntile, int64_t n, int nk, int ngroups,
              WTile W, double* part, Scal S, int j) {
@@ -417,7 +387,6 @@ __global__ void __launch_bounds__(256, DOT_MINB)
   const int tile = (int)(blockIdx.x / (unsigned)ngroups), g = (int)(blockIdx.x % (unsigned)ngroups);
   const int ka = g * DOT_GROUP, kb = min(nk, ka + DOT_GROUP);
   const int64_t e0 = (int64_t)tile * TILE;
-  constexpr int NV = CPLX ? 2 : 1;
   constexpr int U = TILE / 128 < DOT_LOADS ? TILE / 128 : DOT_LOADS;
   const int k = ka + wid;
   const int stop = S.flags[0];
@@ -439,14 +408,12 @@ __global__ void __launch_bounds__(256, DOT_MINB)
     __shared__ unsigned ured[8];
     __shared__ double2 s_h;
     const int64_t i = e0 + threadIdx.x;
-    double x = 0.0, u = 0.0, y = 0.0, v = 0.0;  // this entry and, complex, the other part of it
+    double x = 0.0, u = 0.0, y = 0.0, v = 0.0;  // this double and the other part of its entry
     if (i < n) {
       x = W.w[i];
       u = W.vj[i];
-      if (CPLX) {
-        y = W.w[i ^ 1];
-        v = W.vj[i ^ 1];
-      }
+      y = W.w[i ^ 1];
+      v = W.vj[i ^ 1];
     }
     if (stop) return;
     if (wid == 0) {
@@ -458,14 +425,10 @@ __global__ void __launch_bounds__(256, DOT_MINB)
     }
     __syncthreads();
     const double2 h = s_h;
-    if (CPLX) {
-      const bool im = threadIdx.x & 1;
-      const double2 t = three_term(im ? make_double2(y, x) : make_double2(x, y),
-                                   im ? make_double2(v, u) : make_double2(u, v), h);
-      x = im ? t.y : t.x;
-    } else {
-      x = three_term(x, u, h);
-    }
+    const bool im = threadIdx.x & 1;
+    const double2 t = three_term(im ? make_double2(y, x) : make_double2(x, y),
+                                 im ? make_double2(v, u) : make_double2(u, v), h);
+    x = im ? t.y : t.x;
     const int ew = block_exponent(abs_high_word(x), ured);
     ex += ew;
     int q1, q0;
@@ -487,9 +450,9 @@ __global__ void __launch_bounds__(256, DOT_MINB)
     if (stop) return;
   }
   if (k < kb) {
-    long long s[NV][3];
+    long long s[2][3];  // (re, im)
 #pragma unroll
-    for (int c = 0; c < NV; c++) s[c][0] = s[c][1] = s[c][2] = 0;
+    for (int c = 0; c < 2; c++) s[c][0] = s[c][1] = s[c][2] = 0;
 #pragma unroll 1
     for (int t = 0; t < TILE / 4; t += 32 * U) {
       if (t) {
@@ -506,31 +469,30 @@ __global__ void __launch_bounds__(256, DOT_MINB)
         fx_add(s[0], x1[u].y, x0[u].y, b1.y, b0.y);
         fx_add(s[0], x1[u].z, x0[u].z, b1.z, b0.z);
         fx_add(s[0], x1[u].w, x0[u].w, b1.w, b0.w);
-        if (CPLX) {  // Im conj(v) w = vr wi - vi wr
-          fx_add(s[NV - 1], x1[u].x, x0[u].x, b1.y, b0.y);
-          fx_add(s[NV - 1], -x1[u].y, -x0[u].y, b1.x, b0.x);
-          fx_add(s[NV - 1], x1[u].z, x0[u].z, b1.w, b0.w);
-          fx_add(s[NV - 1], -x1[u].w, -x0[u].w, b1.z, b0.z);
-        }
+        // Im conj(v) w = vr wi - vi wr
+        fx_add(s[1], x1[u].x, x0[u].x, b1.y, b0.y);
+        fx_add(s[1], -x1[u].y, -x0[u].y, b1.x, b0.x);
+        fx_add(s[1], x1[u].z, x0[u].z, b1.w, b0.w);
+        fx_add(s[1], -x1[u].w, -x0[u].w, b1.z, b0.z);
       }
     }
 #pragma unroll
-    for (int c = 0; c < NV; c++) {
+    for (int c = 0; c < 2; c++) {
       const double d = fx_warp_sum(s[c], ex);
-      if (lane == 0) part[((int64_t)k * ntile + tile) * NV + c] = d;
+      if (lane == 0) part[((int64_t)k * ntile + tile) * 2 + c] = d;
     }
   }
   if (!last_block(S.cnt + CNT_DOTS + g, ntile)) return;
   if (k < kb) {
     double a = 0, b = 0;
-    const double* p = part + (int64_t)k * ntile * NV;
+    const double* p = part + (int64_t)k * ntile * 2;
     for (int t = lane; t < ntile; t += 32) {
-      a += __ldcg(p + (int64_t)t * NV);
-      if (CPLX) b += __ldcg(p + (int64_t)t * NV + NV - 1);
+      a += __ldcg(p + (int64_t)t * 2);
+      b += __ldcg(p + (int64_t)t * 2 + 1);
     }
     for (int o = 16; o > 0; o >>= 1) {
       a += __shfl_xor_sync(0xffffffffu, a, o);
-      if (CPLX) b += __shfl_xor_sync(0xffffffffu, b, o);
+      b += __shfl_xor_sync(0xffffffffu, b, o);
     }
     if (lane == 0) {
       S.h2[2 * k] = a;
@@ -603,7 +565,7 @@ struct NextVec {
 // A pass with a coefficient not below 2^-30 |w'| (near an invariant subspace)
 // subtracts in FP64 and takes the norm of the result; its last block then scales
 // the whole vector.
-template <bool CPLX, int TILE, int KS, bool LOCAL>
+template <int TILE, int KS, bool LOCAL>
 __global__ void __launch_bounds__(KS * TILE / 4) k_update_q(const double* V, const int* Q1, const int* E, int64_t ld,
                                                             int ntile, int64_t n, int nk, WTile W, double* w,
                                                             double* part, Scal S, int j, double breakdown_tol,
@@ -611,8 +573,7 @@ __global__ void __launch_bounds__(KS * TILE / 4) k_update_q(const double* V, con
   pdl_begin();
   constexpr int NT = KS * TILE / 4, TP = TILE / 4;
   constexpr int NE = (TILE + NT - 1) / NT;  // entries per thread after the sum over slices
-  constexpr int VW = CPLX ? 2 : 1;
-  extern __shared__ float hf[];  // [VW nk] coefficients times the tile's scale
+  extern __shared__ float hf[];  // [2 nk] coefficients times the tile's scale
   __shared__ double red1[NT / 32];
   __shared__ unsigned ured[NT / 32];
   __shared__ __align__(16) float sred[KS * TILE];
@@ -632,14 +593,13 @@ __global__ void __launch_bounds__(KS * TILE / 4) k_update_q(const double* V, con
     a[q] = in ? w[r0 + i] : 0.0;
     if (LOCAL) {
       vo[q] = in ? W.vj[r0 + i] : 0.0;
-      wo[q] = CPLX && in ? w[(r0 + i) ^ 1] : 0.0;
-      vp[q] = CPLX && in ? W.vj[(r0 + i) ^ 1] : 0.0;
+      wo[q] = in ? w[(r0 + i) ^ 1] : 0.0;
+      vp[q] = in ? W.vj[(r0 + i) ^ 1] : 0.0;
     }
   }
-  for (int t = threadIdx.x; t < VW * nk; t += NT) {
-    const int k = t / VW;
-    const int e = E[(int64_t)k * ntile + tile] - 27;  // value = q1 2^(E - 56 + 29)
-    const double h = S.h2[2 * k + (t - k * VW)];
+  for (int t = threadIdx.x; t < 2 * nk; t += NT) {
+    const int e = E[(int64_t)(t >> 1) * ntile + tile] - 27;  // value = q1 2^(E - 56 + 29)
+    const double h = S.h2[t];
     // |h| 2^e below FP32's range is below 2^-100 of the tile's entries: zero
     hf[t] = e < -126 ? 0.0f : f64_lead_f32(h) * __uint_as_float((unsigned)(e + 127) << 23);
   }
@@ -648,8 +608,8 @@ __global__ void __launch_bounds__(KS * TILE / 4) k_update_q(const double* V, con
   if (wid == 0) {
     double hh = 0;
     unsigned hw = 0;
-    for (int t = lane; t < VW * nk; t += 32) {
-      const double h = S.h2[CPLX ? t : 2 * t];
+    for (int t = lane; t < 2 * nk; t += 32) {
+      const double h = S.h2[t];
       hh += h * h;
       hw = max(hw, abs_high_word(h));
     }
@@ -679,14 +639,10 @@ __global__ void __launch_bounds__(KS * TILE / 4) k_update_q(const double* V, con
     const double2 h = s_h;
 #pragma unroll
     for (int q = 0; q < NE; q++) {
-      if (CPLX) {
-        const bool im = threadIdx.x & 1;  // NT is even: every entry of this thread is the same part
-        const double2 t = three_term(im ? make_double2(wo[q], a[q]) : make_double2(a[q], wo[q]),
-                                     im ? make_double2(vp[q], vo[q]) : make_double2(vo[q], vp[q]), h);
-        a[q] = im ? t.y : t.x;
-      } else {
-        a[q] = three_term(a[q], vo[q], h);
-      }
+      const bool im = threadIdx.x & 1;  // NT is even: every entry of this thread is the same part
+      const double2 t = three_term(im ? make_double2(wo[q], a[q]) : make_double2(a[q], wo[q]),
+                                   im ? make_double2(vp[q], vo[q]) : make_double2(vo[q], vp[q]), h);
+      a[q] = im ? t.y : t.x;
     }
   }
   if (tile == 0 && threadIdx.x == 0) S.alpha[j] += S.h2[2 * j];
@@ -708,19 +664,11 @@ __global__ void __launch_bounds__(KS * TILE / 4) k_update_q(const double* V, con
     for (int k = sl; k < nk; k += KS) {
       const int4 v = __ldcg(p + k * ld4);
       const float v0 = (float)v.x, v1 = (float)v.y, v2 = (float)v.z, v3 = (float)v.w;
-      if (CPLX) {
-        const float hr = hf[2 * k], hi = hf[2 * k + 1];
-        d[0] = fmaf(hr, v0, fmaf(-hi, v1, d[0]));
-        d[1] = fmaf(hr, v1, fmaf(hi, v0, d[1]));
-        d[2] = fmaf(hr, v2, fmaf(-hi, v3, d[2]));
-        d[3] = fmaf(hr, v3, fmaf(hi, v2, d[3]));
-      } else {
-        const float h = hf[k];
-        d[0] = fmaf(h, v0, d[0]);
-        d[1] = fmaf(h, v1, d[1]);
-        d[2] = fmaf(h, v2, d[2]);
-        d[3] = fmaf(h, v3, d[3]);
-      }
+      const float hr = hf[2 * k], hi = hf[2 * k + 1];
+      d[0] = fmaf(hr, v0, fmaf(-hi, v1, d[0]));
+      d[1] = fmaf(hr, v1, fmaf(hi, v0, d[1]));
+      d[2] = fmaf(hr, v2, fmaf(-hi, v3, d[2]));
+      d[3] = fmaf(hr, v3, fmaf(hi, v2, d[3]));
     }
     *reinterpret_cast<float4*>(sred + sl * TILE + pos * 4) = make_float4(d[0], d[1], d[2], d[3]);
     __syncthreads();
@@ -749,13 +697,8 @@ __global__ void __launch_bounds__(KS * TILE / 4) k_update_q(const double* V, con
     const int64_t r = r0 + q * NT + threadIdx.x;
     if (q * NT + (int)threadIdx.x >= TILE || r >= n) continue;
     for (int k = 0; k < nk; k++) {
-      const double v = V[k * n + r];
-      if (CPLX) {
-        const double u = V[k * n + (r ^ 1)], hr = S.h2[2 * k], hi = S.h2[2 * k + 1];
-        a[q] -= (r & 1) ? hr * v + hi * u : hr * v - hi * u;
-      } else {
-        a[q] -= S.h2[2 * k] * v;
-      }
+      const double v = V[k * n + r], u = V[k * n + (r ^ 1)], hr = S.h2[2 * k], hi = S.h2[2 * k + 1];
+      a[q] -= (r & 1) ? hr * v + hi * u : hr * v - hi * u;
     }
     nx.v[r] = a[q];  // not yet scaled (w is still read by other blocks' three-term step)
     nn += a[q] * a[q];

@@ -779,11 +779,11 @@ void gs_step_q(blqh_lanczos* L, int j) {
   const int nk = j + 1, wr = L->mmax + 1, ng = (nk + DOT_GROUP - 1) / DOT_GROUP;
   const int na = grid_for(ctx, L->dim, 1024, 2);
   const WTile W{vj, L->w, L->apart, na, q1_row(L, wr), q0_row(L, wr), qe_row(L, wr), L->npart};
-  launch_chained(ctx, k_alpha<true>, na, 256, 0, vj, L->w, L->dim, L->apart, L->S);
-  if (!LOCAL)
-    launch_chained(ctx, k_local<true, TILE>, L->ntile, TILE / 4, 0, vj, L->w, n, L->apart, na, q1_row(L, wr),
+  launch_chained(ctx, k_alpha, na, 256, 0, vj, L->w, L->dim, L->apart, L->S);
+  if constexpr (!LOCAL)
+    launch_chained(ctx, k_local<TILE>, L->ntile, TILE / 4, 0, vj, L->w, n, L->apart, na, q1_row(L, wr),
                    q0_row(L, wr), qe_row(L, wr), L->npart, L->S, j);
-  launch_chained(ctx, k_dots_q<true, TILE, LOCAL>, ng * L->ntile, 256, 0, L->Q1, L->Q0, L->QE, L->pld, L->ntile, n,
+  launch_chained(ctx, k_dots_q<TILE, LOCAL>, ng * L->ntile, 256, 0, L->Q1, L->Q0, L->QE, L->pld, L->ntile, n,
                  nk, ng, W, L->part, L->S, j);
   const size_t hsm = (size_t)nk * 2 * sizeof(float);
   auto update = [&](auto kern, int threads) {
@@ -791,9 +791,9 @@ void gs_step_q(blqh_lanczos* L, int j) {
                    L->S, j, 1e-13, next_vec(L, j + 1));
   };
   // one slice of vectors per block while the blocks alone give every SM four
-  if constexpr (LOCAL) update(k_update_q<true, 256, 16, true>, 1024);
-  else if (L->ntile >= 4 * ctx->num_sms) update(k_update_q<true, 1024, 1, false>, 256);
-  else update(k_update_q<true, 1024, 4, false>, 1024);
+  if constexpr (LOCAL) update(k_update_q<256, 16, true>, 1024);
+  else if (L->ntile >= 4 * ctx->num_sms) update(k_update_q<1024, 1, false>, 256);
+  else update(k_update_q<1024, 4, false>, 1024);
   count_launch(ctx, TM_REORTH, LOCAL ? 3 : 4);
 }
 
@@ -1109,9 +1109,9 @@ blqh_lanczos* create_impl(blqh_ctx* ctx, const blqh_csr* M, const blqh_lanczos_o
   smem_attr_at_least(k_update_o<false, 4, true>, upd_smem);
   smem_attr_at_least(k_update_o<true, 1, false>, upd_smem);
   const int q_smem = 2 * (L->mmax + 1) * (int)sizeof(float);
-  smem_attr_at_least(k_update_q<true, 256, 16, true>, q_smem);
-  smem_attr_at_least(k_update_q<true, 1024, 4, false>, q_smem);
-  smem_attr_at_least(k_update_q<true, 1024, 1, false>, q_smem);
+  smem_attr_at_least(k_update_q<256, 16, true>, q_smem);
+  smem_attr_at_least(k_update_q<1024, 4, false>, q_smem);
+  smem_attr_at_least(k_update_q<1024, 1, false>, q_smem);
   try {
     const int64_t n = L->dim * L->vw;
     L->V = dalloc<double>(ctx, (size_t)(L->mmax + 1) * n);
@@ -1119,7 +1119,7 @@ blqh_lanczos* create_impl(blqh_ctx* ctx, const blqh_csr* M, const blqh_lanczos_o
     L->psi = dalloc<double>(ctx, n);
     const int m = L->mmax;
     const int max_groups = m / DOT_GROUP + 2;  // vector groups of the dots, one arrival counter each
-    const size_t ns = (size_t)m + (m + 1) + 2 * (m + 1) + 2 * (m + 1) + 4 + m + 4 + (CNT_DOTS + max_groups + 1) / 2;
+    const size_t ns = (size_t)m + (m + 1) + 2 * (m + 1) + 4 + m + 4 + (CNT_DOTS + max_groups + 1) / 2;
     L->scal = dalloc<double>(ctx, ns);
     BLQH_TRY_CUDA(ctx, cudaMemsetAsync(L->scal, 0, ns * 8, ctx->stream));
     double* p = L->scal;
@@ -1127,8 +1127,6 @@ blqh_lanczos* create_impl(blqh_ctx* ctx, const blqh_csr* M, const blqh_lanczos_o
     p += m;
     L->S.beta = p;
     p += m + 1;
-    L->S.h = p;
-    p += 2 * (m + 1);
     L->S.h2 = p;
     p += 2 * (m + 1);
     L->S.nrm = p;
@@ -1218,7 +1216,7 @@ void debug_dots_q(blqh_ctx* ctx, DevBufs& G, const double* V, const double* w, i
     launch_chained(ctx, k_planes_q<TILE>, ntile, TILE / 4, 0, k < nk ? V + k * n : w, n,
                    NextVec{nullptr, nullptr, nullptr, nullptr, q1 + k * pld, q0 + k * pld, qe + (int64_t)k * ntile});
   const WTile W{w, w, apart, 1, q1 + nk * pld, q0 + nk * pld, qe + (int64_t)nk * ntile, npart};
-  launch_chained(ctx, k_dots_q<true, TILE, LOCAL>, ng * ntile, 256, 0, q1, q0, qe, pld, ntile, n, nk, ng, W, part, S,
+  launch_chained(ctx, k_dots_q<TILE, LOCAL>, ng * ntile, 256, 0, q1, q0, qe, pld, ntile, n, nk, ng, W, part, S,
                  0);
 }
 

@@ -142,6 +142,41 @@ def test_even_vectors_and_long_rows(B, kind, sec):
         o.close()
 
 
+@pytest.mark.parametrize("sec", [(8, 8, 4, 0, 1), (12, 12, 6, 3, 5), (14, 14, 7, 0, 3)], ids=str)
+def test_full_pass_near_an_invariant_subspace(B, monkeypatch, sec):
+    """From a nearly converged state the first step's coefficients are not small and the full pass subtracts in FP64,
+    one block then scaling the vector and its planes (256- and 1024-double tiles): the next product is as good as any,
+    and ten steps give the FP64 pass's coefficients (beta_1 ~ 1e-6 known to 1e-15: what follows to 1e-7)."""
+    b, H = build(B, "ground", sec)
+    csr = H.csr()
+    for steps in range(20, 200, 4):
+        L = B.Lanczos(H, max_steps=steps, tol=0.0, seed=2)
+        L.iterate()
+        psi, E = L.ritz_vector(), L.rayleigh()
+        L.close()
+        res = np.linalg.norm(H.spmv(psi) - E * psi)
+        if res < 3e-6:
+            break
+    assert res > 1e-8
+    L = B.Lanczos(H, max_steps=1, tol=0.0, start=psi)
+    L.iterate()
+    x, y = product(L, H.dim)
+    L.close()
+    assert abs(np.linalg.norm(x) - 1) < 1e-13 and abs(np.vdot(psi, x)) < 1e-8
+    e, bound = errors(H, csr, x, y, np.linspace(0, H.dim - 1, 2000).astype(int))
+    assert np.all(e <= bound), float(np.max(e / bound))
+    out = []
+    for env in ("0", "1"):
+        monkeypatch.setenv("BLQH_GS_FP64", env)
+        L = B.Lanczos(H, max_steps=10, tol=0.0, start=psi)
+        L.iterate()
+        out.append(np.concatenate(L.coeffs()))
+        L.close()
+    assert np.max(np.abs(out[0] - out[1])) < 1e-7
+    H.close()
+    b.close()
+
+
 def test_infinite_elements_stay_visible(B):
     """A tunnelling amplitude at the end of FP64's range, which short orbits multiply beyond it: a row with an infinite
     element has no finite product, and the recurrence no finite coefficient."""
