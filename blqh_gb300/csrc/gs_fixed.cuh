@@ -166,12 +166,12 @@ __device__ __forceinline__ int word_exponent(unsigned hw) { return (int)(hw >> 2
 __device__ __forceinline__ int block_exponent(unsigned hw, unsigned* red) { return word_exponent(block_max(hw, red)); }
 
 // xe of a normalized vector v = (w - c) inv for fix_scaled, 2^E <= max |w| < 2^(E+1),
-// |c| <= sqrt(cc): the least power of two above a bound on |v| (at most 4 times the
-// largest entry for negligible c), and no more than 2^0.
+// |c| <= sqrt(cc): a power of two above |v| (at most 4 times the largest entry for
+// negligible c), and no more than 2^0. Integers only, one lane's FP64 would hold the block up.
 __device__ __forceinline__ int scaled_exponent(int E, double cc, double inv) {
-  const double a = __hiloint2double((E + 1 + 1023) << 20, 0);
-  const double c = __hiloint2double((((word_exponent(abs_high_word(cc)) + 2) >> 1) + 1023) << 20, 0);
-  return min(word_exponent(abs_high_word((a + c) * inv * (1 + 0x1p-20))) + 1, 0);
+  const int C = (word_exponent(abs_high_word(cc)) + 2) >> 1;  // sqrt(cc) < 2^C
+  const int sum = C < E - 20 ? E + 1 : max(E + 1, C) + 1;     // |w| + |c| < 2^sum (1 + 2^-20)
+  return min(sum + word_exponent(abs_high_word(inv) + 4) + 1, 0);
 }
 
 // Sum of a pair over the warp, in every lane. (One warp sums what a block needs: an

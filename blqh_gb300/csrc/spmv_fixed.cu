@@ -37,6 +37,9 @@
 
 namespace {
 
+// Up to here one block splits a vector in less than the ~4 us of a second launch (8 entries a thread).
+constexpr int64_t FIX_SHORT = 8192;
+
 // Row exponents, split off-diagonal values and the diagonal: one warp per row. The
 // exponent is raised until the row's sum of |q| stays below 2^67 (rows of up to 512
 // nonzeros always do), so that a product with |x| <= 2^59 units stays below 2^127. A row
@@ -99,6 +102,17 @@ __global__ void __launch_bounds__(256) k_fix_max(const double* __restrict__ x, u
     hw = max(hw, abs_high_word(x[i]));
   hw = block_max(hw, red);
   if (threadIdx.x == 0) atomicMax(xmax, hw);
+}
+// Both in one block, for short vectors: one launch where they are two and a memset.
+__global__ void __launch_bounds__(1024) k_fix_short(const double* __restrict__ x, int2* __restrict__ xq, int* xe,
+                                                    int n, const int* stop) {
+  if (stop && *stop) return;
+  __shared__ unsigned red[32];
+  unsigned hw = 0;
+  for (int i = threadIdx.x; i < n; i += 1024) hw = max(hw, abs_high_word(x[i]));
+  const int e = min(word_exponent(block_max(hw, red)) + 1, 0);
+  if (threadIdx.x == 0) *xe = e;
+  for (int i = threadIdx.x; i < n; i += 1024) xq[i] = fix_scaled(x[i], e);
 }
 __global__ void k_fix_vector(const double* __restrict__ x, int2* __restrict__ xq, int* xe, const unsigned* xmax,
                              int64_t n, const int* stop) {
@@ -224,6 +238,12 @@ void fixed_release(FixedMatrix* F) {
 // x (|x| <= 1, as Krylov vectors are) in fixed point; xmax: scratch.
 void fixed_vector(blqh_ctx* ctx, const double* x, int2* xq, int* xe, unsigned* xmax, int64_t n, const int* stop) {
   TimerScope tm(ctx, TM_MISC);
+  if (n <= FIX_SHORT) {
+    k_fix_short<<<1, 1024, 0, ctx->stream>>>(x, xq, xe, (int)n, stop);
+    BLQH_TRY_CUDA(ctx, cudaGetLastError());
+    count_launch(ctx, TM_MISC);
+    return;
+  }
   const int grid = grid_for(ctx, n, 256, 8);
   BLQH_TRY_CUDA(ctx, cudaMemsetAsync(xmax, 0, sizeof(unsigned), ctx->stream));
   k_fix_max<<<grid, 256, 0, ctx->stream>>>(x, xmax, n, stop);
