@@ -21,11 +21,12 @@
 // gs_ordered.cuh, and then depend on it); complex instances take it on fixed-point
 // planes of the Krylov basis (gs_fixed.cuh), one exponent per vector (57 bits below its
 // largest entry): exact integer dots (error against extended precision, random vectors
-// of 79 to 100,141 complex entries: 0.18 to 0.42 of the FP64 dots'), and the correction in FP32 while every coefficient is below 2^-36 |w|. The
-// FP64 pass of a complex instance took the SM's FP64 pipe 8 FMAs per entry and
-// vector; 96 instances of 5,940 states, 150 steps: 348 -> 134 ms. The lowest Ritz pair comes from
-// Sturm multisection and inverse iteration; the finisher is the FP64
-// regenerated Rayleigh quotient for FP32 values, the stored FP64 CSR otherwise.
+// of 79 to 100,141 complex entries: 0.18 to 0.42 of the FP64 dots'), and the correction
+// in FP32 while every coefficient is below 2^-36 |w|. The FP64 pass of a complex
+// instance took the SM's FP64 pipe 8 FMAs per entry and vector; 96 instances of 5,940
+// states, 150 steps: 348 -> 134 ms. The lowest Ritz pair comes from Sturm
+// multisection and inverse iteration; the finisher is the FP64 regenerated Rayleigh
+// quotient for FP32 values, the stored FP64 CSR otherwise.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -864,7 +865,10 @@ struct blqh_batch {
   double** d_res = nullptr;
   int nrq = 0;
   int threads = 512, lpr = 16, bps = 1, smem = 0, grid = 0;
-  int64_t x_cap = 0;                 // bytes of the shared x area
+  int64_t x_cap = 0;                 // bytes of the shared x area (set_shape may grow it for complex instances)
+  int64_t max_n = 0;                 // longest vector
+  int fixed = 0, smem_max = 0;       // bytes of the other shared memory; of what a block may have
+  std::vector<BInst> hinst;          // the instances that run, as in d_inst
   double mean_row = 0, mean_dim = 0; // over the running instances (tuning class)
   KFn kern = nullptr;
   cudaGraphExec_t gexec = nullptr;
@@ -925,14 +929,46 @@ void configure_shape(blqh_batch* b, int threads, int lpr) {
   b->grid = std::max(1, std::min(b->nrun, ctx->num_sms * b->bps));
 }
 
+// A shape with its x area. Where one block per SM is all there is (by its registers and
+// shared memory, or by the number of instances), the area takes what shared memory is
+// left, so that the gathers of larger complex instances stay in it.
+void set_shape(blqh_batch* b, int threads, int lpr) {
+  blqh_ctx* ctx = b->ctx;
+  int64_t cap = b->x_cap;
+  b->smem = b->fixed + (int)((cap + 15) / 16 * 16);
+  configure_shape(b, threads, lpr);
+  if (b->bps == 1 || b->nrun <= ctx->num_sms) {
+    cudaFuncAttributes fa;  // the kernel's own static shared memory counts against the limit
+    BLQH_TRY_CUDA(ctx, cudaFuncGetAttributes(&fa, reinterpret_cast<const void*>(b->kern)));
+    const int64_t room = (b->smem_max - b->fixed - (int64_t)fa.sharedSizeBytes) / 16 * 16;
+    const int64_t grown = std::min<int64_t>((b->max_n * 8 + 15) / 16 * 16, room);
+    if (grown > cap) {
+      cap = grown;
+      b->smem = b->fixed + (int)cap;
+      configure_shape(b, threads, lpr);
+    }
+  }
+  bool changed = false;
+  for (BInst& I : b->hinst) {
+    const int fits = I.dim * 16 <= cap;
+    if (!I.cplx || I.xsmem == fits) continue;
+    I.xsmem = fits;
+    changed = true;
+  }
+  if (changed)
+    BLQH_TRY_CUDA(ctx, cudaMemcpy(b->d_inst, b->hinst.data(), b->hinst.size() * sizeof(BInst), cudaMemcpyHostToDevice));
+}
+
 // K10 for the batch: each candidate shape runs one round of the most
 // expensive instances (one per resident block) for a few Lanczos steps on the
-// batch's own data; the fastest per instance-step wins and is cached per class.
+// batch's own data, as the solve will run them; the fastest per instance-step wins and
+// is cached per class (batches with planes and without are two; v2: the shape's x area
+// and the planes are part of what was timed).
 void tune_shape(blqh_batch* b) {
   blqh_ctx* ctx = b->ctx;
-  bool any_cplx = false;
-  for (auto* m : b->csr) any_cplx = any_cplx || (m && m->is_complex);
-  const std::string key = tune_key("batch", b->o.value_precision, any_cplx, (int64_t)b->mean_dim, b->mean_row,
+  int kind = 0;  // 1: complex instances among them, 2: with planes
+  for (const BInst& I : b->hinst) kind = std::max(kind, I.cplx ? (I.q1 ? 2 : 1) : 0);
+  const std::string key = tune_key("batch|v2", b->o.value_precision, kind, (int64_t)b->mean_dim, b->mean_row,
                                    b->o.lambda);
   int t = 0, l = 0;
   if (!tune_lookup(key, &t, &l)) {
@@ -941,14 +977,14 @@ void tune_shape(blqh_batch* b) {
     for (int th : {256, 512})
       for (int lp : {4, 8, 16, 32}) {
         if (lp == 4 && b->mean_row >= 24) continue;
-        configure_shape(b, th, lp);
+        set_shape(b, th, lp);
         const int nsub = std::min(b->nrun, ctx->num_sms * b->bps);
         double ms_best = 1e30;
         for (int rep = 0; rep < 2; rep++) {
           BLQH_TRY_CUDA(ctx, cudaMemsetAsync(b->d_counter, 0, sizeof(int), ctx->stream));
           BLQH_TRY_CUDA(ctx, cudaEventRecord(b->ev[0], ctx->stream));
           b->kern<<<std::min(b->grid, nsub), b->threads, b->smem, ctx->stream>>>(b->d_inst, b->d_order, nsub, lam_t,
-                                                                                 b->o.seed, 1e-13, 0, b->d_counter);
+                                                                                 b->o.seed, 1e-13, 1, b->d_counter);
           BLQH_TRY_CUDA(ctx, cudaGetLastError());
           BLQH_TRY_CUDA(ctx, cudaEventRecord(b->ev[1], ctx->stream));
           BLQH_TRY_CUDA(ctx, cudaEventSynchronize(b->ev[1]));
@@ -965,7 +1001,7 @@ void tune_shape(blqh_batch* b) {
       }
     tune_store(key, t, l, best);
   }
-  configure_shape(b, t, l);
+  set_shape(b, t, l);
 }
 
 void batch_create_impl(blqh_batch* b) {
@@ -999,7 +1035,6 @@ void batch_create_impl(blqh_batch* b) {
   b->csr.assign(b->n, nullptr);
   b->N.assign(b->n, 0);
   double nnz_sum = 0, dim_sum = 0;
-  int64_t max_n = 0;
   for (int i = 0; i < b->n; i++) {
     const blqh_basis* B = b->bases[b->bidx[i]];
     if (B->dim == 0) continue;
@@ -1016,16 +1051,15 @@ void batch_create_impl(blqh_batch* b) {
     b->N[i] = M->dim * (M->is_complex ? 2 : 1);
     nnz_sum += (double)M->nnz;
     dim_sum += (double)M->dim;
-    max_n = std::max(max_n, b->N[i]);
+    b->max_n = std::max(b->max_n, b->N[i]);
   }
   // shared memory: the fixed part plus an x area for the instances that fit in it
-  int smem_max = 0;
-  cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
-  const int fixed = batch_fixed_doubles(lam) * 8;
-  const int64_t x_cap = std::min<int64_t>(max_n * 8, (int64_t)std::max(0, 96 * 1024 - fixed));
+  cudaDeviceGetAttribute(&b->smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
+  b->fixed = batch_fixed_doubles(lam) * 8;
+  const int64_t x_cap = std::min<int64_t>(b->max_n * 8, (int64_t)std::max(0, 96 * 1024 - b->fixed));
   b->x_cap = x_cap;
-  b->smem = fixed + (int)((x_cap + 15) / 16 * 16);
-  if (b->smem > smem_max) {
+  b->smem = b->fixed + (int)((x_cap + 15) / 16 * 16);
+  if (b->smem > b->smem_max) {
     set_error(ctx, BLQH_ERR_UNSUPPORTED, "blqh_batch_create: lambda too large for shared memory");
     throw BlqhError{BLQH_ERR_UNSUPPORTED, "smem"};
   }
@@ -1064,7 +1098,7 @@ void batch_create_impl(blqh_batch* b) {
       ctx->last_error.clear();
     }
   b->d_resall = dalloc<double>(ctx, 5 * (size_t)std::max(1, b->n));  // every instance's results, read back at once
-  std::vector<BInst> hi;
+  std::vector<BInst>& hi = b->hinst;
   std::vector<double> cost;
   std::vector<double*> res_ptr;
   for (int i = 0; i < b->n; i++) {
@@ -1109,22 +1143,9 @@ void batch_create_impl(blqh_batch* b) {
     BLQH_TRY_CUDA(ctx, cudaMemcpy(b->d_order, order.data(), order.size() * sizeof(int), cudaMemcpyHostToDevice));
   }
   b->grid = std::max(1, std::min(b->nrun, ctx->num_sms * b->bps));
-  if (b->o.threads == 0 && b->o.lanes_per_row == 0 && tune_enabled() && b->nrun > 0) tune_shape(b);
-  // Where one block per SM is all there is (by its registers and shared memory, or by
-  // the number of instances), the x area takes what shared memory is left, so that
-  // the gathers of larger complex instances stay in it.
-  if (b->nrun && (b->bps == 1 || b->nrun <= ctx->num_sms)) {
-    cudaFuncAttributes fa;  // the kernel's own static shared memory counts against the limit
-    BLQH_TRY_CUDA(ctx, cudaFuncGetAttributes(&fa, reinterpret_cast<const void*>(b->kern)));
-    const int64_t room = (smem_max - fixed - (int64_t)fa.sharedSizeBytes) / 16 * 16;
-    const int64_t cap = std::min<int64_t>((max_n * 8 + 15) / 16 * 16, room);
-    if (cap > b->x_cap) {
-      b->smem = fixed + (int)cap;
-      configure_shape(b, b->threads, b->lpr);
-      for (BInst& I : hi)
-        if (I.cplx) I.xsmem = I.dim * 16 <= cap;
-      BLQH_TRY_CUDA(ctx, cudaMemcpy(b->d_inst, hi.data(), hi.size() * sizeof(BInst), cudaMemcpyHostToDevice));
-    }
+  if (b->nrun) {
+    if (b->o.threads == 0 && b->o.lanes_per_row == 0 && tune_enabled()) tune_shape(b);
+    else set_shape(b, b->threads, b->lpr);
   }
   // mixed precision: one regenerated Rayleigh quotient per instance
   b->rq.assign(b->n, nullptr);
