@@ -1136,8 +1136,11 @@ blqh_lanczos* create_impl(blqh_ctx* ctx, const blqh_csr* M, const blqh_lanczos_o
     L->S.flags = reinterpret_cast<int*>(p);
     p += 4;
     L->S.cnt = reinterpret_cast<unsigned*>(p);
-    // short tiles spread small sectors over more blocks
-    L->tile = n <= 65536 ? 256 : 1024;
+    // Short tiles spread small sectors over more blocks and save a kernel per step; they cost more
+    // reductions and smaller runs of loads. us per step, product included, 256 against 1024, runs of
+    // 100 and 250 steps: 5,940 rows 33.8 : 38.0 and 38.7 : 41.0; 9,402 rows 38.4 : 40.2 and 44.9 : 44.9;
+    // 16,024 rows 48.1 : 46.2 and 57.9 : 52.6; 30,772 rows 85.7 : 71.7 and 103 : 82.2.
+    L->tile = n <= 24576 ? 256 : 1024;
     L->ntile = (int)((n + L->tile - 1) / L->tile);
     L->pld = (int64_t)L->ntile * L->tile;
     L->nblk_dot = (int)((L->dim + GS_ROWS - 1) / GS_ROWS);
