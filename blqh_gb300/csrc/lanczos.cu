@@ -790,9 +790,12 @@ void gs_step_q(blqh_lanczos* L, int j) {
     launch_chained(ctx, kern, L->ntile, threads, hsm, L->V, L->Q1, L->QE, L->pld, L->ntile, n, nk, W, L->w, L->pnorm,
                    L->S, j, 1e-13, next_vec(L, j + 1));
   };
-  // one slice of vectors per block while the blocks alone give every SM four
+  // One slice of vectors per block once the tiles alone give every SM two blocks, else four slices.
+  // us per step, product included, one against four, runs of 100 and 250 steps: 100,141 rows (196 tiles)
+  // 170 : 168 and 213 : 203; 143,143 rows (280) 200 : 197 and 252 : 244; 204,660 rows (400) 305 : 309 and
+  // 373 : 375; 322,203 rows (630) 451 : 474 and 553 : 577.
   if constexpr (LOCAL) update(k_update_q<256, 16, true>, 1024);
-  else if (L->ntile >= 4 * ctx->num_sms) update(k_update_q<1024, 1, false>, 256);
+  else if (L->ntile >= 2 * ctx->num_sms) update(k_update_q<1024, 1, false>, 256);
   else update(k_update_q<1024, 4, false>, 1024);
   count_launch(ctx, TM_REORTH, LOCAL ? 3 : 4);
 }
