@@ -825,10 +825,15 @@ void gs_step_o(blqh_lanczos* L, int j) {
                    j);
   if (L->o.reorth) {
     const int nk = j + 1;
-    // up to 64 tiles: 8 vectors per block (one per warp), summed by each group's last block; beyond, a
+    // few tiles: 8 vectors per block (one per warp), summed by each group's last block; beyond, a
     // kernel for the sums, and more vectors per block once the blocks would fill the GPU over and over:
-    // 4 times for double-float dots (staging w's tile splits it), 16 for FP64 ones (32 at least: 4 per warp)
-    const int finish = nt <= 64;
+    // 4 times for double-float dots (staging w's tile splits it), 16 for FP64 ones (32 at least: 4 per warp).
+    // us per step, product included, last block against kernel, runs of 100 and 200 steps. Real FP64 dots:
+    // 98 tiles 144 : 173 and 154 : 180; 315 tiles 340 : 352 and 380 : 384; 632 tiles 1024 : 1028 and
+    // 1104 : 1098; 1,062 tiles 925 : 923 and 1059 : 1050. Double-float: 35 tiles 50.5 : 51.3 and 59.1 : 58.7;
+    // 59 tiles 92.8 : 92.6 and 102 : 101; 140 tiles 151 : 147 and 167 : 163 (the complex FP64 pass, taken
+    // where there is no room for planes, keeps that line).
+    const int finish = nt <= (df || CPLX ? 64 : 512);
     const int step = finish || df || CPLX ? 8 : 32;
     const int waves = (int)((int64_t)nt * ((nk + step - 1) / step) / ((df ? 4 : 16) * ctx->num_sms));
     const int gk = step * (finish ? 1 : std::max(1, waves)), ng = (nk + gk - 1) / gk;
