@@ -37,9 +37,9 @@
 // launched with programmatic stream serialization: its blocks are placed while the
 // previous kernel drains. Results are reproducible.
 //
-// Measured per step without the SpMV (200 steps, one GB300): 60,096 rows 300 -> 55
-// us, 100,141 rows 311 -> 81 us, 647,079 rows (FP32 values) 496 -> 355 us, 16,024
-// rows (short tiles) 251 -> 38 us.
+// Measured per step without the SpMV (200 steps, one GB300): 60,096 rows 300 -> 52
+// us, 100,141 rows 311 -> 78 us, 647,079 rows (FP32 values) 496 -> 355 us, 16,024
+// rows 251 -> 34 us.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -559,7 +559,7 @@ struct NextVec {
 // Full pass, correction, and the next vector: v_{j+1} = (w' - sum_k h2[k] V_k) /
 // beta_{j+1} with its planes. One block per tile; KS slices of the vectors share
 // it, each thread four entries: KS = 1 (256 threads, 4 KB runs per vector) where
-// the tiles alone give every SM several blocks, else 1024 threads (KS = 4, or 16
+// the tiles alone give every SM two blocks (gs_step_q), else 1024 threads (KS = 4, or 16
 // on 256-entry tiles). Tiles are taken in descending order (see k_dots_q).
 // LOCAL: w' = w - h_j v_j is formed here (see k_dots_q), else k_local left it in w.
 // A pass with a coefficient not below 2^-30 |w'| (near an invariant subspace)

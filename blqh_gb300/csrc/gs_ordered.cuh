@@ -6,9 +6,11 @@
 // rounding. So the order of every sum is part of the result here: tiles of GS_ROWS
 // rows, one warp per (tile, vector) with lane t taking rows t, t + 32, ...;
 // partials summed 256 at a time by warps, then over the warps; the correction
-// summed over even and odd vectors. Complex sectors have no such degeneracy and
-// take the fixed-point pass of gs_fixed.cuh, which is faster. (Complex sectors
-// without room for its planes, or with BLQH_GS_FP64=1, come here too.)
+// summed over even and odd vectors. (The products keep one order up to 2^15 rows;
+// beyond, the tuner's choice of their form is another one.) Complex sectors, where no
+// such degeneracy has been met, take the fixed-point pass of gs_fixed.cuh, which is
+// faster and reproducible too. (Complex sectors without room for its planes, with
+// accumulate = 1 or with BLQH_GS_FP64=1, come here.)
 //
 // FP64-valued runs take FP64 dots (FP64 pipe); FP32-valued runs with double-float
 // accumulation take double-float dots on FP32 planes kept next to each FP64
@@ -207,8 +209,8 @@ __device__ __forceinline__ double warp_sum4(double s0, double s1, double s2, dou
 // so that large sectors stage w's tile once. DF: from the planes (row stride ld),
 // 16-byte loads. With `finish` (few tiles) the last block of a group sums its
 // vectors' partials (part[k][tile]) and sets flags[4] when a coefficient is not
-// below 2^-30 |w|; else k_reduce_o does: at 632 tiles that sum is 8 dependent
-// rounds per vector, 60 us in one block, 7 us in a kernel of one block per vector.
+// below 2^-30 |w|; else k_reduce_o does, one block per vector (where the line lies:
+// gs_step_o).
 template <bool CPLX, bool DF, int KB>
 __global__ void __launch_bounds__(256) k_dots_o(const double* V, const float* Vh, const float* Vl, int64_t ld,
                                                 int64_t dim, int ntile, int nk, int gk, int ngroups, const double* w,

@@ -33,7 +33,8 @@
 // diagonal last, as in the reference (:187). Pass 0 counts the entries with |value|
 // > 1e-10; pass 1 sorts them by column (bitonic, per warp) and writes them.
 //
-// Bound by instruction issue and shared-memory latency. Nphi = 30, Ne = 10 (100,141
+// Bound by latency with few warps (the tables in shared memory leave 13 of 64 per SM;
+// issue 34 %) and the FP64 pipe (51 %: phases and sums). Nphi = 30, Ne = 10 (100,141
 // rows, 10 translations), whole build: 93 -> 10 ms against every translate.
 #include <algorithm>
 #include <cmath>

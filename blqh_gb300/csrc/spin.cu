@@ -42,9 +42,9 @@
 // carries momentum K, an explicit signed sum otherwise (short orbits). Odd nphi, a
 // twist theta_x (the tables are read at |mt - n|, which a wrapped translate turns
 // into nphi - |mt - n|) and a parallel-field phase with tunnelling are not
-// translation covariant and enumerate every translate. Rows are generated once, into a staging buffer, and
-// compacted after the scan. Bound by issue and shared-memory latency: Nphi = 8,
-// 16,024 states, K = 3: 257 -> 1.0 ms.
+// translation covariant and enumerate every translate. Rows are generated once, into
+// a staging buffer, and compacted after the scan. Bound by the FP64 pipe (63 % busy) and
+// shared-memory latency (issue 40 %): Nphi = 8, 16,024 states, K = 3: 257 -> 1.0 ms.
 #include <algorithm>
 #include <cmath>
 #include <string>
